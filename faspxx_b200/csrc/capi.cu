@@ -502,6 +502,10 @@ int fasp_gpu_mat_set_rowclass(fasp_gpu_mat A, int mode)
 int fasp_gpu_mat_set_col16(fasp_gpu_mat A, int on)
 {
     if (!A) return kErrInputPar;
+    if (on) { // formed when first turned on
+        int e = m_build_col16(A->M, A->c.stream);
+        if (e) return e;
+    }
     A->M.cd16On = on != 0;
     return kOk;
 }
@@ -509,7 +513,7 @@ int fasp_gpu_mat_set_col16(fasp_gpu_mat A, int on)
 int fasp_gpu_mat_col16_info(fasp_gpu_mat A, int* built, int* inUse)
 {
     if (!A) return kErrInputPar;
-    if (built) *built = A->M.cd16 != nullptr;
+    if (built) *built = A->M.near16;
     if (inUse) *inUse = A->M.cd16 != nullptr && A->M.cd16On && !A->M.rcOn;
     return kOk;
 }

@@ -210,9 +210,10 @@ struct Mat {
     int       lanes = 8;         // lanes per row of the SpMV (autotuned or from row lengths)
     bool      diagConst = false; // every row stores a diagonal entry, all with one value
     int16_t*  cd16 = nullptr;    // colInd - row when every entry is within 32,767 columns
+    bool      near16 = false;    // such offsets exist: every entry is that near its row
     bool      cd16On = false;    // the thread-per-row kernels use cd16 (opt-in: measured
                                  // slower than the 32-bit colInd on B200)
-    uint32_t  tileSpan = 0;      // most entries of a 256-row tile (m_tile_span), 0 unknown
+    uint32_t  tileSpan = 0;      // most entries of a 256-row tile (m_inspect), 0 unknown
     double    diagValue = 0.0;
     uint32_t  maxRowLen = 0;
     double    meanRowLen = 0;
@@ -365,11 +366,17 @@ int m_residual(Ctx& c, const Mat& A, const double* b, const double* x, double* r
 int m_residual(Ctx& c, const Mat& A, const float* b, const float* x, float* r,
                const double* xinf);
 int m_transpose(Ctx& c, const Mat& A, Mat& T);                            // CSR -> CSC, exact
-// Builds M.cd16 (16-bit column offsets) when every |col - row| <= 32767; otherwise leaves it
-// null. Synchronises the stream.
+// Builds M.cd16 (16-bit column offsets) when every |col - row| <= 32767 (near16); otherwise
+// leaves it null. Synchronises the stream.
 int m_build_col16(Mat& M, cudaStream_t s);
-// Mat::tileSpan from the row pointers (the block tiles' fit test, csr_tile_rows).
-int m_tile_span(Mat& M, cudaStream_t s);
+// Checks rowPtr and colInd (CheckCSR, src/MATUtil.cxx:110-174: kErrMatData) and fills what a Mat
+// holds beyond its sizes, rowPtr, colInd and val: diagonal, longest row, tile span, 16-bit
+// reach, lanes and, when asked for, the row-class form. Synchronises the stream (upload.cu).
+int m_inspect(Mat& T, bool classes, cudaStream_t s);
+// Orders s after everything enqueued on the legacy default stream so far.
+int after_legacy_stream(cudaStream_t s);
+// cudaMalloc with the spare bytes every matrix array has; kErrAlloc.
+int dmalloc(void** p, size_t bytes);
 // Tile waits that ran out in the kernels of spmv.cu and solvers.cu (bulk copies that never
 // landed).
 unsigned tile_timeouts_spmv();

@@ -1,6 +1,6 @@
-// spmv.cu -- CSRx matrices in HBM: upload and validation, SpMV (MAT::Apply), residual
-// (MAT::Residual), CSR->CSC transpose (MAT::TransInPlace), the lanes-per-row autotuner and
-// the sampled outer product of the adjoint gradient.
+// spmv.cu -- CSRx matrices in HBM: SpMV (MAT::Apply), residual (MAT::Residual), CSR->CSC
+// transpose (MAT::TransInPlace), the lanes-per-row autotuner and the sampled outer product of
+// the adjoint gradient.
 //
 // SpMV mapping: a group of L lanes (L = 1, 2, ..., 32) owns one row; the lanes stride over
 // the row's entries so that a warp reads 32/L consecutive rows' values and column indices
@@ -9,9 +9,6 @@
 // L = 32 the warp-per-row vector kernel; L is chosen from the mean row length or timed.
 #include <algorithm>
 #include <cstdlib>
-#include <cstring>
-#include <map>
-#include <unordered_map>
 #include <vector>
 
 #include "internal.h"
@@ -268,25 +265,6 @@ int m_residual(Ctx& c, const Mat& A, const float* b, const float* x, float* r,
 
 // ---- setup-time kernels ----------------------------------------------------------------
 
-// MAT::FormDiagPtr (MAT.cxx:917-928): first position whose column equals the row; rows
-// without a diagonal keep 0. GetDiag (MAT.cxx:256-267) reads values there (1 if pattern).
-__global__ void k_diag(uint32_t nrow, const uint32_t* __restrict__ rowPtr,
-                       const uint32_t* __restrict__ colInd, const double* __restrict__ val,
-                       uint32_t* __restrict__ diagPtr, double* __restrict__ diag)
-{
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nrow;
-         i += (size_t)gridDim.x * blockDim.x) {
-        uint32_t d = 0;
-        for (uint32_t k = rowPtr[i]; k < rowPtr[i + 1]; ++k)
-            if (colInd[k] == i) {
-                d = k;
-                break;
-            }
-        diagPtr[i] = d;
-        if (diag) diag[i] = val ? val[d] : 1.0;
-    }
-}
-
 __global__ void k_to_f32(size_t n, const double* __restrict__ a, float* __restrict__ b)
 {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -294,357 +272,7 @@ __global__ void k_to_f32(size_t n, const double* __restrict__ a, float* __restri
         b[i] = (float)a[i];
 }
 
-static int dmalloc(void** p, size_t bytes)
-{
-    // 32 spare bytes keep vectorised/bulk tail accesses inside the allocation (the warp
-    // tiles' 16-byte loads read up to 3 entries past the last one)
-    cudaError_t e = cudaMalloc(p, bytes + 32);
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        cudaGetLastError();
-        return kErrAlloc;
-    }
-    return kOk;
-}
-
-void m_free(Mat& M)
-{
-    cudaFree(M.rowPtr);
-    cudaFree(M.colInd);
-    cudaFree(M.diagPtr);
-    cudaFree(M.val);
-    cudaFree(M.val32);
-    cudaFree(M.diag);
-    cudaFree(M.rcCls);
-    cudaFree(M.rcOff);
-    cudaFree(M.rcDelta);
-    cudaFree(M.rcVal);
-    cudaFree(M.rcVal32);
-    cudaFree(M.skMask);
-    cudaFree(M.cd16);
-    M = Mat();
-}
-
-// ---- 16-bit column offsets ------------------------------------------------------------------
-// cd16[k] = colInd[k] - row(k) when every entry is within 32,767 columns of its row (banded
-// FDM/FEM matrices up to bandwidths of 32,767, the 128^3 Laplacian's is 16,384): the
-// thread-per-row kernels then read 2 bytes per entry instead of 4 and form the column by one
-// add, with the entries and their order unchanged -- the same results bit for bit.
-__global__ void k_col16(uint32_t nrow, const uint32_t* __restrict__ rowPtr,
-                        const uint32_t* __restrict__ colInd, int16_t* __restrict__ out,
-                        unsigned* __restrict__ outOfRange)
-{
-    for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrow;
-         r += (size_t)gridDim.x * blockDim.x) {
-        bool bad = false;
-        for (uint32_t k = rowPtr[r]; k < rowPtr[r + 1]; ++k) {
-            const long long d = (long long)colInd[k] - (long long)r;
-            if (d < -32767 || d > 32767)
-                bad = true;
-            else
-                out[k] = (int16_t)d;
-        }
-        if (bad) atomicOr(outOfRange, 1u);
-    }
-}
-
-int m_build_col16(Mat& M, cudaStream_t s)
-{
-    if (M.grid || M.nnz == 0 || !M.colInd || M.cd16) return kOk;
-    int16_t* out = nullptr;
-    unsigned* flag = nullptr;
-    int e;
-    if ((e = dmalloc((void**)&out, ((size_t)M.nnz + 8) * 2)) ||
-        (e = dmalloc((void**)&flag, 4))) {
-        cudaFree(out);
-        return e;
-    }
-    FB_CUDA(cudaMemsetAsync(flag, 0, 4, s));
-    k_col16<<<std::max(1, std::min(ceil_div(M.nrow, kBlock), 148 * 8)), kBlock, 0, s>>>(
-        M.nrow, M.rowPtr, M.colInd, out, flag);
-    FB_CUDA(cudaGetLastError());
-    unsigned h = 0;
-    FB_CUDA(cudaMemcpyAsync(&h, flag, 4, cudaMemcpyDeviceToHost, s));
-    FB_CUDA(cudaStreamSynchronize(s));
-    cudaFree(flag);
-    if (h) {
-        cudaFree(out); // some entry is too far from its row: keep 32-bit columns only
-        return kOk;
-    }
-    M.cd16 = out;
-    return kOk;
-}
-
-// The most entries any 256-row tile covers once widened to multiples of 4: the block tiles
-// of csr_tile_rows take a matrix only when every tile fits a stage.
-__global__ void k_tile_span(uint32_t nrow, const uint32_t* __restrict__ rowPtr,
-                            unsigned* __restrict__ span)
-{
-    const size_t ntiles = ((size_t)nrow + kTileRows - 1) / kTileRows;
-    unsigned m = 0;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < ntiles;
-         t += (size_t)gridDim.x * blockDim.x) {
-        const size_t r0 = t * kTileRows;
-        const size_t r1 = r0 + kTileRows < nrow ? r0 + kTileRows : nrow;
-        const unsigned long long a = rowPtr[r0] & ~3u;
-        const unsigned long long ar = ((unsigned long long)rowPtr[r1] + 3) & ~3ull;
-        const unsigned long long w = ar - a;
-        m = max(m, (unsigned)(w < 0xffffffffull ? w : 0xffffffffull));
-    }
-    atomicMax(span, m);
-}
-
-int m_tile_span(Mat& M, cudaStream_t s)
-{
-    M.tileSpan = 0;
-    if (M.grid || M.nrow == 0 || !M.rowPtr) return kOk;
-    unsigned* d = nullptr;
-    int e;
-    if ((e = dmalloc((void**)&d, 4))) return e;
-    FB_CUDA(cudaMemsetAsync(d, 0, 4, s));
-    const int tiles = ceil_div(M.nrow, (int)kTileRows);
-    k_tile_span<<<std::max(1, std::min(ceil_div(tiles, kBlock), 148 * 8)), kBlock, 0, s>>>(
-        M.nrow, M.rowPtr, d);
-    FB_CUDA(cudaGetLastError());
-    unsigned h = 0;
-    FB_CUDA(cudaMemcpyAsync(&h, d, 4, cudaMemcpyDeviceToHost, s));
-    FB_CUDA(cudaStreamSynchronize(s));
-    cudaFree(d);
-    M.tileSpan = h;
-    return kOk;
-}
-
 unsigned tile_timeouts_spmv() { return tile_timeouts(); }
-
-// ---- row classes ------------------------------------------------------------------------
-// A row's class is its length, its column offsets col - row and its values (bit patterns),
-// in CSR order. Constant-coefficient stencil matrices have a handful of classes (interior,
-// faces, edges, corners), so the SpMV streams a 2-byte class id per row instead of 8 to 12
-// bytes per entry. The table is built only when it stays small against the matrix.
-
-constexpr uint32_t kRcMaxClasses = 4096;
-constexpr uint32_t kRcMaxRowLen = 64;
-
-struct RowClasses {
-    std::vector<uint16_t> cls;
-    std::vector<uint32_t> off{0};
-    std::vector<int32_t>  delta;
-    std::vector<double>   val;
-};
-
-static bool build_row_classes(uint32_t nrow, const uint32_t* rp, const uint32_t* ci,
-                              const double* v, RowClasses& R)
-{
-    if (nrow == 0 || nrow > 0x7fffffffu) return false;
-    const size_t nnz = rp[nrow];
-    const size_t maxEntries = std::max<size_t>(64, nnz / 8);
-    R.cls.resize(nrow);
-    std::unordered_map<uint64_t, std::vector<uint32_t>> buckets;
-    for (uint32_t row = 0; row < nrow; ++row) {
-        const uint32_t b = rp[row], e = rp[row + 1], len = e - b;
-        if (len > kRcMaxRowLen) return false;
-        uint64_t h = 1469598103934665603ull ^ len;
-        for (uint32_t k = b; k < e; ++k) {
-            const uint64_t d = (uint64_t)(uint32_t)(int32_t)((int64_t)ci[k] - (int64_t)row);
-            uint64_t bits;
-            std::memcpy(&bits, &v[k], 8);
-            h = (h ^ d) * 1099511628211ull;
-            h = (h ^ bits) * 1099511628211ull;
-        }
-        auto& cand = buckets[h];
-        uint32_t id = 0xffffffffu;
-        for (uint32_t c : cand) {
-            const uint32_t cb = R.off[c], ce = R.off[c + 1];
-            if (ce - cb != len) continue;
-            bool same = true;
-            for (uint32_t k = 0; k < len && same; ++k)
-                same = R.delta[cb + k] == (int32_t)((int64_t)ci[b + k] - (int64_t)row) &&
-                       std::memcmp(&R.val[cb + k], &v[b + k], 8) == 0;
-            if (same) {
-                id = c;
-                break;
-            }
-        }
-        if (id == 0xffffffffu) {
-            id = (uint32_t)R.off.size() - 1;
-            if (id >= kRcMaxClasses || R.delta.size() + len > maxEntries) return false;
-            for (uint32_t k = b; k < e; ++k) {
-                const int64_t d = (int64_t)ci[k] - (int64_t)row;
-                if (d < INT32_MIN || d > INT32_MAX) return false;
-                R.delta.push_back((int32_t)d);
-                R.val.push_back(v[k]);
-            }
-            R.off.push_back((uint32_t)R.delta.size());
-            cand.push_back(id);
-        }
-        R.cls[row] = (uint16_t)id;
-    }
-    return true;
-}
-
-// Stencil masks: when the classes' column offsets, taken together, are at most kMaxStencil
-// distinct values each carrying one value (bitwise) wherever it occurs, and every class
-// lists its offsets in ascending order (the CSR order), each row is a bit mask over that
-// sorted offset list. Summing the present entries in list order is the CSR order.
-static bool build_stencil_masks(const RowClasses& R, Mat& T, std::vector<uint16_t>& rowMask)
-{
-    std::map<int32_t, double> U;
-    const uint32_t C = (uint32_t)R.off.size() - 1;
-    for (uint32_t c = 0; c < C; ++c)
-        for (uint32_t k = R.off[c]; k < R.off[c + 1]; ++k) {
-            if (k > R.off[c] && R.delta[k] <= R.delta[k - 1]) return false;
-            auto it = U.find(R.delta[k]);
-            if (it == U.end())
-                U.emplace(R.delta[k], R.val[k]);
-            else if (std::memcmp(&it->second, &R.val[k], 8) != 0)
-                return false;
-        }
-    if (U.empty() || U.size() > (size_t)kMaxStencil) return false;
-    std::map<int32_t, int> pos;
-    T.skLen = 0;
-    for (auto& kv : U) {
-        pos[kv.first] = (int)T.skLen;
-        T.skDelta[T.skLen] = kv.first;
-        T.skVal[T.skLen] = kv.second;
-        ++T.skLen;
-    }
-    std::vector<uint16_t> cm(C, 0);
-    for (uint32_t c = 0; c < C; ++c)
-        for (uint32_t k = R.off[c]; k < R.off[c + 1]; ++k) cm[c] |= (uint16_t)(1u << pos[R.delta[k]]);
-    rowMask.resize(R.cls.size());
-    for (size_t r = 0; r < R.cls.size(); ++r) rowMask[r] = cm[R.cls[r]];
-    return true;
-}
-
-static int upload_row_classes(Mat& T, const RowClasses& R, cudaStream_t s)
-{
-    const uint32_t C = (uint32_t)R.off.size() - 1, E = (uint32_t)R.delta.size();
-    int e;
-    if ((e = dmalloc((void**)&T.rcCls, (size_t)T.nrow * 2 + 16)) ||
-        (e = dmalloc((void**)&T.rcOff, ((size_t)C + 1) * 4)) ||
-        (e = dmalloc((void**)&T.rcDelta, (size_t)E * 4 + 16)) ||
-        (e = dmalloc((void**)&T.rcVal, (size_t)E * 8 + 16)))
-        return e;
-    FB_CUDA(cudaMemcpyAsync(T.rcCls, R.cls.data(), (size_t)T.nrow * 2, cudaMemcpyHostToDevice, s));
-    FB_CUDA(cudaMemcpyAsync(T.rcOff, R.off.data(), ((size_t)C + 1) * 4, cudaMemcpyHostToDevice, s));
-    FB_CUDA(cudaMemcpyAsync(T.rcDelta, R.delta.data(), (size_t)E * 4, cudaMemcpyHostToDevice, s));
-    FB_CUDA(cudaMemcpyAsync(T.rcVal, R.val.data(), (size_t)E * 8, cudaMemcpyHostToDevice, s));
-    std::vector<uint16_t> rowMask;
-    if (build_stencil_masks(R, T, rowMask)) {
-        if ((e = dmalloc((void**)&T.skMask, (size_t)T.nrow * 2 + 16))) return e;
-        FB_CUDA(cudaMemcpyAsync(T.skMask, rowMask.data(), (size_t)T.nrow * 2,
-                                cudaMemcpyHostToDevice, s));
-    } else {
-        T.skLen = 0;
-    }
-    FB_CUDA(cudaStreamSynchronize(s)); // the host vectors die with the caller
-    T.rcClasses = C;
-    T.rcEntries = E;
-    T.rcOn = true;
-    return kOk;
-}
-
-// CheckCSR (src/MATUtil.cxx:110-174) on host arrays: sizes, monotone row pointers, column
-// indices in range. A failed check returns ERROR_MAT_DATA and uploads nothing, so no kernel
-// ever indexes outside the matrix.
-static int check_csr(uint32_t nrow, uint32_t mcol, uint32_t nnz, const uint32_t* rowPtr,
-                     const uint32_t* colInd)
-{
-    if (nrow == 0 || mcol == 0 || nnz == 0) return kErrMatSize;
-    if (rowPtr[0] != 0 || rowPtr[nrow] != nnz) return kErrMatData;
-    for (uint32_t j = 0; j < nrow; ++j)
-        if (rowPtr[j] > rowPtr[j + 1]) return kErrMatData;
-    for (uint32_t k = 0; k < nnz; ++k)
-        if (colInd[k] >= mcol) return kErrMatData;
-    return kOk;
-}
-
-int m_upload(Mat& M, uint32_t nrow, uint32_t mcol, uint32_t nnz, const uint32_t* rowPtr,
-             const uint32_t* colInd, const double* values, bool hostPtrs, cudaStream_t s)
-{
-    std::vector<uint32_t> hrp, hci;
-    const uint32_t* crp = rowPtr;
-    const uint32_t* cci = colInd;
-    if (!hostPtrs) {
-        // device arrays: validate a host copy before any kernel touches them
-        hrp.resize((size_t)nrow + 1);
-        hci.resize(nnz);
-        FB_CUDA(cudaMemcpy(hrp.data(), rowPtr, hrp.size() * 4, cudaMemcpyDeviceToHost));
-        FB_CUDA(cudaMemcpy(hci.data(), colInd, hci.size() * 4, cudaMemcpyDeviceToHost));
-        crp = hrp.data();
-        cci = hci.data();
-    }
-    int e = check_csr(nrow, mcol, nnz, crp, cci);
-    if (e) return e;
-    uint32_t maxLen = 0;
-    for (uint32_t j = 0; j < nrow; ++j) maxLen = std::max(maxLen, crp[j + 1] - crp[j]);
-
-    Mat T;
-    T.nrow = nrow;
-    T.mcol = mcol;
-    T.nnz = nnz;
-    T.maxRowLen = maxLen;
-    T.meanRowLen = (double)nnz / nrow;
-    cudaGetDevice(&T.dev);
-    const cudaMemcpyKind kind = hostPtrs ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
-    if ((e = dmalloc((void**)&T.rowPtr, ((size_t)nrow + 1) * 4)) ||
-        (e = dmalloc((void**)&T.colInd, (size_t)nnz * 4)) ||
-        (e = dmalloc((void**)&T.diagPtr, (size_t)nrow * 4)) ||
-        (e = dmalloc((void**)&T.diag, (size_t)nrow * 8)) ||
-        (values && (e = dmalloc((void**)&T.val, (size_t)nnz * 8)))) {
-        m_free(T);
-        return e;
-    }
-    FB_CUDA(cudaMemcpyAsync(T.rowPtr, rowPtr, ((size_t)nrow + 1) * 4, kind, s));
-    FB_CUDA(cudaMemcpyAsync(T.colInd, colInd, (size_t)nnz * 4, kind, s));
-    if (values) FB_CUDA(cudaMemcpyAsync(T.val, values, (size_t)nnz * 8, kind, s));
-    k_diag<<<std::max(1, std::min(ceil_div(nrow, kBlock), 148 * 8)), kBlock, 0, s>>>(
-        nrow, T.rowPtr, T.colInd, T.val, T.diagPtr, T.diag);
-    FB_CUDA(cudaGetLastError());
-    T.lanes = lanes_for(T.meanRowLen);
-    std::vector<double> hv;
-    const double* cv = values;
-    if (values && !hostPtrs) {
-        hv.resize(nnz);
-        FB_CUDA(cudaMemcpy(hv.data(), values, (size_t)nnz * 8, cudaMemcpyDeviceToHost));
-        cv = hv.data();
-    }
-    if (values && nrow == mcol && nrow > 0) { // one diagonal value (bitwise) in every row?
-        bool same = true, first = true;
-        double d0 = 0.0;
-        for (uint32_t r = 0; r < nrow && same; ++r) {
-            bool found = false;
-            for (uint32_t k = crp[r]; k < crp[r + 1]; ++k)
-                if (cci[k] == r) {
-                    found = true;
-                    if (first) {
-                        d0 = cv[k];
-                        first = false;
-                    } else if (std::memcmp(&cv[k], &d0, 8) != 0) {
-                        same = false;
-                    }
-                    break;
-                }
-            same = same && found;
-        }
-        T.diagConst = same && d0 != 0.0;
-        T.diagValue = d0;
-    }
-    if (values && T.lanes == 1) {
-        RowClasses R;
-        if (build_row_classes(nrow, crp, cci, cv, R) && (e = upload_row_classes(T, R, s))) {
-            m_free(T);
-            return e;
-        }
-    }
-    if ((e = m_build_col16(T, s)) || (e = m_tile_span(T, s))) {
-        m_free(T);
-        return e;
-    }
-    FB_CUDA(cudaStreamSynchronize(s));
-    M = T;
-    return kOk;
-}
 
 int Mat::ensure32(cudaStream_t s)
 {
@@ -788,8 +416,6 @@ int m_transpose(Ctx& c, const Mat& A, Mat& T)
     int e;
     if ((e = dmalloc((void**)&R.rowPtr, ((size_t)m + 1) * 4)) ||
         (e = dmalloc((void**)&R.colInd, (size_t)nnz * 4)) ||
-        (e = dmalloc((void**)&R.diagPtr, (size_t)m * 4)) ||
-        (e = dmalloc((void**)&R.diag, (size_t)m * 8)) ||
         (A.val && (e = dmalloc((void**)&R.val, (size_t)nnz * 8))) ||
         (e = dmalloc((void**)&cnt, (size_t)m * 4)) || (e = dmalloc((void**)&fill, (size_t)m * 4)) ||
         (e = dmalloc((void**)&pos, (size_t)nnz * 4)) ||
@@ -812,22 +438,19 @@ int m_transpose(Ctx& c, const Mat& A, Mat& T)
     k_row_of<<<gr, kBlock, 0, s>>>(n, A.rowPtr, rowOf);
     k_scatter_pos<<<gn, kBlock, 0, s>>>(nnz, A.colInd, R.rowPtr, fill, pos);
     k_sort_gather<<<gm, kBlock, 0, s>>>(m, R.rowPtr, pos, rowOf, A.val, R.colInd, R.val);
-    k_diag<<<gm, kBlock, 0, s>>>(m, R.rowPtr, R.colInd, R.val, R.diagPtr, R.diag);
     FB_CUDA(cudaGetLastError());
-    FB_CUDA(cudaStreamSynchronize(s));
+    e = m_inspect(R, false, s);
     cudaFree(cnt);
     cudaFree(fill);
     cudaFree(pos);
     cudaFree(rowOf);
-    R.meanRowLen = (double)nnz / m;
-    std::vector<uint32_t> hrp((size_t)m + 1);
-    FB_CUDA(cudaMemcpy(hrp.data(), R.rowPtr, hrp.size() * 4, cudaMemcpyDeviceToHost));
-    for (uint32_t j = 0; j < m; ++j) R.maxRowLen = std::max(R.maxRowLen, hrp[j + 1] - hrp[j]);
-    R.lanes = A.lanes;
-    if ((e = m_build_col16(R, s)) || (e = m_tile_span(R, s))) {
+    if (e) {
         m_free(R);
         return e;
     }
+    R.diagConst = false; // the solvers on a transpose read its diagonal vector
+    R.diagValue = 0.0;
+    R.lanes = A.lanes;
     T = R;
     return kOk;
 }

@@ -258,10 +258,10 @@ int fasp_gpu_mat_set_lanes(fasp_gpu_mat A, int lanes);
 int fasp_gpu_mat_set_rowclass(fasp_gpu_mat A, int mode);
 int fasp_gpu_mat_rowclass_info(fasp_gpu_mat A, int* mode, uint32_t* classes, uint32_t* entries,
                                uint32_t* stencil);
-/* 16-bit column offsets of the CSR form (opt-in): built at upload (and for transposes) when
+/* 16-bit column offsets of the CSR form (opt-in): available (built = 1, transposes too) when
  * every stored entry lies within 32,767 columns of its row -- banded FDM/FEM matrices, the
- * 128^3 Laplacian's bandwidth is 16,384 -- as colInd[k] - row; with on = 1 the
- * thread-per-row kernels (lanes = 1) stream 2 bytes per entry for the columns instead of 4
+ * 128^3 Laplacian's bandwidth is 16,384 -- as colInd[k] - row, formed when first turned
+ * on; with on = 1 the thread-per-row kernels (lanes = 1) stream 2 bytes per entry for the columns instead of 4
  * and form each column by one add. The entries and their order are unchanged, so results
  * are bit-identical. Off by default: on B200 the 2-byte loads measured slower than the
  * 4-byte colInd (128^3 CSR CG, FP32 iterations 17.4 against 14.9 ms). Set it before a
