@@ -637,10 +637,7 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
     h->nrhs = nrhs;
     const size_t vN = (size_t)nrhs * N;
     auto dm = [&](void** p, size_t bytes) {
-        if (!e && cudaMalloc(p, bytes + 16) != cudaSuccess) {
-            cudaGetLastError();
-            e = kErrAlloc;
-        }
+        if (!e) e = dev_alloc_bytes(p, bytes + 16, h->c.stream);
     };
     dm((void**)&h->sysRow, (count + 1) * 4);
     dm((void**)&h->order, count * 4);
@@ -670,8 +667,8 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
         std::stable_sort(ord.begin(), ord.end(), [&](uint32_t a, uint32_t b) {
             return hs[a + 1] - hs[a] > hs[b + 1] - hs[b];
         });
-        cudaMemcpy(h->sysRow, hs.data(), (count + 1) * 4, cudaMemcpyHostToDevice);
-        cudaMemcpy(h->order, ord.data(), count * 4, cudaMemcpyHostToDevice);
+        cudaMemcpyAsync(h->sysRow, hs.data(), (count + 1) * 4, cudaMemcpyHostToDevice, h->c.stream);
+        cudaMemcpyAsync(h->order, ord.data(), count * 4, cudaMemcpyHostToDevice, h->c.stream);
         batch_dinv<<<std::max(1, std::min(ceil_div(N, 256), 148 * 8)), 256, 0, h->c.stream>>>(
             N, h->M.diag, h->dinv, h->dinv32);
         if (cudaStreamSynchronize(h->c.stream) != cudaSuccess) e = kErrCuda;
@@ -687,14 +684,14 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
 int fasp_gpu_batch_destroy(fasp_gpu_batch h)
 {
     if (!h) return kOk;
-    cudaStreamSynchronize(h->c.stream);
+    cudaDeviceSynchronize();
     m_free(h->M);
     for (void* p : {(void*)h->sysRow, (void*)h->order, (void*)h->dinv, (void*)h->dinv32,
                     (void*)h->r64, (void*)h->z64, (void*)h->p0, (void*)h->p1, (void*)h->q64,
                     (void*)h->b32, (void*)h->x32, (void*)h->r32, (void*)h->z32,
                     (void*)h->p032, (void*)h->p132, (void*)h->q32, (void*)h->rnorm,
                     (void*)h->resRel, (void*)h->iters, (void*)h->queue})
-        cudaFree(p);
+        dev_free(p);
     h->c.destroy();
     delete h;
     return kOk;

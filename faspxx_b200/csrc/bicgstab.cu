@@ -560,17 +560,17 @@ int BiEngine<T>::init(Ctx* ctx, const Mat* M, int jac, const T* dinvv, bool grap
     const size_t bytes = ((size_t)n + 4) * sizeof(T);
     T** vecs[] = {&x, &rj, &r0s, &pj2[0], &pj2[1], &ptmp2[0], &ptmp2[1], &sj, &stmp};
     for (T** v : vecs)
-        if (cudaMalloc(v, bytes) != cudaSuccess) {
-            cudaGetLastError();
+        if (dev_alloc(v, bytes, c->stream)) {
             destroy();
             return kErrAlloc;
         }
-    if (cudaMalloc(&ctl, sizeof(BiCtl)) || cudaMallocHost(&hctl, sizeof(BiCtl)) ||
-        cudaMallocHost(&hstatus, sizeof(int))) {
-        cudaGetLastError();
+    if (dev_alloc(&ctl, sizeof(BiCtl), c->stream) || !(hctl = (BiCtl*)pinned_get())) {
         destroy();
         return kErrAlloc;
     }
+    // the status word follows the control block in its page-locked block
+    static_assert(sizeof(BiCtl) + sizeof(int) <= kPinnedBlock, "one page-locked block");
+    hstatus = (int*)(hctl + 1);
     std::memset(hctl, 0, sizeof(BiCtl));
     hctl->histScale = 1.0;
     if (useGraph) {
@@ -594,13 +594,13 @@ void BiEngine<T>::destroy()
     gexec = nullptr;
     T** vecs[] = {&x, &rj, &r0s, &pj2[0], &pj2[1], &ptmp2[0], &ptmp2[1], &sj, &stmp};
     for (T** v : vecs) {
-        cudaFree(*v);
+        dev_free(*v);
         *v = nullptr;
     }
-    cudaFree(ctl);
+    dev_free(ctl);
     ctl = nullptr;
-    if (hctl) cudaFreeHost(hctl);
-    if (hstatus) cudaFreeHost(hstatus);
+    pinned_put(hctl);
+    
     hctl = nullptr;
     hstatus = nullptr;
 }

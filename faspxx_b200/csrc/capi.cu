@@ -8,47 +8,6 @@ using namespace fb;
 
 namespace fb {
 
-int Ctx::init(int device)
-{
-    dev = device;
-    if (cudaSetDevice(device) != cudaSuccess) {
-        cudaGetLastError();
-        return kErrNoDevice;
-    }
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device);
-    nsm = v > 0 ? v : 148;
-    if (nsm * 16 > kMaxGrid) nsm = kMaxGrid / 16;
-    FB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    ownStream = true;
-    FB_CUDA(cudaMalloc(&red.partials, sizeof(double) * kMaxRedValues * kMaxGrid));
-    FB_CUDA(cudaMalloc(&red.ticket, sizeof(unsigned) * 4));
-    FB_CUDA(cudaMemset(red.ticket, 0, sizeof(unsigned) * 4));
-    FB_CUDA(cudaMalloc(&dslot, sizeof(double) * kSlots));
-    FB_CUDA(cudaMemset(dslot, 0, sizeof(double) * kSlots));
-    FB_CUDA(cudaMallocHost(&hslot, sizeof(double) * kSlots));
-    return kOk;
-}
-
-void Ctx::destroy()
-{
-    if (stream) cudaStreamSynchronize(stream);
-    for (cudaEvent_t& ev : joinEv)
-        if (ev) {
-            cudaEventDestroy(ev);
-            ev = nullptr;
-        }
-    cudaFree(red.partials);
-    cudaFree(red.ticket);
-    cudaFree(dslot);
-    if (hslot) cudaFreeHost(hslot);
-    if (ownStream && stream) cudaStreamDestroy(stream);
-    red = Scratch{nullptr, nullptr};
-    dslot = nullptr;
-    hslot = nullptr;
-    stream = nullptr;
-}
-
 int Ctx::join_from(cudaStream_t user)
 {
     if (user == stream) return kOk;
@@ -215,8 +174,12 @@ int fasp_gpu_malloc(void** p, size_t bytes)
 {
     if (cudaMalloc(p, bytes) != cudaSuccess) {
         cudaGetLastError();
-        *p = nullptr;
-        return kErrAlloc;
+        dev_trim(); // what the pool keeps may be what is missing
+        if (cudaMalloc(p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            *p = nullptr;
+            return kErrAlloc;
+        }
     }
     return kOk;
 }
@@ -345,7 +308,7 @@ int fasp_gpu_mat_add(double a, fasp_gpu_mat A, double b, fasp_gpu_mat B, fasp_gp
 int fasp_gpu_mat_destroy(fasp_gpu_mat A)
 {
     if (!A) return kOk;
-    cudaStreamSynchronize(A->c.stream);
+    cudaDeviceSynchronize(); // whichever streams still use the arrays
     if (A->T) fasp_gpu_mat_destroy(A->T);
     m_free(A->M);
     A->c.destroy();
@@ -751,10 +714,10 @@ int fasp_gpu_solver_solve_host(fasp_gpu_solver s, const double* b, double* x, fa
     const size_t bytes = (size_t)S.n * 8;
     if (!S.hostB) {
         // device staging for the host entry point, kept for the solver's lifetime
-        if (cudaMalloc(&S.hostB, bytes + 16) || cudaMalloc(&S.hostX, bytes + 16)) {
-            cudaGetLastError();
-            return kErrAlloc;
-        }
+        int e;
+        if ((e = dev_alloc(&S.hostB, bytes + 16, S.c.stream)) ||
+            (e = dev_alloc(&S.hostX, bytes + 16, S.c.stream)))
+            return e;
     }
     int e = kOk;
     if (cudaMemcpyAsync(S.hostB, b, bytes, cudaMemcpyHostToDevice, S.c.stream) ||

@@ -1728,14 +1728,17 @@ int CGEngine<T>::init(Ctx* ctx, const Mat* M, int jac, const T* dinvv, bool grap
     dinv = dinvv;
     useGraph = graph;
     const size_t bytes = ((size_t)n + 4) * sizeof(T);
-    if (cudaMalloc(&x, bytes) || cudaMalloc(&r, bytes) || cudaMalloc(&q, bytes) ||
-        cudaMalloc(&P0, bytes) || cudaMalloc(&P1, bytes) ||
-        (jacobi && cudaMalloc(&z, bytes)) || cudaMalloc(&ctl, sizeof(CGCtl)) ||
-        cudaMallocHost(&hctl, sizeof(CGCtl)) || cudaMallocHost(&hstatus, sizeof(int))) {
-        cudaGetLastError();
+    cudaStream_t s = c->stream;
+    if (dev_alloc(&x, bytes, s) || dev_alloc(&r, bytes, s) || dev_alloc(&q, bytes, s) ||
+        dev_alloc(&P0, bytes, s) || dev_alloc(&P1, bytes, s) ||
+        (jacobi && dev_alloc(&z, bytes, s)) || dev_alloc(&ctl, sizeof(CGCtl), s) ||
+        !(hctl = (CGCtl*)pinned_get())) {
         destroy();
         return kErrAlloc;
     }
+    // the status word follows the control block in its page-locked block
+    static_assert(sizeof(CGCtl) + sizeof(int) <= kPinnedBlock, "one page-locked block");
+    hstatus = (int*)(hctl + 1);
     if (!jacobi) z = r;
     std::memset(hctl, 0, sizeof(CGCtl));
     hctl->histScale = 1.0;
@@ -1825,10 +1828,7 @@ int CGEngine<T>::init(Ctx* ctx, const Mat* M, int jac, const T* dinvv, bool grap
         }
         if (cgrid > 0) {
             // the control flow needs no barrier state, but the kernel takes the pointer
-            if (cudaMalloc(&bar, sizeof(GridBar)) != cudaSuccess) {
-                cudaGetLastError();
-                return kErrAlloc;
-            }
+            if (dev_alloc(&bar, sizeof(GridBar), c->stream)) return kErrAlloc;
             FB_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), c->stream));
             cluster = persistent = true;
             return kOk;
@@ -1847,10 +1847,7 @@ int CGEngine<T>::init(Ctx* ctx, const Mat* M, int jac, const T* dinvv, bool grap
         pgrid = nb * c->nsm;
         if (pgrid > kMaxGrid) pgrid = kMaxGrid;
         if (coop && nb > 0) {
-            if (cudaMalloc(&bar, sizeof(GridBar)) != cudaSuccess) {
-                cudaGetLastError();
-                return kErrAlloc;
-            }
+            if (dev_alloc(&bar, sizeof(GridBar), c->stream)) return kErrAlloc;
             FB_CUDA(cudaMemsetAsync(bar, 0, sizeof(GridBar), c->stream));
             persistent = true;
         }
@@ -1931,19 +1928,19 @@ void CGEngine<T>::destroy()
 {
     if (gexec) cudaGraphExecDestroy(gexec);
     gexec = nullptr;
-    cudaFree(x);
-    cudaFree(r);
-    cudaFree(q);
-    cudaFree(P0);
-    cudaFree(P1);
-    if (jacobi) cudaFree(z);
-    cudaFree(ctl);
-    cudaFree(bar);
+    dev_free(x);
+    dev_free(r);
+    dev_free(q);
+    dev_free(P0);
+    dev_free(P1);
+    if (jacobi) dev_free(z);
+    dev_free(ctl);
+    dev_free(bar);
     bar = nullptr;
     persistent = cluster = dsmem = false;
     cgrid = 0;
-    if (hctl) cudaFreeHost(hctl);
-    if (hstatus) cudaFreeHost(hstatus);
+    pinned_put(hctl);
+    
     x = r = z = q = P0 = P1 = nullptr;
     ctl = nullptr;
     hctl = nullptr;

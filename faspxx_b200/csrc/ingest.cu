@@ -189,7 +189,7 @@ int m_from_coo(Ctx& c, uint32_t nrow, uint32_t mcol, uint32_t nnz, const uint32_
     if (!rowInd || !colInd || !values) return kErrInputPar;
     if (nrow == 0 || mcol == 0 || nnz == 0) return kErrMatSize;
     cudaStream_t s = c.stream;
-    Tmp t;
+    Tmp t(s);
     int e;
     const uint32_t *ri = nullptr, *ci = nullptr;
     const double* va = nullptr;
@@ -224,7 +224,7 @@ int m_from_csr_raw(Ctx& c, uint32_t nrow, uint32_t mcol, uint32_t nnz, const uin
     if (!rowPtr || !colInd || !values) return kErrInputPar;
     if (nrow == 0 || mcol == 0 || nnz == 0) return kErrMatSize;
     cudaStream_t s = c.stream;
-    Tmp t;
+    Tmp t(s);
     int e;
     const uint32_t *rpIn = nullptr, *ci = nullptr;
     const double* va = nullptr;

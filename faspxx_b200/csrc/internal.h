@@ -92,7 +92,25 @@ __device__ __forceinline__ double eval(const Scal& s)
 
 constexpr int kSlots = 256;
 
-// Execution context: one stream, its reduction scratch and scalar slots.
+// ---- memory (mem.cu) --------------------------------------------------------------------
+// Device memory from the current device's pool, ready for work on s (for other streams after
+// s has been waited for): kErrAlloc. dev_free takes it back at once, so whoever frees has
+// waited for the work that uses it.
+int dev_alloc_bytes(void** p, size_t bytes, cudaStream_t s);
+template <typename T>
+inline int dev_alloc(T** p, size_t bytes, cudaStream_t s)
+{
+    return dev_alloc_bytes(reinterpret_cast<void**>(p), bytes, s);
+}
+void dev_free(void* p);
+void dev_trim(); // the current device's free pool memory goes back to the device
+// Page-locked host blocks of kPinnedBlock bytes, zeroed; null when there are none.
+constexpr size_t kPinnedBlock = 4096;
+void* pinned_get();
+void  pinned_put(void* p);
+
+// Execution context: one stream, its reduction scratch and scalar slots; init takes an idle
+// one where there is one, destroy leaves it for the next (mem.cu).
 struct Ctx {
     int          dev = 0;
     int          nsm = 148;
@@ -375,8 +393,8 @@ int m_build_col16(Mat& M, cudaStream_t s);
 int m_inspect(Mat& T, bool classes, cudaStream_t s);
 // Orders s after everything enqueued on the legacy default stream so far.
 int after_legacy_stream(cudaStream_t s);
-// cudaMalloc with the spare bytes every matrix array has; kErrAlloc.
-int dmalloc(void** p, size_t bytes);
+// dev_alloc with the spare bytes every matrix array has.
+int dmalloc(void** p, size_t bytes, cudaStream_t s);
 // Tile waits that ran out in the kernels of spmv.cu and solvers.cu (bulk copies that never
 // landed).
 unsigned tile_timeouts_spmv();

@@ -20,24 +20,25 @@ constexpr int      kSegMax = 4096;           // keys one block sorts in shared m
 constexpr int      kSegThreads = 512;
 constexpr uint64_t kPad = ~0ull;
 
-// Device memory released when the conversion returns (cudaFree waits for the device).
+// Device memory of one conversion on stream s, released when it returns (every conversion
+// has waited for its stream by then; a failed one waits here).
 struct Tmp {
+    cudaStream_t       s;
     std::vector<void*> ptrs;
+    explicit Tmp(cudaStream_t st) : s(st) {}
+    Tmp(const Tmp&) = delete;
+    Tmp& operator=(const Tmp&) = delete;
     ~Tmp()
     {
-        for (void* p : ptrs) cudaFree(p);
+        cudaStreamSynchronize(s);
+        for (void* p : ptrs) dev_free(p);
     }
     template <typename T>
     int get(T** p, size_t count)
     {
-        *p = nullptr;
-        if (cudaMalloc((void**)p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
-            *p = nullptr;
-            return kErrAlloc;
-        }
-        ptrs.push_back(*p);
-        return kOk;
+        const int e = dev_alloc(p, std::max<size_t>(count, 1) * sizeof(T), s);
+        if (!e) ptrs.push_back(*p);
+        return e;
     }
 };
 

@@ -192,13 +192,13 @@ int Pcd::setup(Ctx& c, const Mat* M, int t, double w, const fasp_gpu_params& p)
     A = M;
     if (type != 1) return kOk;
     const size_t n = M->nrow;
-    if (cudaMalloc(&dinv, (n + 2) * 8) || cudaMalloc(&dinv32, (n + 4) * 4) ||
-        cudaMalloc(&work, (n + 2) * 8)) {
-        cudaGetLastError();
-        return kErrAlloc;
-    }
+    int e;
+    if ((e = dev_alloc(&dinv, (n + 2) * 8, c.stream)) ||
+        (e = dev_alloc(&dinv32, (n + 4) * 4, c.stream)) ||
+        (e = dev_alloc(&work, (n + 2) * 8, c.stream)))
+        return e;
     // Jacobi::Setup: GetDiag, Reciprocal, Scale(weight) (Iter.cxx:45-47)
-    int e = v_recip_scale(c, M->nrow, weight, M->diag, dinv);
+    e = v_recip_scale(c, M->nrow, weight, M->diag, dinv);
     if (e) return e;
     return to32(c, M->nrow, dinv, dinv32);
 }
@@ -213,10 +213,10 @@ void Pcd::destroy()
         pcd_mg_free(mg);
         mg = nullptr;
     }
-    cudaFree(dinv);
-    cudaFree(dinv32);
-    cudaFree(work);
-    cudaFree(work32);
+    dev_free(dinv);
+    dev_free(dinv32);
+    dev_free(work);
+    dev_free(work32);
     dinv = nullptr;
     dinv32 = nullptr;
     work = nullptr;
@@ -239,10 +239,8 @@ int Pcd::solve(Ctx& c, const T* b, T* x, std::vector<double>* hist, double* norm
     T* work;
     const T* dinv;
     if constexpr (std::is_same<T, float>::value) {
-        if (!work32 && cudaMalloc(&work32, ((size_t)n + 4) * 4) != cudaSuccess) {
-            cudaGetLastError();
-            return kErrAlloc;
-        }
+        int ea;
+        if (!work32 && (ea = dev_alloc(&work32, ((size_t)n + 4) * 4, c.stream))) return ea;
         work = work32;
         dinv = dinv32;
     } else {
@@ -360,17 +358,15 @@ template int Pcd::solve<float>(Ctx&, const float*, float*, std::vector<double>*,
 // ---- setup -------------------------------------------------------------------------------
 
 template <typename T>
-static int alloc_vecs(std::vector<T*>& w, int k, uint32_t n)
+static int alloc_vecs(std::vector<T*>& w, int k, uint32_t n, cudaStream_t s)
 {
     const size_t bytes = ((size_t)n + 4) * sizeof(T);
     for (int i = 0; i < k; ++i) {
         T* p = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            return kErrAlloc;
-        }
-        cudaMemset(p, 0, bytes);
+        const int e = dev_alloc(&p, bytes, s);
+        if (e) return e;
         w.push_back(p);
+        FB_CUDA(cudaMemsetAsync(p, 0, bytes, s));
     }
     return kOk;
 }
@@ -418,9 +414,9 @@ int SolverImpl::setup(fasp_gpu_mat Mh)
     }
     switch (alg) {
         case FASP_GPU_CG: {
-            if ((e = alloc_vecs(w, 5, n))) return e; // rk pk zk ax safe
+            if ((e = alloc_vecs(w, 5, n, c.stream))) return e; // rk pk zk ax safe
             dhistCap = cfg.prm.maxIter + 2;
-            if (cudaMalloc(&dhist, (size_t)dhistCap * 8) != cudaSuccess) return kErrAlloc;
+            if ((e = dev_alloc(&dhist, (size_t)dhistCap * 8, c.stream))) return e;
             const bool fusable = cfg.pcd == 0 || (pcd.pure() && pcd.prm.maxIter == 1);
             if (fusable && cfg.precision == FASP_GPU_FP64) {
                 cg64 = new CGEngine<double>();
@@ -451,20 +447,20 @@ int SolverImpl::setup(fasp_gpu_mat Mh)
         case FASP_GPU_BICGSTAB: {
             if (cfg.precision == FASP_GPU_MIXED) {
                 // FP64: the outer residual; FP32: the inner solve's 12 vectors + b, e
-                if ((e = alloc_vecs(w, 1, n)) || (e = alloc_vecs(w32, 14, n))) return e;
+                if ((e = alloc_vecs(w, 1, n, c.stream)) || (e = alloc_vecs(w32, 14, n, c.stream))) return e;
                 if ((e = Ah->M.ensure32(c.stream))) return e;
             } else if (cfg.precision == FASP_GPU_MIXED_RELIABLE) {
                 // FP64 x and residual; the FP32 engine holds the iteration's vectors
-                if ((e = alloc_vecs(w, 2, n))) return e;
+                if ((e = alloc_vecs(w, 2, n, c.stream))) return e;
                 if ((e = Ah->M.ensure32(c.stream))) return e;
-            } else if ((e = alloc_vecs(w, 12, n))) {
+            } else if ((e = alloc_vecs(w, 12, n, c.stream))) {
                 return e;
             }
             // Identity or one Jacobi sweep from zero: the device-driven engine
             const bool fusable = (A->val || A->grid) && (cfg.pcd == 0 || (pcd.pure() && pcd.prm.maxIter == 1));
             if (fusable) {
                 dhistCap = cfg.prm.maxIter + 2;
-                if (cudaMalloc(&dhist, (size_t)dhistCap * 8) != cudaSuccess) return kErrAlloc;
+                if ((e = dev_alloc(&dhist, (size_t)dhistCap * 8, c.stream))) return e;
                 if (cfg.precision == FASP_GPU_MIXED ||
                     cfg.precision == FASP_GPU_MIXED_RELIABLE) {
                     bi32 = new BiEngine<float>();
@@ -498,43 +494,43 @@ int SolverImpl::setup(fasp_gpu_mat Mh)
             ldV = ((size_t)n + 31) & ~(size_t)31; // every basis vector 256-byte aligned
             if (cfg.precision == FASP_GPU_MIXED) {
                 // FP64 outer residual; FP32 wk tmp safe + b, e and the FP32 bases
-                if ((e = alloc_vecs(w, 1, n)) || (e = alloc_vecs(w32, 5, n))) return e;
+                if ((e = alloc_vecs(w, 1, n, c.stream)) || (e = alloc_vecs(w32, 5, n, c.stream))) return e;
                 if ((e = Ah->M.ensure32(c.stream))) return e;
                 const size_t vb = (size_t)(maxRestart + 1) * ldV * 4;
-                if (cudaMalloc(&V32, vb + 16) != cudaSuccess) return kErrAlloc;
-                cudaMemset(V32, 0, vb);
+                if ((e = dev_alloc(&V32, vb + 16, c.stream))) return e;
+                FB_CUDA(cudaMemsetAsync(V32, 0, vb, c.stream));
                 if (alg == FASP_GPU_FGMRES) {
-                    if (cudaMalloc(&Z32, vb + 16) != cudaSuccess) return kErrAlloc;
-                    cudaMemset(Z32, 0, vb);
+                    if ((e = dev_alloc(&Z32, vb + 16, c.stream))) return e;
+                    FB_CUDA(cudaMemsetAsync(Z32, 0, vb, c.stream));
                 }
             } else {
-                if ((e = alloc_vecs(w, 3, n))) return e; // wk tmp safe
+                if ((e = alloc_vecs(w, 3, n, c.stream))) return e; // wk tmp safe
                 const size_t vb = (size_t)(maxRestart + 1) * ldV * 8;
-                if (cudaMalloc(&V, vb + 16) != cudaSuccess) return kErrAlloc;
-                cudaMemset(V, 0, vb);
+                if ((e = dev_alloc(&V, vb + 16, c.stream))) return e;
+                FB_CUDA(cudaMemsetAsync(V, 0, vb, c.stream));
                 if (alg == FASP_GPU_FGMRES) {
-                    if (cudaMalloc(&Z, vb + 16) != cudaSuccess) return kErrAlloc;
-                    cudaMemset(Z, 0, vb);
+                    if ((e = dev_alloc(&Z, vb + 16, c.stream))) return e;
+                    FB_CUDA(cudaMemsetAsync(Z, 0, vb, c.stream));
                 }
             }
             const size_t gmSize = gm_layout_size(maxRestart);
-            if (cudaMalloc(&gm, gmSize * 8) != cudaSuccess) return kErrAlloc;
-            cudaMemset(gm, 0, gmSize * 8);
-            if (cudaMalloc(&gmc, sizeof(GmCtl)) != cudaSuccess ||
-                cudaMallocHost(&hgmc, sizeof(GmCtl)) != cudaSuccess)
-                return kErrAlloc;
+            if ((e = dev_alloc(&gm, gmSize * 8, c.stream))) return e;
+            FB_CUDA(cudaMemsetAsync(gm, 0, gmSize * 8, c.stream));
+            static_assert(sizeof(GmCtl) <= kPinnedBlock, "control data in one page-locked block");
+            if ((e = dev_alloc(&gmc, sizeof(GmCtl), c.stream))) return e;
+            if (!(hgmc = (GmCtl*)pinned_get())) return kErrAlloc;
             dhistCap = cfg.prm.maxIter + 2;
-            if (cudaMalloc(&dhist, (size_t)dhistCap * 8) != cudaSuccess) return kErrAlloc;
+            if ((e = dev_alloc(&dhist, (size_t)dhistCap * 8, c.stream))) return e;
             break;
         }
         case FASP_GPU_MG: {
             if (!mgIn.empty()) {
-                if ((e = alloc_vecs(w, 1, n))) return e; // r
+                if ((e = alloc_vecs(w, 1, n, c.stream))) return e; // r
                 if ((e = mg_setup_transfers())) return e;
                 break;
             }
             // MG::SetupALL + SetupLevel with identity transfers (MG.cxx:26-79)
-            if ((e = alloc_vecs(w, 1, n))) return e; // r
+            if ((e = alloc_vecs(w, 1, n, c.stream))) return e; // r
             const uint32_t L = cfg.mgLevels;
             mgSmooth.resize(L);
             mgCoarse.resize(L);
@@ -543,7 +539,7 @@ int SolverImpl::setup(fasp_gpu_mat Mh)
                 if ((e = mgCoarse[l].setup(c, A, 1, cfg.mgCoarseWeight, cfg.mgCoarsePrm))) return e;
             }
             std::vector<double*> lv;
-            if ((e = alloc_vecs(lv, 2 * L, n))) return e;
+            if ((e = alloc_vecs(lv, 2 * L, n, c.stream))) return e;
             for (uint32_t l = 0; l < L; ++l) {
                 mgB.push_back(lv[2 * l]);
                 mgX.push_back(lv[2 * l + 1]);
@@ -578,31 +574,32 @@ void SolverImpl::clean()
 
 void SolverImpl::destroy()
 {
-    for (double* p : w) cudaFree(p);
+    if (A) cudaDeviceSynchronize(); // whatever still runs on what is released below
+    for (double* p : w) dev_free(p);
     w.clear();
-    for (float* p : w32) cudaFree(p);
+    for (float* p : w32) dev_free(p);
     w32.clear();
-    cudaFree(V32);
-    cudaFree(Z32);
+    dev_free(V32);
+    dev_free(Z32);
     V32 = Z32 = nullptr;
-    cudaFree(V);
-    cudaFree(Z);
-    cudaFree(gm);
-    cudaFree(gmc);
-    if (hgmc) cudaFreeHost(hgmc);
+    dev_free(V);
+    dev_free(Z);
+    dev_free(gm);
+    dev_free(gmc);
+    pinned_put(hgmc);
     gmc = nullptr;
     hgmc = nullptr;
-    cudaFree(safe);
-    cudaFree(dhist);
-    cudaFree(hostB);
-    cudaFree(hostX);
+    dev_free(safe);
+    dev_free(dhist);
+    dev_free(hostB);
+    dev_free(hostX);
     V = Z = gm = safe = dhist = hostB = hostX = nullptr;
     pcd.destroy();
     for (auto& p : mgSmooth) p.destroy();
     for (auto& p : mgCoarse) p.destroy();
-    for (double* p : mgB) cudaFree(p);
-    for (double* p : mgX) cudaFree(p);
-    for (double* p : mgRes) cudaFree(p);
+    for (double* p : mgB) dev_free(p);
+    for (double* p : mgX) dev_free(p);
+    for (double* p : mgRes) dev_free(p);
     mgRes.clear();
     for (Mat* m : mgOwn) {
         m_free(*m);
@@ -830,7 +827,7 @@ int SolverImpl::cg_device(const double* b, double* x, fasp_gpu_info* info)
             patches.push_back({h.numIter, h.resAbs});
             finished = true;
         } else if (reason == kSave) { // CG.cxx:138
-            if (!safe && cudaMalloc(&safe, ((size_t)n + 2) * 8) != cudaSuccess) return kErrAlloc;
+            if (!safe && (e = dev_alloc(&safe, ((size_t)n + 2) * 8, c.stream))) return e;
             v_copy(c, n, E.x, safe);
         } else if (reason == kStag) { // CG.cxx:153-181
             true_res();
@@ -2367,12 +2364,12 @@ int SolverImpl::mg_setup_transfers()
         if ((e = mgCoarse[l].setup(c, mgA[l + 1], 1, cfg.mgCoarseWeight, cfg.mgCoarsePrm)))
             return e;
         std::vector<double*> v;
-        if ((e = alloc_vecs(v, 2, mgA[l + 1]->nrow))) return e;
+        if ((e = alloc_vecs(v, 2, mgA[l + 1]->nrow, c.stream))) return e;
         mgB.push_back(v[0]);
         mgX.push_back(v[1]);
         std::vector<double*> r;
         if (l > 0) {
-            if ((e = alloc_vecs(r, 1, mgA[l]->nrow))) return e;
+            if ((e = alloc_vecs(r, 1, mgA[l]->nrow, c.stream))) return e;
             mgRes.push_back(r[0]);
         } else {
             mgRes.push_back(nullptr); // level 0 uses the solver's residual vector

@@ -119,7 +119,7 @@ int m_mult(Ctx& c, const Mat& L, const Mat& R, Mat& C)
     if (L.nrow == 0 || R.mcol == 0) return kErrMatSize;
     cudaStream_t s = c.stream;
     const uint32_t n = L.nrow;
-    Tmp t;
+    Tmp t(s);
     int e;
     uint32_t *cnt = nullptr, *coff = nullptr, *tiles = nullptr;
     unsigned long long* total = nullptr;
@@ -249,7 +249,7 @@ int m_add(Ctx& c, double a, const Mat& A, double b, const Mat& B, Mat& C)
     if (cap > 0xffffffffull) return kErrMatSize;
     cudaStream_t s = c.stream;
     const uint32_t n = A.nrow;
-    Tmp t;
+    Tmp t(s);
     int e;
     uint32_t *tci = nullptr, *nout = nullptr, *crp = nullptr, *tiles = nullptr, *cci = nullptr;
     double *tva = nullptr, *cva = nullptr;

@@ -279,13 +279,13 @@ int Mat::ensure32(cudaStream_t s)
     if (!val) return kOk;
     int e;
     if (!val32) {
-        if ((e = dmalloc((void**)&val32, (size_t)nnz * 4))) return e;
+        if ((e = dmalloc((void**)&val32, (size_t)nnz * 4, s))) return e;
         k_to_f32<<<std::max(1, std::min(ceil_div(nnz, kBlock), 148 * 8)), kBlock, 0, s>>>(
             nnz, val, val32);
         FB_CUDA(cudaGetLastError());
     }
     if (rcVal && !rcVal32) {
-        if ((e = dmalloc((void**)&rcVal32, (size_t)rcEntries * 4 + 16))) return e;
+        if ((e = dmalloc((void**)&rcVal32, (size_t)rcEntries * 4 + 16, s))) return e;
         k_to_f32<<<std::max(1, std::min(ceil_div(rcEntries, kBlock), 148 * 8)), kBlock, 0, s>>>(
             rcEntries, rcVal, rcVal32);
         FB_CUDA(cudaGetLastError());
@@ -413,21 +413,21 @@ int m_transpose(Ctx& c, const Mat& A, Mat& T)
     R.nnz = nnz;
     R.dev = A.dev;
     uint32_t *cnt = nullptr, *fill = nullptr, *pos = nullptr, *rowOf = nullptr;
+    cudaStream_t s = c.stream;
     int e;
-    if ((e = dmalloc((void**)&R.rowPtr, ((size_t)m + 1) * 4)) ||
-        (e = dmalloc((void**)&R.colInd, (size_t)nnz * 4)) ||
-        (A.val && (e = dmalloc((void**)&R.val, (size_t)nnz * 8))) ||
-        (e = dmalloc((void**)&cnt, (size_t)m * 4)) || (e = dmalloc((void**)&fill, (size_t)m * 4)) ||
-        (e = dmalloc((void**)&pos, (size_t)nnz * 4)) ||
-        (e = dmalloc((void**)&rowOf, (size_t)nnz * 4))) {
+    if ((e = dmalloc((void**)&R.rowPtr, ((size_t)m + 1) * 4, s)) ||
+        (e = dmalloc((void**)&R.colInd, (size_t)nnz * 4, s)) ||
+        (A.val && (e = dmalloc((void**)&R.val, (size_t)nnz * 8, s))) ||
+        (e = dmalloc((void**)&cnt, (size_t)m * 4, s)) || (e = dmalloc((void**)&fill, (size_t)m * 4, s)) ||
+        (e = dmalloc((void**)&pos, (size_t)nnz * 4, s)) ||
+        (e = dmalloc((void**)&rowOf, (size_t)nnz * 4, s))) {
         m_free(R);
-        cudaFree(cnt);
-        cudaFree(fill);
-        cudaFree(pos);
-        cudaFree(rowOf);
+        dev_free(cnt);
+        dev_free(fill);
+        dev_free(pos);
+        dev_free(rowOf);
         return e;
     }
-    cudaStream_t s = c.stream;
     const int gn = std::max(1, std::min(ceil_div(nnz, kBlock), c.nsm * 8));
     const int gm = std::max(1, std::min(ceil_div(m, kBlock), c.nsm * 8));
     const int gr = std::max(1, std::min(ceil_div(n, kBlock), c.nsm * 8));
@@ -440,10 +440,10 @@ int m_transpose(Ctx& c, const Mat& A, Mat& T)
     k_sort_gather<<<gm, kBlock, 0, s>>>(m, R.rowPtr, pos, rowOf, A.val, R.colInd, R.val);
     FB_CUDA(cudaGetLastError());
     e = m_inspect(R, false, s);
-    cudaFree(cnt);
-    cudaFree(fill);
-    cudaFree(pos);
-    cudaFree(rowOf);
+    dev_free(cnt);
+    dev_free(fill);
+    dev_free(pos);
+    dev_free(rowOf);
     if (e) {
         m_free(R);
         return e;
@@ -461,8 +461,8 @@ int m_autotune(Ctx& c, Mat& A)
     if (A.grid) return kOk; // grid operators run thread per row (lanes = 1) only
     double *x = nullptr, *y = nullptr;
     int e;
-    if ((e = dmalloc((void**)&x, (size_t)A.mcol * 8)) || (e = dmalloc((void**)&y, (size_t)A.nrow * 8))) {
-        cudaFree(x);
+    if ((e = dmalloc((void**)&x, (size_t)A.mcol * 8, c.stream)) || (e = dmalloc((void**)&y, (size_t)A.nrow * 8, c.stream))) {
+        dev_free(x);
         return e;
     }
     FB_CUDA(cudaMemsetAsync(x, 0, (size_t)A.mcol * 8, c.stream));
@@ -490,8 +490,8 @@ int m_autotune(Ctx& c, Mat& A)
     A.lanes = cudaGetLastError() == cudaSuccess ? bestL : orig;
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
-    cudaFree(x);
-    cudaFree(y);
+    dev_free(x);
+    dev_free(y);
     return kOk;
 }
 
@@ -648,7 +648,7 @@ int m_create_stencil(Mat& M, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t npt
     T.diagValue = diagv;
     cudaGetDevice(&T.dev);
     int e;
-    if ((e = dmalloc((void**)&T.diag, (size_t)T.nrow * 8))) return e;
+    if ((e = dmalloc((void**)&T.diag, (size_t)T.nrow * 8, s))) return e;
     k_fill_const<<<std::max(1, std::min(ceil_div(T.nrow, kBlock), 148 * 8)), kBlock, 0, s>>>(
         T.nrow, diagv, T.diag);
     FB_CUDA(cudaGetLastError());

@@ -13,16 +13,7 @@ namespace fb {
 
 // 32 spare bytes keep vectorised/bulk tail accesses inside the allocation (the warp
 // tiles' 16-byte loads read up to 3 entries past the last one)
-int dmalloc(void** p, size_t bytes)
-{
-    cudaError_t e = cudaMalloc(p, bytes + 32);
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        cudaGetLastError();
-        return kErrAlloc;
-    }
-    return kOk;
-}
+int dmalloc(void** p, size_t bytes, cudaStream_t s) { return dev_alloc_bytes(p, bytes + 32, s); }
 
 namespace {
 
@@ -364,7 +355,7 @@ bool class_masks(const std::vector<uint32_t>& off, const std::vector<int32_t>& d
 // Device memory of one upload's temporaries.
 struct Slab {
     void* p = nullptr;
-    ~Slab() { cudaFree(p); }
+    ~Slab() { dev_free(p); }
 };
 
 constexpr unsigned long long kClassSeeds[3] = {1469598103934665603ull, 0x9e3779b97f4a7c15ull,
@@ -374,19 +365,19 @@ constexpr unsigned long long kClassSeeds[3] = {1469598103934665603ull, 0x9e3779b
 
 void m_free(Mat& M)
 {
-    cudaFree(M.rowPtr);
-    cudaFree(M.colInd);
-    cudaFree(M.diagPtr);
-    cudaFree(M.val);
-    cudaFree(M.val32);
-    cudaFree(M.diag);
-    cudaFree(M.rcCls);
-    cudaFree(M.rcOff);
-    cudaFree(M.rcDelta);
-    cudaFree(M.rcVal);
-    cudaFree(M.rcVal32);
-    cudaFree(M.skMask);
-    cudaFree(M.cd16);
+    dev_free(M.rowPtr);
+    dev_free(M.colInd);
+    dev_free(M.diagPtr);
+    dev_free(M.val);
+    dev_free(M.val32);
+    dev_free(M.diag);
+    dev_free(M.rcCls);
+    dev_free(M.rcOff);
+    dev_free(M.rcDelta);
+    dev_free(M.rcVal);
+    dev_free(M.rcVal32);
+    dev_free(M.skMask);
+    dev_free(M.cd16);
     M = Mat();
 }
 
@@ -411,7 +402,7 @@ int finish_classes(Mat& T, const ClassSlots* S, Inspect* ins, cudaStream_t s, Cl
                  vOff = (dOff + cap * 4 + 15) & ~(size_t)15;
     Slab slab;
     int e;
-    if ((e = dmalloc(&slab.p, vOff + cap * 8))) return e;
+    if ((e = dmalloc(&slab.p, vOff + cap * 8, s))) return e;
     Small* t = (Small*)slab.p;
     int32_t* delta = (int32_t*)((char*)slab.p + dOff);
     double* tval = (double*)((char*)slab.p + vOff);
@@ -432,10 +423,10 @@ int finish_classes(Mat& T, const ClassSlots* S, Inspect* ins, cudaStream_t s, Cl
     FB_CUDA(cudaStreamSynchronize(s));
     std::vector<uint16_t> cm;
     const bool masks = class_masks(off, hd, hv, T, cm);
-    if ((e = dmalloc((void**)&T.rcOff, ((size_t)C + 1) * 4)) ||
-        (e = dmalloc((void**)&T.rcDelta, (size_t)E * 4 + 16)) ||
-        (e = dmalloc((void**)&T.rcVal, (size_t)E * 8 + 16)) ||
-        (masks && (e = dmalloc((void**)&T.skMask, (size_t)T.nrow * 2 + 16))))
+    if ((e = dmalloc((void**)&T.rcOff, ((size_t)C + 1) * 4, s)) ||
+        (e = dmalloc((void**)&T.rcDelta, (size_t)E * 4 + 16, s)) ||
+        (e = dmalloc((void**)&T.rcVal, (size_t)E * 8 + 16, s)) ||
+        (masks && (e = dmalloc((void**)&T.skMask, (size_t)T.nrow * 2 + 16, s))))
         return e;
     FB_CUDA(cudaMemcpyAsync(T.rcOff, t->off, ((size_t)C + 1) * 4, cudaMemcpyDeviceToDevice, s));
     FB_CUDA(cudaMemcpyAsync(T.rcDelta, delta, (size_t)E * 4, cudaMemcpyDeviceToDevice, s));
@@ -458,11 +449,11 @@ int finish_classes(Mat& T, const ClassSlots* S, Inspect* ins, cudaStream_t s, Cl
 
 void drop_classes(Mat& T)
 {
-    cudaFree(T.rcCls);
-    cudaFree(T.rcOff);
-    cudaFree(T.rcDelta);
-    cudaFree(T.rcVal);
-    cudaFree(T.skMask);
+    dev_free(T.rcCls);
+    dev_free(T.rcOff);
+    dev_free(T.rcDelta);
+    dev_free(T.rcVal);
+    dev_free(T.skMask);
     T.rcCls = T.skMask = nullptr;
     T.rcOff = nullptr;
     T.rcDelta = nullptr;
@@ -486,8 +477,8 @@ int m_inspect(Mat& T, bool classes, cudaStream_t s)
     const int grid = std::max(1, std::min(ceil_div(nrow, kBlock), 148 * 8));
     Slab slab;
     int e;
-    if ((e = dmalloc(&slab.p, sizeof(Work))) || (e = dmalloc((void**)&T.diagPtr, (size_t)nrow * 4)) ||
-        (e = dmalloc((void**)&T.diag, (size_t)nrow * 8)))
+    if ((e = dmalloc(&slab.p, sizeof(Work), s)) || (e = dmalloc((void**)&T.diagPtr, (size_t)nrow * 4, s)) ||
+        (e = dmalloc((void**)&T.diag, (size_t)nrow * 8, s)))
         return e;
     Work* w = (Work*)slab.p;
     T.meanRowLen = (double)nnz / nrow;
@@ -503,7 +494,7 @@ int m_inspect(Mat& T, bool classes, cudaStream_t s)
     int attempt = 0;
     do {
         if (classes) {
-            if ((e = dmalloc((void**)&T.rcCls, (size_t)nrow * 2 + 16))) return e;
+            if ((e = dmalloc((void**)&T.rcCls, (size_t)nrow * 2 + 16, s))) return e;
             FB_CUDA(cudaMemsetAsync(w->slots.key, 0, sizeof(w->slots.key), s));
             FB_CUDA(cudaMemsetAsync(w->slots.rep, 0xff, sizeof(w->slots.rep), s));
             FB_CUDA(cudaMemsetAsync(&w->ins.classes, 0, 4, s));
@@ -552,9 +543,9 @@ int m_upload(Mat& M, uint32_t nrow, uint32_t mcol, uint32_t nnz, const uint32_t*
     int e;
     auto fill = [&]() -> int {
         const cudaMemcpyKind kind = hostPtrs ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
-        if ((e = dmalloc((void**)&T.rowPtr, ((size_t)nrow + 1) * 4)) ||
-            (e = dmalloc((void**)&T.colInd, (size_t)nnz * 4)) ||
-            (values && (e = dmalloc((void**)&T.val, (size_t)nnz * 8))))
+        if ((e = dmalloc((void**)&T.rowPtr, ((size_t)nrow + 1) * 4, s)) ||
+            (e = dmalloc((void**)&T.colInd, (size_t)nnz * 4, s)) ||
+            (values && (e = dmalloc((void**)&T.val, (size_t)nnz * 8, s))))
             return e;
         // device arrays may still be being written by work on the legacy default stream
         // (torch's, say): the copies wait for it, as a blocking copy there would
@@ -595,7 +586,7 @@ int m_build_col16(Mat& M, cudaStream_t s)
 {
     if (!M.near16 || M.cd16) return kOk;
     int e;
-    if ((e = dmalloc((void**)&M.cd16, ((size_t)M.nnz + 8) * 2))) return e;
+    if ((e = dmalloc((void**)&M.cd16, ((size_t)M.nnz + 8) * 2, s))) return e;
     k_col16<<<std::max(1, std::min(ceil_div(M.nrow, kBlock), 148 * 8)), kBlock, 0, s>>>(
         M.nrow, M.rowPtr, M.colInd, M.cd16);
     FB_CUDA(cudaGetLastError());
