@@ -391,6 +391,9 @@ int m_build_col16(Mat& M, cudaStream_t s);
 // holds beyond its sizes, rowPtr, colInd and val: diagonal, longest row, tile span, 16-bit
 // reach, lanes and, when asked for, the row-class form. Synchronises the stream (upload.cu).
 int m_inspect(Mat& T, bool classes, cudaStream_t s);
+// M takes T's sizes, rowPtr, colInd and val (dmalloc'd, written on s) and what m_inspect
+// finds in them; on failure T is released.
+int m_adopt(Mat& M, Mat& T, cudaStream_t s);
 // Orders s after everything enqueued on the legacy default stream so far.
 int after_legacy_stream(cudaStream_t s);
 // dev_alloc with the spare bytes every matrix array has.

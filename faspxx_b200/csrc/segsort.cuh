@@ -277,6 +277,46 @@ int stage(Tmp& t, cudaStream_t s, const T* src, size_t count, bool onDevice, con
 }
 
 
+// What sort_row_keys has to do: rows of 2 to 8 and of 9 to 32 keys, block segments, rows of
+// more than kSegMax keys and the longest of those.
+struct SortPlan {
+    unsigned n8, n32, segs, huge, maxHuge;
+};
+
+// Rows by length. With lists: also each segment and each huge row (start, length), in any
+// order.
+__global__ void __launch_bounds__(256) k_sort_plan(uint32_t nrow, const uint32_t* __restrict__ rowPtr,
+                                                   SortPlan* __restrict__ P, uint2* __restrict__ segs,
+                                                   uint2* __restrict__ huge)
+{
+    unsigned n8 = 0, n32 = 0;
+    for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < nrow;
+         r += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t b = rowPtr[r], len = rowPtr[r + 1] - b;
+        if (len <= 1) continue;
+        if (len <= 8) {
+            ++n8;
+        } else if (len <= 32) {
+            ++n32;
+        } else {
+            const unsigned ns = (unsigned)(((size_t)len + kSegMax - 1) / kSegMax);
+            const unsigned at = atomicAdd(&P->segs, ns);
+            if (segs)
+                for (unsigned k = 0; k < ns; ++k) {
+                    const uint32_t o = k * (uint32_t)kSegMax;
+                    segs[at + k] = make_uint2(b + o, min((uint32_t)kSegMax, len - o));
+                }
+            if (len > (uint32_t)kSegMax) {
+                const unsigned h = atomicAdd(&P->huge, 1u);
+                if (huge) huge[h] = make_uint2(b, len);
+                atomicMax(&P->maxHuge, len);
+            }
+        }
+    }
+    if (__syncthreads_or(n8 != 0) && threadIdx.x == 0) atomicOr(&P->n8, 1u);
+    if (__syncthreads_or(n32 != 0) && threadIdx.x == 0) atomicOr(&P->n32, 1u);
+}
+
 // Sorts the keys of every row segment [rowPtr[r], rowPtr[r + 1]) ascending (rowPtr on the
 // device, 0-based; keys unique within a row, so the order is fully determined).
 int sort_row_keys(Ctx& c, Tmp& t, uint32_t nrow, const uint32_t* rowPtr, uint64_t* keys,
@@ -284,58 +324,40 @@ int sort_row_keys(Ctx& c, Tmp& t, uint32_t nrow, const uint32_t* rowPtr, uint64_
 {
     cudaStream_t s = c.stream;
     int e;
-    std::vector<uint32_t> hrp((size_t)nrow + 1);
-    FB_CUDA(cudaMemcpyAsync(hrp.data(), rowPtr, hrp.size() * 4, cudaMemcpyDeviceToHost, s));
-    FB_CUDA(cudaStreamSynchronize(s));
-    // row classes by length
-    std::vector<uint2> segs, huge;
-    uint32_t maxHuge = 0;
-    bool small8 = false, small32 = false;
-    for (uint32_t r = 0; r < nrow; ++r) {
-        const uint32_t b = hrp[r], len = hrp[r + 1] - b;
-        if (len <= 1) continue;
-        if (len <= 8) {
-            small8 = true;
-        } else if (len <= 32) {
-            small32 = true;
-        } else if (len <= (uint32_t)kSegMax) {
-            segs.push_back(make_uint2(b, len));
-        } else {
-            for (uint32_t o = 0; o < len; o += kSegMax)
-                segs.push_back(make_uint2(b + o, std::min<uint32_t>(kSegMax, len - o)));
-            huge.push_back(make_uint2(b, len));
-            maxHuge = std::max(maxHuge, len);
-        }
-    }
-    if (small8) k_sort_short<8><<<grid_for((size_t)nrow * 8, 256), 256, 0, s>>>(nrow, 1, rowPtr, keys);
-    if (small32) k_sort_short<32><<<grid_for((size_t)nrow * 32, 256), 256, 0, s>>>(nrow, 8, rowPtr, keys);
+    SortPlan* dp = nullptr;
+    SortPlan p;
+    if ((e = t.get(&dp, 1))) return e;
+    const int gp = grid_for(nrow, 256);
+    FB_CUDA(cudaMemsetAsync(dp, 0, sizeof(p), s));
+    k_sort_plan<<<gp, 256, 0, s>>>(nrow, rowPtr, dp, nullptr, nullptr);
     FB_CUDA(cudaGetLastError());
-    uint2* dseg = nullptr;
-    if (!segs.empty()) {
-        if ((e = t.get(&dseg, segs.size()))) return e;
-        FB_CUDA(cudaMemcpyAsync(dseg, segs.data(), segs.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
-        for (size_t o = 0; o < segs.size(); o += 0x7fffffffu) {
-            const size_t cnt = std::min<size_t>(segs.size() - o, 0x7fffffffu);
-            k_sort_segment<<<(unsigned)cnt, kSegThreads, 0, s>>>(dseg + o, keys);
-        }
-        FB_CUDA(cudaGetLastError());
+    FB_CUDA(cudaMemcpyAsync(&p, dp, sizeof(p), cudaMemcpyDeviceToHost, s));
+    FB_CUDA(cudaStreamSynchronize(s));
+    if (p.n8) k_sort_short<8><<<grid_for((size_t)nrow * 8, 256), 256, 0, s>>>(nrow, 1, rowPtr, keys);
+    if (p.n32) k_sort_short<32><<<grid_for((size_t)nrow * 32, 256), 256, 0, s>>>(nrow, 8, rowPtr, keys);
+    FB_CUDA(cudaGetLastError());
+    if (!p.segs) return kOk;
+    uint2 *segs = nullptr, *dh = nullptr;
+    if ((e = t.get(&segs, p.segs)) || (e = t.get(&dh, p.huge))) return e;
+    FB_CUDA(cudaMemsetAsync(dp, 0, sizeof(p), s));
+    k_sort_plan<<<gp, 256, 0, s>>>(nrow, rowPtr, dp, segs, dh);
+    for (size_t o = 0; o < p.segs; o += 0x7fffffffu) {
+        const size_t cnt = std::min<size_t>(p.segs - o, 0x7fffffffu);
+        k_sort_segment<<<(unsigned)cnt, kSegThreads, 0, s>>>(segs + o, keys);
     }
-    if (!huge.empty()) {
-        uint2* dh = nullptr;
-        uint64_t* alt = nullptr;
-        if ((e = t.get(&dh, huge.size())) || (e = t.get(&alt, nkeys))) return e;
-        FB_CUDA(cudaMemcpyAsync(dh, huge.data(), huge.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
-        const uint32_t nh = (uint32_t)huge.size();
-        const dim3 g((unsigned)std::min<size_t>((maxHuge + 255) / 256, 1024), std::min<uint32_t>(nh, 65535));
-        uint64_t *src = keys, *dst = alt;
-        for (uint64_t w = kSegMax; w < maxHuge; w *= 2) {
-            k_merge_pass<<<g, 256, 0, s>>>(nh, dh, (uint32_t)w, src, dst);
-            std::swap(src, dst);
-        }
-        if (src != keys) k_copy_rows<<<g, 256, 0, s>>>(nh, dh, src, keys);
-        FB_CUDA(cudaGetLastError());
+    FB_CUDA(cudaGetLastError());
+    if (!p.huge) return kOk;
+    uint64_t* alt = nullptr;
+    if ((e = t.get(&alt, nkeys))) return e;
+    const dim3 g((unsigned)std::min<size_t>((p.maxHuge + 255) / 256, 1024),
+                 std::min<uint32_t>(p.huge, 65535));
+    uint64_t *src = keys, *dst = alt;
+    for (uint64_t w = kSegMax; w < p.maxHuge; w *= 2) {
+        k_merge_pass<<<g, 256, 0, s>>>(p.huge, dh, (uint32_t)w, src, dst);
+        std::swap(src, dst);
     }
-
+    if (src != keys) k_copy_rows<<<g, 256, 0, s>>>(p.huge, dh, src, keys);
+    FB_CUDA(cudaGetLastError());
     return kOk;
 }
 

@@ -520,6 +520,20 @@ int m_inspect(Mat& T, bool classes, cudaStream_t s)
     return kOk;
 }
 
+int m_adopt(Mat& M, Mat& T, cudaStream_t s)
+{
+    cudaGetDevice(&T.dev);
+    int e = T.nrow == 0 || T.mcol == 0 || T.nnz == 0 ? kErrMatSize : m_inspect(T, true, s);
+    if (!e && cudaStreamSynchronize(s) != cudaSuccess) e = kErrCuda;
+    if (e) {
+        cudaStreamSynchronize(s);
+        m_free(T);
+        return e;
+    }
+    M = T;
+    return kOk;
+}
+
 int after_legacy_stream(cudaStream_t s)
 {
     cudaEvent_t ev;
