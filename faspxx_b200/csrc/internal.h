@@ -383,7 +383,7 @@ int m_residual(Ctx& c, const Mat& A, const double* b, const double* x, double* r
                const double* xinf);
 int m_residual(Ctx& c, const Mat& A, const float* b, const float* x, float* r,
                const double* xinf);
-int m_transpose(Ctx& c, const Mat& A, Mat& T);                            // CSR -> CSC, exact
+int m_transpose(Ctx& c, const Mat& A, Mat& T); // CSR -> CSC, exact (transpose.cu)
 // Builds M.cd16 (16-bit column offsets) when every |col - row| <= 32767 (near16); otherwise
 // leaves it null. Synchronises the stream.
 int m_build_col16(Mat& M, cudaStream_t s);

@@ -361,5 +361,123 @@ int sort_row_keys(Ctx& c, Tmp& t, uint32_t nrow, const uint32_t* rowPtr, uint64_
     return kOk;
 }
 
+// ---- rows of up to kRankMost entries in their final order, one pass -------------------------
+// An entry on its way into its row: ordered by (column, position in the input).
+struct __align__(16) Rec {
+    uint32_t col, pos;
+    double   val;
+};
+
+constexpr uint32_t kRankMost = 128;    // longest row of k_rank_rows: its work grows with len^2
+constexpr uint32_t kRankRows = 64;     // rows of a block's turn
+constexpr uint32_t kRankEntries = 2048; // entries of a block's turn, in shared memory
+
+// Where k_rank_rows reads entry q: records scattered into their rows, or raw CSR arrays
+// (whose columns start at base).
+struct RecSource {
+    const Rec* rec;
+    __device__ __forceinline__ void get(size_t q, uint64_t* key, double* val) const
+    {
+        const Rec r = rec[q];
+        *key = (uint64_t)r.col << 32 | r.pos;
+        *val = r.val;
+    }
+};
+struct CsrSource {
+    const uint32_t* ci;
+    const double*   va;
+    const uint32_t* base;
+    __device__ __forceinline__ void get(size_t q, uint64_t* key, double* val) const
+    {
+        *key = (uint64_t)(ci[q] - *base) << 32 | (uint32_t)q;
+        *val = va[q];
+    }
+};
+
+// Row r's entries are inPtr[r] - *base (base null: 0) and on; its place is [outPtr[r],
+// outPtr[r + 1]), one longer where miss[r] asks for a 0.0 diagonal (HOLES: the input segment
+// has that spare place too, at its end). An entry's place is the number of its row's keys
+// below its own (keys are unique), counted in shared memory, plus one past an inserted
+// diagonal: no sort, no second pass to insert, no gather of values by position, and all
+// global reads and writes of a block are one contiguous range. Bound by the reads of shared
+// memory, one key per (entry, entry of its row).
+template <bool HOLES, class Source>
+__global__ void __launch_bounds__(256) k_rank_rows(uint32_t nrow, const uint32_t* __restrict__ inPtr,
+                                                   const uint32_t* __restrict__ base,
+                                                   const uint32_t* __restrict__ outPtr,
+                                                   const uint8_t* __restrict__ miss, Source src,
+                                                   uint32_t* __restrict__ outCol,
+                                                   double* __restrict__ outVal)
+{
+    __shared__ uint64_t key[kRankEntries];
+    __shared__ double val[kRankEntries];
+    __shared__ uint32_t ib[kRankRows + 1], ob[kRankRows];
+    __shared__ uint8_t ms[kRankRows];
+    const uint32_t t = threadIdx.x, in0 = base ? *base : 0u;
+    const size_t nt = ((size_t)nrow + kRankRows - 1) / kRankRows;
+    for (size_t tile = blockIdx.x; tile < nt; tile += gridDim.x) {
+        const uint32_t r0 = (uint32_t)(tile * kRankRows);
+        const uint32_t rows = nrow - r0 < kRankRows ? nrow - r0 : kRankRows;
+        __syncthreads();
+        if (t <= rows) ib[t] = inPtr[r0 + t] - in0;
+        if (t < rows) {
+            ob[t] = outPtr[r0 + t];
+            ms[t] = miss ? miss[r0 + t] : (uint8_t)0;
+        }
+        __syncthreads();
+        for (uint32_t s = 0; s < rows;) {
+            // as many rows as fit (at least one: a row has at most kRankMost entries and a hole)
+            const uint32_t g = (uint32_t)__syncthreads_count(
+                t >= s && t < rows && ib[t + 1] - ib[s] <= kRankEntries);
+            const uint32_t c0 = ib[s], n = ib[s + g] - c0;
+            for (uint32_t q = t; q < n; q += blockDim.x) src.get((size_t)c0 + q, &key[q], &val[q]);
+            __syncthreads();
+            for (uint32_t q = t; q < n; q += blockDim.x) {
+                uint32_t lo = s, hi = s + g; // the row: ib[lo] - c0 <= q < ib[hi] - c0
+                while (hi - lo > 1) {
+                    const uint32_t mid = (lo + hi) / 2;
+                    if (ib[mid] - c0 <= q)
+                        lo = mid;
+                    else
+                        hi = mid;
+                }
+                const uint32_t b = ib[lo] - c0;
+                const uint32_t e = ib[lo + 1] - c0 - (HOLES ? ms[lo] : 0u);
+                if (HOLES && q >= e) continue; // the spare place
+                const uint64_t k = key[q];
+                uint32_t below = 0;
+#pragma unroll 4
+                for (uint32_t j = b; j < e; ++j) below += key[j] < k ? 1u : 0u;
+                const uint32_t col = (uint32_t)(k >> 32);
+                const size_t o = (size_t)ob[lo] + below + (ms[lo] && col > r0 + lo ? 1u : 0u);
+                outCol[o] = col;
+                if (outVal) outVal[o] = val[q];
+            }
+            if (t >= s && t < s + g && ms[t]) { // the row's explicit 0.0 diagonal
+                const uint32_t b = ib[t] - c0, e = ib[t + 1] - c0 - (HOLES ? 1u : 0u);
+                uint32_t below = 0;
+                for (uint32_t j = b; j < e; ++j) below += (uint32_t)(key[j] >> 32) < r0 + t ? 1u : 0u;
+                outCol[(size_t)ob[t] + below] = r0 + t;
+                outVal[(size_t)ob[t] + below] = 0.0;
+            }
+            __syncthreads();
+            s += g;
+        }
+    }
+}
+
+template <bool HOLES, class Source>
+int rank_rows(Ctx& c, uint32_t nrow, const uint32_t* inPtr, const uint32_t* base,
+              const uint32_t* outPtr, const uint8_t* miss, Source src, uint32_t* outCol,
+              double* outVal)
+{
+    const auto kern = k_rank_rows<HOLES, Source>;
+    const int g = std::max(1, std::min(ceil_div(nrow, (int)kRankRows),
+                                       resident_grid(c, (const void*)kern, 256)));
+    kern<<<g, 256, 0, c.stream>>>(nrow, inPtr, base, outPtr, miss, src, outCol, outVal);
+    FB_CUDA(cudaGetLastError());
+    return kOk;
+}
+
 } // namespace
 } // namespace fb

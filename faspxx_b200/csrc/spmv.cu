@@ -1,6 +1,5 @@
-// spmv.cu -- CSRx matrices in HBM: SpMV (MAT::Apply), residual (MAT::Residual), CSR->CSC
-// transpose (MAT::TransInPlace), the lanes-per-row autotuner and the sampled outer product of
-// the adjoint gradient.
+// spmv.cu -- CSRx matrices in HBM: SpMV (MAT::Apply), residual (MAT::Residual), the
+// lanes-per-row autotuner and the sampled outer product of the adjoint gradient.
 //
 // SpMV mapping: a group of L lanes (L = 1, 2, ..., 32) owns one row; the lanes stride over
 // the row's entries so that a warp reads 32/L consecutive rows' values and column indices
@@ -290,168 +289,6 @@ int Mat::ensure32(cudaStream_t s)
             rcEntries, rcVal, rcVal32);
         FB_CUDA(cudaGetLastError());
     }
-    return kOk;
-}
-
-// ---- transpose: CSR -> CSC in exactly MAT::TransInPlace's order (MAT.cxx:479-538) -------
-// Column counts by atomics, an exclusive scan, a scatter that records each entry's original
-// position, then each output row (input column) sorted by original position: since CSR
-// positions increase with the row index, that is the ascending-row order the reference's
-// row-by-row scatter produces.
-
-__global__ void k_col_count(uint32_t nnz, const uint32_t* __restrict__ colInd,
-                            uint32_t* __restrict__ cnt)
-{
-    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz;
-         k += (size_t)gridDim.x * blockDim.x)
-        atomicAdd(&cnt[colInd[k]], 1u);
-}
-
-// single-block exclusive scan of cnt[0..m) into out[0..m]
-__global__ void k_scan(uint32_t m, const uint32_t* __restrict__ cnt, uint32_t* __restrict__ out)
-{
-    __shared__ uint32_t warpTot[32];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (uint32_t base = 0; base < m; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        uint32_t v = i < m ? cnt[i] : 0, incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) warpTot[wid] = incl;
-        __syncthreads();
-        if (wid == 0) {
-            uint32_t w = lane < (int)(blockDim.x >> 5) ? warpTot[lane] : 0, wi = w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
-                if (lane >= o) wi += t;
-            }
-            warpTot[lane] = wi - w; // exclusive warp offsets
-        }
-        __syncthreads();
-        if (i < m) out[i] = carry + warpTot[wid] + incl - v;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry += warpTot[wid] + incl;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[m] = carry;
-}
-
-__global__ void k_row_of(uint32_t nrow, const uint32_t* __restrict__ rowPtr,
-                         uint32_t* __restrict__ rowOf)
-{
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nrow;
-         i += (size_t)gridDim.x * blockDim.x)
-        for (uint32_t k = rowPtr[i]; k < rowPtr[i + 1]; ++k) rowOf[k] = (uint32_t)i;
-}
-
-__global__ void k_scatter_pos(uint32_t nnz, const uint32_t* __restrict__ colInd,
-                              const uint32_t* __restrict__ tRowPtr, uint32_t* __restrict__ fill,
-                              uint32_t* __restrict__ pos)
-{
-    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz;
-         k += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t c = colInd[k];
-        const uint32_t slot = tRowPtr[c] + atomicAdd(&fill[c], 1u);
-        pos[slot] = (uint32_t)k;
-    }
-}
-
-// sort each segment of pos by value (insertion sort per thread), then gather rows/values
-__global__ void k_sort_gather(uint32_t m, const uint32_t* __restrict__ tRowPtr,
-                              uint32_t* __restrict__ pos, const uint32_t* __restrict__ rowOf,
-                              const double* __restrict__ val, uint32_t* __restrict__ tColInd,
-                              double* __restrict__ tVal)
-{
-    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < m;
-         c += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t b = tRowPtr[c], e = tRowPtr[c + 1];
-        for (uint32_t i = b + 1; i < e; ++i) {
-            const uint32_t key = pos[i];
-            uint32_t j = i;
-            while (j > b && pos[j - 1] > key) {
-                pos[j] = pos[j - 1];
-                --j;
-            }
-            pos[j] = key;
-        }
-        for (uint32_t i = b; i < e; ++i) {
-            const uint32_t p = pos[i];
-            tColInd[i] = rowOf[p];
-            if (val) tVal[i] = val[p];
-        }
-    }
-}
-
-// The transpose of a grid operator is the grid operator with every offset negated (the
-// same coefficients), in ascending order of the negated flattened offsets.
-static int grid_transpose(Ctx& c, const Mat& A, Mat& T)
-{
-    std::vector<int32_t> dx(A.skLen), dy(A.skLen), dz(A.skLen);
-    for (uint32_t k = 0; k < A.skLen; ++k) {
-        dx[k] = -A.gd[0][k];
-        dy[k] = -A.gd[1][k];
-        dz[k] = -A.gd[2][k];
-    }
-    return m_create_stencil(T, A.gdim[0], A.gdim[1], A.gdim[2], A.skLen, dx.data(), dy.data(),
-                            dz.data(), A.skVal, c.stream);
-}
-
-int m_transpose(Ctx& c, const Mat& A, Mat& T)
-{
-    if (A.grid) return grid_transpose(c, A, T);
-    const uint32_t m = A.mcol, n = A.nrow, nnz = A.nnz;
-    Mat R;
-    R.nrow = m;
-    R.mcol = n;
-    R.nnz = nnz;
-    R.dev = A.dev;
-    uint32_t *cnt = nullptr, *fill = nullptr, *pos = nullptr, *rowOf = nullptr;
-    cudaStream_t s = c.stream;
-    int e;
-    if ((e = dmalloc((void**)&R.rowPtr, ((size_t)m + 1) * 4, s)) ||
-        (e = dmalloc((void**)&R.colInd, (size_t)nnz * 4, s)) ||
-        (A.val && (e = dmalloc((void**)&R.val, (size_t)nnz * 8, s))) ||
-        (e = dmalloc((void**)&cnt, (size_t)m * 4, s)) || (e = dmalloc((void**)&fill, (size_t)m * 4, s)) ||
-        (e = dmalloc((void**)&pos, (size_t)nnz * 4, s)) ||
-        (e = dmalloc((void**)&rowOf, (size_t)nnz * 4, s))) {
-        m_free(R);
-        dev_free(cnt);
-        dev_free(fill);
-        dev_free(pos);
-        dev_free(rowOf);
-        return e;
-    }
-    const int gn = std::max(1, std::min(ceil_div(nnz, kBlock), c.nsm * 8));
-    const int gm = std::max(1, std::min(ceil_div(m, kBlock), c.nsm * 8));
-    const int gr = std::max(1, std::min(ceil_div(n, kBlock), c.nsm * 8));
-    FB_CUDA(cudaMemsetAsync(cnt, 0, (size_t)m * 4, s));
-    FB_CUDA(cudaMemsetAsync(fill, 0, (size_t)m * 4, s));
-    k_col_count<<<gn, kBlock, 0, s>>>(nnz, A.colInd, cnt);
-    k_scan<<<1, 1024, 0, s>>>(m, cnt, R.rowPtr);
-    k_row_of<<<gr, kBlock, 0, s>>>(n, A.rowPtr, rowOf);
-    k_scatter_pos<<<gn, kBlock, 0, s>>>(nnz, A.colInd, R.rowPtr, fill, pos);
-    k_sort_gather<<<gm, kBlock, 0, s>>>(m, R.rowPtr, pos, rowOf, A.val, R.colInd, R.val);
-    FB_CUDA(cudaGetLastError());
-    e = m_inspect(R, false, s);
-    dev_free(cnt);
-    dev_free(fill);
-    dev_free(pos);
-    dev_free(rowOf);
-    if (e) {
-        m_free(R);
-        return e;
-    }
-    R.diagConst = false; // the solvers on a transpose read its diagonal vector
-    R.diagValue = 0.0;
-    R.lanes = A.lanes;
-    T = R;
     return kOk;
 }
 
