@@ -1,4 +1,6 @@
-// batch.cu -- many independent Jacobi-PCG solves in one persistent launch.
+// batch.cu -- many independent Jacobi-PCG solves on one GPU. Systems whose vectors fit a
+// thread-block cluster's shared memory (65,536 values: 16,384 rows with four right-hand
+// sides) run in batch_resident.cuh; what follows is the kernels of larger ones.
 //
 // The systems are the diagonal blocks of one CSRx matrix (global row and column indices,
 // block k = rows sysRow[k]..sysRow[k+1]); each has nrhs right-hand sides stored right-hand-
@@ -19,6 +21,7 @@
 #include <vector>
 
 #include "../../include/fasp_b200.h"
+#include "batch_resident.cuh"
 #include "internal.h"
 
 namespace fb {
@@ -555,6 +558,102 @@ __global__ void batch_dinv(uint32_t N, const double* diag, double* d64, float* d
     }
 }
 
+// ---- the sliced copy of the matrix for the resident kernels --------------------------------
+
+// Per slice of 32 rows of one system: the longest row (in units of 32 entries that is the slice's
+// size); every row's length; *bad when a column leaves its system (the systems are the
+// diagonal blocks). slice -> system by a search of sliceBase.
+__global__ void batch_slices(uint32_t count, uint32_t slices, const uint32_t* __restrict__ sysRow,
+                             const uint32_t* __restrict__ sliceBase,
+                             const uint32_t* __restrict__ rowPtr,
+                             const uint32_t* __restrict__ colInd, uint32_t* __restrict__ wide,
+                             uint16_t* __restrict__ rowLen, unsigned long long* __restrict__ total,
+                             int* __restrict__ bad)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    unsigned long long sum = 0;
+    for (size_t w = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < slices;
+         w += ((size_t)gridDim.x * blockDim.x) >> 5) {
+        uint32_t lo = 0, hi = count;
+        while (hi - lo > 1) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (sliceBase[mid] <= w)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        const uint32_t s0 = sysRow[lo], s1 = sysRow[lo + 1];
+        const uint32_t row = s0 + (uint32_t)(w - sliceBase[lo]) * 32u + lane;
+        uint32_t len = 0;
+        if (row < s1) {
+            const uint32_t b = rowPtr[row], e = rowPtr[row + 1];
+            len = e - b;
+            for (uint32_t k = b; k < e; ++k)
+                if (colInd[k] < s0 || colInd[k] >= s1) *bad = 1;
+            rowLen[row] = (uint16_t)(len < 65535u ? len : 65535u);
+        }
+        const uint32_t m = __reduce_max_sync(0xffffffffu, len);
+        if (lane == 0) {
+            wide[w] = m;
+            sum += m;
+        }
+    }
+    if (lane == 0 && sum) atomicAdd(total, sum);
+}
+
+// Entry k of row r of slice w -> place (sliceOff[w] + k) * 32 + lane, its column relative to
+// the system.
+__global__ void batch_fill_slices(uint32_t count, uint32_t slices,
+                                  const uint32_t* __restrict__ sysRow,
+                                  const uint32_t* __restrict__ sliceBase,
+                                  const uint32_t* __restrict__ sliceOff,
+                                  const uint32_t* __restrict__ rowPtr,
+                                  const uint32_t* __restrict__ colInd,
+                                  const double* __restrict__ val, uint16_t* __restrict__ col,
+                                  double* __restrict__ sval, float* __restrict__ sval32)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    for (size_t w = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < slices;
+         w += ((size_t)gridDim.x * blockDim.x) >> 5) {
+        uint32_t lo = 0, hi = count;
+        while (hi - lo > 1) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (sliceBase[mid] <= w)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        const uint32_t s0 = sysRow[lo], s1 = sysRow[lo + 1];
+        const uint32_t row = s0 + (uint32_t)(w - sliceBase[lo]) * 32u + lane;
+        if (row >= s1) continue;
+        const uint32_t b = rowPtr[row], e = rowPtr[row + 1];
+        for (uint32_t k = b; k < e; ++k) {
+            const size_t o = ((size_t)sliceOff[w] + (k - b)) * 32 + lane;
+            col[o] = (uint16_t)(colInd[k] - s0);
+            sval[o] = val[k];
+            sval32[o] = (float)val[k];
+        }
+    }
+}
+
+// The resident kernels' size classes, largest systems first: cluster size and threads a
+// block. A class takes systems whose rows, split evenly over the cluster in whole slices, fit
+// the blocks' arrays (threads * values per thread / right-hand sides rows a block). Blocks
+// of 256 and 512 threads leave room for four and two on an SM, which hides the block barriers
+// of small systems.
+constexpr int kResClasses = 6;
+struct ResClass {
+    int cluster, threads;
+};
+constexpr ResClass kRes[kResClasses] = {{8, 1024}, {4, 1024}, {2, 1024}, {1, 1024}, {1, 512}, {1, 256}};
+
+// The rows of the largest system of class c.
+inline uint32_t res_rows(int c, uint32_t nr)
+{
+    const uint32_t per = (uint32_t)(kRes[c].threads * kResVals) / nr; // a multiple of 32
+    return std::min<uint32_t>(per * (uint32_t)kRes[c].cluster, 65536u);   // 16-bit columns
+}
+
 } // namespace fb
 
 using namespace fb;
@@ -574,16 +673,112 @@ struct fasp_gpu_batch_s {
     double*   resRel = nullptr;
     uint32_t* iters = nullptr;
     unsigned* queue = nullptr;
-    int       block = 256;  // autotuned
+    int       block = 256;  // of batch_pcg / batch_pcg_rel
     int       blocksPerSM = 4;
     double    lastMs = 0.0;
+    // systems of the resident kernels: order[far .. count), by class; order[0 .. far) are too
+    // large for a cluster and run in batch_pcg / batch_pcg_rel
+    uint32_t  far = 0;
+    uint32_t  cls[kResClasses + 1] = {}; // class c: order[cls[c] .. cls[c + 1])
+    uint32_t *sliceBase = nullptr, *sliceOff = nullptr;
+    uint16_t *rowLen = nullptr, *col = nullptr;
+    double*   sval = nullptr;
+    float*    sval32 = nullptr;
 };
 
 namespace {
 
+// Right-hand sides a resident kernel is built for: 1, 2 or 4 (3 run as 4, the last one zero).
+inline uint32_t res_rhs(uint32_t nrhs) { return nrhs <= 2 ? nrhs : 4; }
+
+template <typename T, int NR, int TH, bool REL>
+int launch_resident(fasp_gpu_batch_s& B, const ResArgs<T>& a, int cluster, bool follow)
+{
+    const auto kern = batch_resident<T, NR, TH, REL>;
+    const size_t smem = (size_t)3 * TH * kResVals * sizeof(T);
+    FB_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(TH);
+    cfg.gridDim = dim3((unsigned)cluster);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = B.c.stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int resident = 0;
+    FB_CUDA(cudaOccupancyMaxActiveClusters(&resident, (const void*)kern, &cfg));
+    cfg.gridDim = dim3((unsigned)(cluster * std::max(1, std::min(resident, (int)a.items))));
+    cfg.numAttrs = follow ? 2 : 1;
+    FB_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+    B.c.launches += 1;
+    return kOk;
+}
+
+template <typename T, int NR, bool REL>
+int launch_class(fasp_gpu_batch_s& B, const ResArgs<T>& a, const ResClass& k, bool follow)
+{
+    switch (k.threads) {
+        case 1024: return launch_resident<T, NR, 1024, REL>(B, a, k.cluster, follow);
+        case 512: return launch_resident<T, NR, 512, REL>(B, a, k.cluster, follow);
+        default: return launch_resident<T, NR, 256, REL>(B, a, k.cluster, follow);
+    }
+}
+
+// Every class of the resident systems, largest first; the classes follow one another
+// programmatically, so a class's blocks move in as the previous one's leave.
+template <typename T, bool REL>
+int run_resident(fasp_gpu_batch_s& B, ResArgs<T> a)
+{
+    const uint32_t* cls = B.cls;
+    cudaMemsetAsync(B.queue, 0, sizeof(unsigned) * (kResClasses + 1), B.c.stream);
+    unsigned* const queue = B.queue;
+    bool follow = false;
+    for (int k = 0; k < kResClasses; ++k) {
+        if (cls[k] == cls[k + 1]) continue;
+        a.first = cls[k];
+        a.items = cls[k + 1] - cls[k];
+        a.queue = queue + k;
+        int e;
+        switch (res_rhs(B.nrhs)) {
+            case 1: e = launch_class<T, 1, REL>(B, a, kRes[k], follow); break;
+            case 2: e = launch_class<T, 2, REL>(B, a, kRes[k], follow); break;
+            default: e = launch_class<T, 4, REL>(B, a, kRes[k], follow); break;
+        }
+        if (e) return e;
+        follow = true;
+    }
+    return kOk;
+}
+
+template <typename T>
+ResArgs<T> res_args(fasp_gpu_batch_s& B, const T* val, const T* dinv, const T* b, T* x,
+                    double relTol, uint32_t maxIter)
+{
+    return ResArgs<T>{0, 0, B.nrhs, B.M.nrow, B.sysRow, B.order, B.sliceBase, B.sliceOff, B.rowLen,
+                      B.col, val, dinv, b, x, B.iters, B.resRel, relTol, maxIter, nullptr, nullptr,
+                      nullptr, nullptr, 0.0};
+}
+
 template <typename T>
 int launch_batch(fasp_gpu_batch_s& B, BatchArgs<T> a)
 {
+    if (B.far < B.count) {
+        int e;
+        if constexpr (sizeof(T) == 8)
+            e = run_resident<T, false>(B, res_args<T>(B, B.sval, B.dinv, a.b, a.x, a.relTol, a.maxIter));
+        else
+            e = run_resident<T, false>(B, res_args<T>(B, B.sval32, B.dinv32, a.b, a.x, a.relTol, a.maxIter));
+        if (e) return e;
+    }
+    a.count = B.far;
+    if (a.count == 0) return kOk;
     const int grid = B.c.nsm * B.blocksPerSM;
     cudaMemsetAsync(B.queue, 0, sizeof(unsigned), B.c.stream);
     switch (B.nrhs) {
@@ -594,6 +789,81 @@ int launch_batch(fasp_gpu_batch_s& B, BatchArgs<T> a)
     }
     B.c.launches += 1;
     return cudaGetLastError() == cudaSuccess ? kOk : kErrCuda;
+}
+
+// Sorts the systems (ord, longest first) into the resident kernels' classes and builds the
+// sliced copy of the matrix. Columns outside their system: kErrMatData. Where padding the
+// slices would more than double the entries (one long row among short ones), or a row is longer
+// than a 16-bit length, every system runs in batch_pcg / batch_pcg_rel instead.
+int slice_systems(fasp_gpu_batch_s& B, const std::vector<uint32_t>& hs, std::vector<uint32_t>& ord)
+{
+    cudaStream_t s = B.c.stream;
+    const uint32_t count = B.count;
+    std::vector<uint32_t> base((size_t)count + 1, 0);
+    for (uint32_t k = 0; k < count; ++k) base[k + 1] = base[k] + (hs[k + 1] - hs[k] + 31) / 32;
+    const uint32_t slices = base[count];
+    uint32_t* wide = nullptr;
+    struct Seen {
+        unsigned long long total;
+        int                bad;
+    }* seen = nullptr;
+    int e;
+    auto get = [&](auto** p, size_t bytes) { return dev_alloc_bytes((void**)p, bytes + 16, s); };
+    if ((e = get(&B.sliceBase, ((size_t)count + 1) * 4)) || (e = get(&B.sliceOff, (size_t)slices * 4)) ||
+        (e = get(&B.rowLen, (size_t)B.M.nrow * 2)))
+        return e;
+    FB_CUDA(cudaMemcpyAsync(B.sysRow, hs.data(), hs.size() * 4, cudaMemcpyHostToDevice, s));
+    FB_CUDA(cudaMemcpyAsync(B.sliceBase, base.data(), base.size() * 4, cudaMemcpyHostToDevice, s));
+    if ((e = get(&wide, (size_t)slices * 4)) || (e = get(&seen, sizeof(Seen)))) {
+        dev_free(wide);
+        return e;
+    }
+    auto inspect = [&]() -> int {
+        const int g = std::max(1, std::min(ceil_div((long long)slices * 32, 256), 148 * 8));
+        FB_CUDA(cudaMemsetAsync(seen, 0, sizeof(Seen), s));
+        batch_slices<<<g, 256, 0, s>>>(count, slices, B.sysRow, B.sliceBase, B.M.rowPtr, B.M.colInd,
+                                       wide, B.rowLen, &seen->total, &seen->bad);
+        FB_CUDA(cudaGetLastError());
+        Seen h;
+        std::vector<uint32_t> off(slices);
+        FB_CUDA(cudaMemcpyAsync(&h, seen, sizeof(h), cudaMemcpyDeviceToHost, s));
+        FB_CUDA(cudaMemcpyAsync(off.data(), wide, (size_t)slices * 4, cudaMemcpyDeviceToHost, s));
+        FB_CUDA(cudaStreamSynchronize(s));
+        if (h.bad) return kErrMatData;
+        const bool fits = B.M.maxRowLen < 65535u && h.total * 32 <= 2ull * B.M.nnz + 32ull * slices;
+        const uint32_t nr = res_rhs(B.nrhs);
+        uint32_t at = 0; // ord is by falling size
+        while (at < count && (!fits || hs[ord[at] + 1] - hs[ord[at]] > res_rows(0, nr))) ++at;
+        B.far = B.cls[0] = at;
+        for (int k = 0; k < kResClasses; ++k) {
+            if (k + 1 < kResClasses)
+                while (at < count && hs[ord[at] + 1] - hs[ord[at]] > res_rows(k + 1, nr)) ++at;
+            else
+                at = count;
+            B.cls[k + 1] = at;
+        }
+        if (!fits) return kOk;
+        uint32_t sum = 0;
+        for (uint32_t w = 0; w < slices; ++w) {
+            const uint32_t m = off[w];
+            off[w] = sum;
+            sum += m;
+        }
+        const size_t ne = (size_t)sum * 32;
+        if ((e = get(&B.col, ne * 2)) || (e = get(&B.sval, ne * 8)) || (e = get(&B.sval32, ne * 4)))
+            return e;
+        FB_CUDA(cudaMemcpyAsync(B.sliceOff, off.data(), (size_t)slices * 4, cudaMemcpyHostToDevice, s));
+        batch_fill_slices<<<g, 256, 0, s>>>(count, slices, B.sysRow, B.sliceBase, B.sliceOff,
+                                            B.M.rowPtr, B.M.colInd, B.M.val, B.col, B.sval, B.sval32);
+        FB_CUDA(cudaGetLastError());
+        FB_CUDA(cudaStreamSynchronize(s));
+        return kOk;
+    };
+    e = inspect();
+    if (e) cudaStreamSynchronize(s);
+    dev_free(wide);
+    dev_free(seen);
+    return e;
 }
 
 } // namespace
@@ -620,46 +890,20 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
     int e = h->c.init(library_device());
     // the matrix upload validates the structure (CheckCSR) before any kernel reads it
     if (!e) e = m_upload(h->M, N, N, nnz, rowPtr, colInd, values, false, h->c.stream);
-    if (!e) {
-        // each row's columns must stay inside its own system (block diagonal)
-        std::vector<uint32_t> rp(N + 1), ci(nnz);
-        cudaMemcpy(rp.data(), h->M.rowPtr, (N + 1) * 4, cudaMemcpyDeviceToHost);
-        cudaMemcpy(ci.data(), h->M.colInd, (size_t)nnz * 4, cudaMemcpyDeviceToHost);
-        for (uint32_t k = 0; k < count && !e; ++k)
-            for (uint32_t i = hs[k]; i < hs[k + 1] && !e; ++i)
-                for (uint32_t q = rp[i]; q < rp[i + 1]; ++q)
-                    if (ci[q] < hs[k] || ci[q] >= hs[k + 1]) {
-                        e = kErrMatData;
-                        break;
-                    }
-    }
     h->count = count;
     h->nrhs = nrhs;
     const size_t vN = (size_t)nrhs * N;
     auto dm = [&](void** p, size_t bytes) {
         if (!e) e = dev_alloc_bytes(p, bytes + 16, h->c.stream);
     };
-    dm((void**)&h->sysRow, (count + 1) * 4);
-    dm((void**)&h->order, count * 4);
-    dm((void**)&h->dinv, N * 8);
-    dm((void**)&h->dinv32, N * 4);
-    dm((void**)&h->r64, vN * 8);
-    dm((void**)&h->z64, vN * 8);
-    dm((void**)&h->p0, vN * 8);
-    dm((void**)&h->p1, vN * 8);
-    dm((void**)&h->q64, vN * 8);
-    dm((void**)&h->b32, vN * 4);
-    dm((void**)&h->x32, vN * 4);
-    dm((void**)&h->r32, vN * 4);
-    dm((void**)&h->z32, vN * 4);
-    dm((void**)&h->p032, vN * 4);
-    dm((void**)&h->p132, vN * 4);
-    dm((void**)&h->q32, vN * 4);
+    dm((void**)&h->sysRow, ((size_t)count + 1) * 4);
+    dm((void**)&h->order, (size_t)count * 4);
+    dm((void**)&h->dinv, (size_t)N * 8);
+    dm((void**)&h->dinv32, (size_t)N * 4);
     dm((void**)&h->rnorm, (size_t)count * nrhs * 8);
     dm((void**)&h->resRel, (size_t)count * nrhs * 8);
     dm((void**)&h->iters, (size_t)count * nrhs * 4);
-    dm((void**)&h->queue, 16);
-    if (!e) e = h->M.ensure32(h->c.stream);
+    dm((void**)&h->queue, sizeof(unsigned) * (kResClasses + 1));
     if (!e) {
         // longest systems first
         std::vector<uint32_t> ord(count);
@@ -667,8 +911,29 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
         std::stable_sort(ord.begin(), ord.end(), [&](uint32_t a, uint32_t b) {
             return hs[a + 1] - hs[a] > hs[b + 1] - hs[b];
         });
-        cudaMemcpyAsync(h->sysRow, hs.data(), (count + 1) * 4, cudaMemcpyHostToDevice, h->c.stream);
-        cudaMemcpyAsync(h->order, ord.data(), count * 4, cudaMemcpyHostToDevice, h->c.stream);
+        e = slice_systems(*h, hs, ord);
+        if (!e && (cudaMemcpyAsync(h->order, ord.data(), (size_t)count * 4, cudaMemcpyHostToDevice,
+                                   h->c.stream) != cudaSuccess ||
+                   cudaStreamSynchronize(h->c.stream) != cudaSuccess))
+            e = kErrCuda;
+    }
+    // vectors in global memory: the refinement's, and those of systems too large for a cluster
+    dm((void**)&h->r64, vN * 8);
+    dm((void**)&h->b32, vN * 4);
+    dm((void**)&h->x32, vN * 4);
+    if (h->far) {
+        dm((void**)&h->z64, vN * 8);
+        dm((void**)&h->p0, vN * 8);
+        dm((void**)&h->p1, vN * 8);
+        dm((void**)&h->q64, vN * 8);
+        dm((void**)&h->r32, vN * 4);
+        dm((void**)&h->z32, vN * 4);
+        dm((void**)&h->p032, vN * 4);
+        dm((void**)&h->p132, vN * 4);
+        dm((void**)&h->q32, vN * 4);
+        if (!e) e = h->M.ensure32(h->c.stream);
+    }
+    if (!e) {
         batch_dinv<<<std::max(1, std::min(ceil_div(N, 256), 148 * 8)), 256, 0, h->c.stream>>>(
             N, h->M.diag, h->dinv, h->dinv32);
         if (cudaStreamSynchronize(h->c.stream) != cudaSuccess) e = kErrCuda;
@@ -690,7 +955,9 @@ int fasp_gpu_batch_destroy(fasp_gpu_batch h)
                     (void*)h->r64, (void*)h->z64, (void*)h->p0, (void*)h->p1, (void*)h->q64,
                     (void*)h->b32, (void*)h->x32, (void*)h->r32, (void*)h->z32,
                     (void*)h->p032, (void*)h->p132, (void*)h->q32, (void*)h->rnorm,
-                    (void*)h->resRel, (void*)h->iters, (void*)h->queue})
+                    (void*)h->resRel, (void*)h->iters, (void*)h->queue,
+                    (void*)h->sliceBase, (void*)h->sliceOff, (void*)h->rowLen, (void*)h->col,
+                    (void*)h->sval, (void*)h->sval32})
         dev_free(p);
     h->c.destroy();
     delete h;
@@ -732,15 +999,26 @@ int fasp_gpu_batch_solve(fasp_gpu_batch h, const double* b, double* x, double re
                            B.dinv32, nullptr, B.x32, B.r32, B.z32, B.p032, B.p132, B.q32,
                            B.iters, B.resRel, relTol, maxIter, B.queue};
         const BatchRel f{B.M.val, b, x, innerRelTol > 0 && innerRelTol < 1 ? innerRelTol : 1e-2};
-        const int grid = B.c.nsm * B.blocksPerSM;
-        cudaMemsetAsync(B.queue, 0, sizeof(unsigned), B.c.stream);
-        switch (nr) {
-            case 1: batch_pcg_rel<1><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
-            case 2: batch_pcg_rel<2><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
-            case 3: batch_pcg_rel<3><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
-            default: batch_pcg_rel<4><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+        if (B.far < cnt) {
+            ResArgs<float> r = res_args<float>(B, B.sval32, B.dinv32, nullptr, nullptr, relTol, maxIter);
+            r.val64 = B.sval;
+            r.b64 = b;
+            r.x64 = x;
+            r.delta = f.delta;
+            e = run_resident<float, true>(B, r);
         }
-        B.c.launches += 1;
+        a.count = B.far;
+        if (!e && a.count) {
+            const int grid = B.c.nsm * B.blocksPerSM;
+            cudaMemsetAsync(B.queue, 0, sizeof(unsigned), B.c.stream);
+            switch (nr) {
+                case 1: batch_pcg_rel<1><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+                case 2: batch_pcg_rel<2><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+                case 3: batch_pcg_rel<3><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+                default: batch_pcg_rel<4><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+            }
+            B.c.launches += 1;
+        }
         if (cudaGetLastError() != cudaSuccess) e = kErrCuda;
     } else {
         // FP64 refinement around FP32 inner solves, x0 = 0

@@ -413,8 +413,10 @@ typedef struct fasp_gpu_batch_s* fasp_gpu_batch;
 int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
                           const uint32_t* rowPtr, const uint32_t* colInd,
                           const double* values, uint32_t nrhs, fasp_gpu_batch* out);
-/* Thread-block shape of the persistent launch: block (128, 256 or 512 threads) and blocks
- * per SM; the autotuner in the Python/C++ layers times the choices. */
+/* Thread-block shape of the persistent launch that solves the systems too large for the
+ * on-chip kernels (more than 65,536 rows x right-hand sides): block (128, 256 or 512 threads)
+ * and blocks per SM; the autotuner in the Python/C++ layers times the choices. The on-chip
+ * kernels choose cluster and block by each system's size. */
 int fasp_gpu_batch_set_shape(fasp_gpu_batch bt, int block, int blocksPerSM);
 /* Solves all systems from x0 = 0 to ||r|| < relTol ||b|| per right-hand side (device b, x).
  * precision FASP_GPU_MIXED runs FP32 inner CG to innerRelTol inside FP64 refinement;
