@@ -101,18 +101,20 @@ __device__ __forceinline__ void bulk_copy_g2s_plain(void* dst, const void* src, 
 // instruction-bound). The copies start on 16-byte boundaries (the range starts are) and
 // round their length up to 16 bytes: at most 8 bytes past the last element, inside every
 // vector's allocation. False when a wait ran out: the block has then drained its copies in
-// flight (bounded) and stopped.
-template <typename T, typename Src, typename Consume, typename Ready>
+// flight (bounded) and stopped. BACK: the chunks from the last to the first.
+template <typename T, bool BACK = false, typename Src, typename Consume, typename Ready>
 __device__ __forceinline__ bool dc_stream(DcRing& ring, size_t e0, size_t e1, int nItem, Src src,
                                           Consume consume, Ready ready,
                                           uint32_t pre = (uint32_t)kDcStages)
 {
     constexpr uint32_t C = DcShape<T>::C;
     const uint32_t tid = threadIdx.x;
-    const uint32_t total = (uint32_t)((e1 - e0 + C - 1) / C) * (uint32_t)nItem;
+    const uint32_t chunks = (uint32_t)((e1 - e0 + C - 1) / C);
+    const uint32_t total = chunks * (uint32_t)nItem;
+    const size_t start = BACK && chunks ? e0 + (size_t)(chunks - 1) * C : e0;
     // the issuing thread's position: the next item to copy
     int iv = 0, is = 0;
-    size_t ib = e0;
+    size_t ib = start;
     auto issue = [&]() {
         const uint32_t len = (uint32_t)std::min((size_t)C, e1 - ib);
         const uint32_t bytes = (len * (uint32_t)sizeof(T) + 15u) & ~15u;
@@ -125,7 +127,7 @@ __device__ __forceinline__ bool dc_stream(DcRing& ring, size_t e0, size_t e1, in
         if (++is == kDcStages) is = 0;
         if (++iv == nItem) {
             iv = 0;
-            ib += C;
+            ib = BACK ? ib - C : ib + C;
         }
     };
     if (tid == 0) {
@@ -149,7 +151,7 @@ __device__ __forceinline__ bool dc_stream(DcRing& ring, size_t e0, size_t e1, in
     __syncthreads();
     int v = 0, st = 0;
     uint32_t ph = 0;
-    size_t base = e0;
+    size_t base = start;
     for (uint32_t k = 0; k < total; ++k) {
         // the consumers hold warp-collective sums: a warp consumes only if all its lanes saw
         // the bytes land
@@ -175,7 +177,7 @@ __device__ __forceinline__ bool dc_stream(DcRing& ring, size_t e0, size_t e1, in
         if (++st == kDcStages) st = 0, ph ^= 1u;
         if (++v == nItem) {
             v = 0;
-            base += C;
+            base = BACK ? base - C : base + C;
         }
     }
     return true;
@@ -546,7 +548,7 @@ __global__ void __launch_bounds__(kDcThreads, 2) k_dc_update(DcArgs<T> P, GmLayo
         if (v == wv) return P.w;
         return P.V + (size_t)(v - (WLAST ? 1 : 2)) * P.ld;
     };
-    dc_stream<T>(ring, e0, e1, nItem, src, [&](int v, size_t base, const T* st, uint32_t len) {
+    dc_stream<T, true>(ring, e0, e1, nItem, src, [&](int v, size_t base, const T* st, uint32_t len) {
         if (v == 0) {
             dc_load<T>(st, len, u);
 #pragma unroll
