@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <mutex>
 #include <set>
+#include <type_traits>
 #include <utility>
 
 #include "common.cuh"
@@ -259,7 +260,137 @@ struct DcApply {
     T*         wout;
 };
 
-// Value slots: a_l at l, then (with w) b_l at j + l, c at 2j, and d last.
+// The step's scalar work, in the last block of a dots pass: the totals of the partials, the
+// completed column j - 1 with its Givens step and the tentative column j. Value slots: a_l
+// at l, then (with w) b_l at j + l, c at 2j, and d last. Hs: shared memory for kDcMaxK *
+// (kDcMaxK + 2) doubles.
+template <bool HASW>
+__device__ __forceinline__ void dc_finish(Scratch s, const GmLayout& L, GmCtl* g, int j, int nv,
+                                          double* Hs)
+{
+    __shared__ double tot[kDcMaxNV];
+    __shared__ double col[kDcMaxK + 2], hcol[kDcMaxK], var[2];
+    __shared__ GmCtl gs;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    // The Hessenberg columns 0 .. j-2 ([j][j], row i from column i - 1), the tentative column
+    // j - 1 and the rotations, which earlier steps wrote, are asked for first, all threads at once;
+    // they arrive while the partials are summed.
+    constexpr int kHs = (kDcMaxK * kDcMaxK + kDcThreads - 1) / kDcThreads;
+    const size_t m = L.m;
+    double hs[kHs], hc = 0.0, hsn = 0.0, hcs = 0.0, hvar = 0.0;
+#pragma unroll
+    for (int q = 0; q < kHs; ++q) {
+        const int e = (int)tid + q * kDcThreads, i = j > 0 ? e / j : 0, l = e - i * j;
+        hs[q] = e < j * j && l + 1 >= i && l < j - 1 ? L.hraw[(size_t)i * m + l] : 0.0;
+    }
+    if ((int)tid < j) {
+        hc = L.hraw[(size_t)tid * m + (j - 1)];
+        hsn = L.hsin[tid];
+        hcs = L.hcos[tid];
+    }
+    if (tid < 2 && j >= 1) hvar = L.var[j - 1 + (int)tid];
+    if (tid == 32) gs = *g;
+    // totals: warp q adds value v = q, q + 8, ... over the blocks (lane l takes blocks l,
+    // l + 32, ... in order, then a shuffle tree); a lane's loads for a value are issued
+    // together, two values at a time
+    const uint32_t G = gridDim.x;
+    for (int v0 = wid; v0 < nv; v0 += 2 * kDcWarps) {
+        double x[2][kDcMaxGrid / 32];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < kDcMaxGrid / 32; ++q) {
+                const int v = v0 + h * kDcWarps;
+                const uint32_t b = lane + 32u * q;
+                x[h][q] = v < nv && b < G ? __ldcg(&s.partials[(size_t)v * G + b]) : 0.0;
+            }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            double a = 0.0;
+#pragma unroll
+            for (int q = 0; q < kDcMaxGrid / 32; ++q) a += x[h][q];
+            a = warp_reduce(a, kSum);
+            if (lane == 0 && v0 + h * kDcWarps < nv) tot[v0 + h * kDcWarps] = a;
+        }
+    }
+    double* snS = Hs + (size_t)kDcMaxK * kDcMaxK;
+    double* csS = snS + kDcMaxK;
+#pragma unroll
+    for (int q = 0; q < kHs; ++q) {
+        const int e = (int)tid + q * kDcThreads;
+        if (e < j * j) Hs[e] = hs[q];
+    }
+    if ((int)tid < j) {
+        snS[tid] = hsn;
+        csS[tid] = hcs;
+    }
+    if (tid < 2) var[tid] = hvar;
+    __syncthreads();
+#define HR(i, l) L.hraw[(size_t)(i) * m + (l)]
+    const double* A = tot;     // a_l
+    const double* B = tot + j; // b_l (with w)
+    double t = 1.0, tinv = 1.0;
+    if (j >= 1) {
+        // re-orthogonalisation of u: column j - 1 gains a, its subdiagonal is ||u - Q a||
+        double ssq = 0.0;
+        for (int l = 0; l < j; ++l) ssq = fma(A[l], A[l], ssq);
+        const double t2 = tot[nv - 1] - ssq;
+        t = t2 > 0.0 ? sqrt(t2) : (t2 <= 0.0 ? 0.0 : t2); // a NaN stays NaN
+        tinv = 1.0 / t;
+        if ((int)tid <= j) { // j <= kDcMaxK < kDcThreads
+            const double v = (int)tid < j ? hc + A[tid] : t;
+            col[tid] = v;
+            HR(tid, j - 1) = v;
+        }
+        __syncthreads();
+    }
+    // the tentative column j: h_i = (b_i - sum_l H(i, l) a_l) / t, rows i < j, in l order
+    double hj = 0.0, gco = 0.0;
+    if (HASW) {
+        if (j == 0) {
+            gco = hj = tot[2 * j];
+        } else {
+            for (int i = tid; i < j; i += kDcThreads) {
+                double acc = B[i];
+                for (int l = i > 0 ? i - 1 : 0; l < j; ++l)
+                    acc = fma(-(l == j - 1 ? col[i] : Hs[i * j + l]), A[l], acc);
+                hcol[i] = acc * tinv;
+            }
+            double ab = 0.0;
+            for (int l = 0; l < j; ++l) ab = fma(A[l], B[l], ab);
+            gco = (tot[2 * j] - ab) * tinv;
+            hj = (gco - t * A[j - 1]) * tinv;
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && j >= 1) { // iteration j: the Givens step on the completed column j - 1
+        auto C = [&](int i) -> double& { return col[i]; };
+        auto Sn = [&](int i) { return snS[i]; };
+        auto Cs = [&](int i) { return csS[i]; };
+        auto Var = [&](int i) -> double& { return var[i == j - 1 ? 0 : 1]; };
+        gm_givens_serial(L, j, j - 1, t, C, Sn, Cs, Var, &gs);
+        L.var[j - 1] = var[0];
+        L.var[j] = var[1];
+        *g = gs;
+    }
+    __syncthreads();
+    if (j >= 1)
+        for (int i = tid; i <= j; i += kDcThreads) L.hh[(size_t)i * m + (j - 1)] = col[i];
+    if constexpr (HASW) {
+        if (gs.stop) return;
+        for (int i = tid; i <= j; i += kDcThreads) HR(i, j) = i < j ? hcol[i] : hj;
+        for (int l = tid; l < j; l += kDcThreads) {
+            L.ca[l] = A[l];
+            L.cb[l] = B[l];
+        }
+        if (tid == 0) {
+            L.cs[0] = gco;
+            L.cs[1] = tinv;
+        }
+    }
+#undef HR
+}
+
 template <typename T, bool HASW, int SH = 0, int MODE = 0>
 __global__ void __launch_bounds__(kDcThreads, 2)
 k_dc_dots(DcArgs<T> P, Scratch s, GmLayout L, GmCtl* g, DcApply<T> Ap)
@@ -269,9 +400,6 @@ k_dc_dots(DcArgs<T> P, Scratch s, GmLayout L, GmCtl* g, DcApply<T> Ap)
     extern __shared__ __align__(16) unsigned char dc_raw[];
     DcRing& ring = *reinterpret_cast<DcRing*>(dc_raw);
     __shared__ double wacc[kDcWarps][kDcMaxNV];
-    __shared__ double tot[kDcMaxNV];
-    __shared__ double col[kDcMaxK + 2], hcol[kDcMaxK], var[2];
-    __shared__ GmCtl gs;
     __shared__ bool amLast;
     // launched programmatically after the product or the previous update pass: every input
     // may still be in flight until the grid dependency resolves; the update pass that
@@ -396,113 +524,7 @@ k_dc_dots(DcArgs<T> P, Scratch s, GmLayout L, GmCtl* g, DcApply<T> Ap)
     if (tid == 0) amLast = last_block_ticket(s.ticket);
     __syncthreads();
     if (!amLast) return;
-    // totals: warp q adds value v = q, q + 8, ... over the blocks (lane l takes blocks l,
-    // l + 32, ... in order, then a shuffle tree); a lane's loads for a value are issued
-    // together, two values at a time
-    const uint32_t G = gridDim.x;
-    for (int v0 = wid; v0 < nv; v0 += 2 * kDcWarps) {
-        double x[2][kDcMaxGrid / 32];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int q = 0; q < kDcMaxGrid / 32; ++q) {
-                const int v = v0 + h * kDcWarps;
-                const uint32_t b = lane + 32u * q;
-                x[h][q] = v < nv && b < G ? __ldcg(&s.partials[(size_t)v * G + b]) : 0.0;
-            }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            double a = 0.0;
-#pragma unroll
-            for (int q = 0; q < kDcMaxGrid / 32; ++q) a += x[h][q];
-            a = warp_reduce(a, kSum);
-            if (lane == 0 && v0 + h * kDcWarps < nv) tot[v0 + h * kDcWarps] = a;
-        }
-    }
-    // the finalize reads the Hessenberg columns 0 .. j-2 and the rotations from shared memory
-    // (the ring's stages are free now): loaded by all threads at once rather than one
-    // dependent global load at a time
-    double* Hs = reinterpret_cast<double*>(ring.st); // [j][j], row i from column i - 1
-    double* snS = Hs + (size_t)kDcMaxK * kDcMaxK;
-    double* csS = snS + kDcMaxK;
-    const size_t m = L.m;
-    for (int e = tid; e < j * j; e += kDcThreads) {
-        const int i = e / j, l = e - i * j;
-        if (l + 1 >= i && l < j - 1) Hs[e] = L.hraw[(size_t)i * m + l];
-    }
-    for (int i = tid; i < j; i += kDcThreads) {
-        snS[i] = L.hsin[i];
-        csS[i] = L.hcos[i];
-    }
-    if (tid == 32) gs = *g;
-    if (tid == 64 && j >= 1) {
-        var[0] = L.var[j - 1];
-        var[1] = L.var[j];
-    }
-    __syncthreads();
-#define HR(i, l) L.hraw[(size_t)(i) * m + (l)]
-    const double* A = tot;     // a_l
-    const double* B = tot + j; // b_l (with w)
-    double t = 1.0, tinv = 1.0;
-    if (j >= 1) {
-        // re-orthogonalisation of u: column j - 1 gains a, its subdiagonal is ||u - Q a||
-        double ssq = 0.0;
-        for (int l = 0; l < j; ++l) ssq = fma(A[l], A[l], ssq);
-        const double t2 = tot[nv - 1] - ssq;
-        t = t2 > 0.0 ? sqrt(t2) : (t2 <= 0.0 ? 0.0 : t2); // a NaN stays NaN
-        tinv = 1.0 / t;
-        for (int i = tid; i <= j; i += kDcThreads) {
-            const double v = i < j ? HR(i, j - 1) + A[i] : t;
-            col[i] = v;
-            HR(i, j - 1) = v;
-        }
-        __syncthreads();
-    }
-    // the tentative column j: h_i = (b_i - sum_l H(i, l) a_l) / t, rows i < j, in l order
-    double hj = 0.0, gco = 0.0;
-    if (HASW) {
-        if (j == 0) {
-            gco = hj = tot[2 * j];
-        } else {
-            for (int i = tid; i < j; i += kDcThreads) {
-                double acc = B[i];
-                for (int l = i > 0 ? i - 1 : 0; l < j; ++l)
-                    acc = fma(-(l == j - 1 ? col[i] : Hs[i * j + l]), A[l], acc);
-                hcol[i] = acc * tinv;
-            }
-            double ab = 0.0;
-            for (int l = 0; l < j; ++l) ab = fma(A[l], B[l], ab);
-            gco = (tot[2 * j] - ab) * tinv;
-            hj = (gco - t * A[j - 1]) * tinv;
-        }
-    }
-    __syncthreads();
-    if (tid == 0 && j >= 1) { // iteration j: the Givens step on the completed column j - 1
-        auto C = [&](int i) -> double& { return col[i]; };
-        auto Sn = [&](int i) { return snS[i]; };
-        auto Cs = [&](int i) { return csS[i]; };
-        auto Var = [&](int i) -> double& { return var[i == j - 1 ? 0 : 1]; };
-        gm_givens_serial(L, j, j - 1, t, C, Sn, Cs, Var, &gs);
-        L.var[j - 1] = var[0];
-        L.var[j] = var[1];
-        *g = gs;
-    }
-    __syncthreads();
-    if (j >= 1)
-        for (int i = tid; i <= j; i += kDcThreads) L.hh[(size_t)i * m + (j - 1)] = col[i];
-    if constexpr (HASW) {
-        if (gs.stop) return;
-        for (int i = tid; i <= j; i += kDcThreads) HR(i, j) = i < j ? hcol[i] : hj;
-        for (int l = tid; l < j; l += kDcThreads) {
-            L.ca[l] = A[l];
-            L.cb[l] = B[l];
-        }
-        if (tid == 0) {
-            L.cs[0] = gco;
-            L.cs[1] = tinv;
-        }
-    }
-#undef HR
+    dc_finish<HASW>(s, L, g, j, nv, reinterpret_cast<double*>(ring.st));
 }
 
 // ---- the update pass -----------------------------------------------------------------
@@ -597,6 +619,182 @@ __global__ void __launch_bounds__(kDcThreads, 2) k_dc_update(DcArgs<T> P, GmLayo
     }, ready, WLAST ? (uint32_t)wv : (uint32_t)kDcStages);
 }
 
+// ---- both passes without the ring (FP64, systems of up to kDcDirect groups a thread) --------
+// A system of a few hundred thousand rows leaves the ring one chunk a block: the pass is then
+// a chain of one wait, one block barrier and one refill per vector. Here a thread
+// holds its NG 16-byte groups of u and w and loads its groups of 8 basis vectors at once, with no
+// barrier before the block's sums. Measured on B200 (a GMRES(30) step, product included): 36K rows
+// 33.3 -> 18.5 us, 262K rows 38.3 -> 27.3 us. With four groups a thread (314K rows) it
+// measured slower than the ring, 40.6 against 37.5 us, and in several turns over a larger
+// system more so (885K rows 83.9 against 61.7 us): few loads in flight per SM once its registers
+// allow two blocks only.
+constexpr int kDcDirect = 2;
+
+// Groups base + i * 256 + tid of a vector, i < NG; elements at or past n read as zero.
+__device__ __forceinline__ double2 dc_group(const double* v, uint32_t g, uint32_t n)
+{
+    if (2u * g + 1u < n) return *reinterpret_cast<const double2*>(v + 2u * (size_t)g);
+    return make_double2(2u * g < n ? v[2u * (size_t)g] : 0.0, 0.0);
+}
+
+// MODE 0, 1, 2: the pass also forms w = A M u (k_gm_apply's modes), each thread its own rows
+// (row_apply: the bits of the product kernel), and stores it for the update pass; -1: w is
+// given, or there is none.
+template <bool HASW, int NG, int MODE>
+__global__ void __launch_bounds__(kDcThreads, 2)
+k_dc_dots_direct(DcArgs<double> P, Scratch s, GmLayout L, GmCtl* g, DcApply<double> Ap)
+{
+    __shared__ double wacc[kDcWarps][kDcMaxNV];
+    __shared__ double Hs[kDcMaxK * (kDcMaxK + 2)];
+    __shared__ bool amLast;
+    pdl_wait();
+    pdl_release();
+    if (g->stop) return;
+    const int j = P.j, nv = HASW ? 2 * j + 2 : j + 1;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n = P.n;
+    const uint32_t g0 = blockIdx.x * (uint32_t)(NG * kDcThreads) + tid;
+    double2 u[NG], w[NG];
+    double uu = 0.0, uw = 0.0;
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+        u[i] = dc_group(P.V + (size_t)j * P.ld, g0 + i * kDcThreads, n);
+        w[i] = HASW && MODE < 0 ? dc_group(P.w, g0 + i * kDcThreads, n) : make_double2(0.0, 0.0);
+    }
+    if constexpr (MODE >= 0) {
+        const double* uv = P.V + (size_t)j * P.ld;
+        const double* dinv = Ap.dinv;
+        auto xv = [&](uint32_t k) { return MODE == 1 ? uv[k] * dinv[k] : uv[k]; };
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            const uint32_t r = 2u * (g0 + i * kDcThreads);
+            double t[2] = {0.0, 0.0};
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (r + e < n) {
+                    t[e] = row_apply<double, false>(Ap.A, r + e, xv);
+                    if (MODE == 2) t[e] = t[e] * dinv[r + e];
+                    Ap.wout[r + e] = t[e];
+                }
+            w[i] = make_double2(t[0], t[1]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+        uu = fma(u[i].y, u[i].y, fma(u[i].x, u[i].x, uu));
+        uw = fma(u[i].y, w[i].y, fma(u[i].x, w[i].x, uw));
+    }
+    for (int l0 = 0; l0 < j; l0 += 8) {
+        double x[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) x[q] = 0.0;
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            double2 v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                v[q] = l0 + q < j ? dc_group(P.V + (size_t)(l0 + q) * P.ld, g0 + i * kDcThreads, n)
+                                  : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                x[q] = fma(v[q].y, u[i].y, fma(v[q].x, u[i].x, x[q]));
+                if (HASW) x[q + 8] = fma(v[q].y, w[i].y, fma(v[q].x, w[i].x, x[q + 8]));
+            }
+        }
+        const double sum = warp_sum16(x);
+        const int r = (int)(lane >> 1) & 15, q = r & 7;
+        if (!(lane & 1) && l0 + q < j && (HASW || r < 8)) wacc[wid][(r < 8 ? 0 : j) + l0 + q] = sum;
+    }
+    uu = warp_reduce(uu, kSum);
+    uw = warp_reduce(uw, kSum);
+    if (lane == 0) {
+        if (HASW) wacc[wid][2 * j] = uw;
+        wacc[wid][nv - 1] = uu;
+    }
+    __syncthreads();
+    for (int v = tid; v < nv; v += kDcThreads) {
+        double a = 0.0;
+        for (int q = 0; q < kDcWarps; ++q) a += wacc[q][v];
+        s.partials[(size_t)v * gridDim.x + blockIdx.x] = a;
+    }
+    __syncthreads();
+    if (tid == 0) amLast = last_block_ticket(s.ticket);
+    __syncthreads();
+    if (!amLast) return;
+    dc_finish<HASW>(s, L, g, j, nv, Hs);
+}
+
+template <int NG>
+__global__ void __launch_bounds__(kDcThreads, 2)
+k_dc_update_direct(DcArgs<double> P, GmLayout L, const GmCtl* g, bool formed)
+{
+    __shared__ double ca[kDcMaxK], cb[kDcMaxK];
+    pdl_release();
+    const int j = P.j;
+    const uint32_t tid = threadIdx.x, n = P.n;
+    const uint32_t g0 = blockIdx.x * (uint32_t)(NG * kDcThreads) + tid;
+    // u is read while the dots pass finalises, and w unless that pass forms it; the
+    // coefficients once it has finished
+    double2 u[NG], w[NG], sa[NG], sb[NG];
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+        u[i] = dc_group(P.V + (size_t)j * P.ld, g0 + i * kDcThreads, n);
+        w[i] = formed ? make_double2(0.0, 0.0) : dc_group(P.w, g0 + i * kDcThreads, n);
+        sa[i] = sb[i] = make_double2(0.0, 0.0);
+    }
+    pdl_wait();
+    if (g->stop) return;
+    if (formed)
+#pragma unroll
+        for (int i = 0; i < NG; ++i) w[i] = dc_group(P.w, g0 + i * kDcThreads, n);
+    for (int l = tid; l < j; l += kDcThreads) {
+        ca[l] = L.ca[l];
+        cb[l] = L.cb[l];
+    }
+    const double gco = L.cs[0], tinv = L.cs[1];
+    __syncthreads();
+    for (int l0 = 0; l0 < j; l0 += 8) {
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            double2 v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                v[q] = l0 + q < j ? dc_group(P.V + (size_t)(l0 + q) * P.ld, g0 + i * kDcThreads, n)
+                                  : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                if (l0 + q >= j) break;
+                const double al = ca[l0 + q], bl = cb[l0 + q];
+                sa[i].x = fma(al, v[q].x, sa[i].x);
+                sa[i].y = fma(al, v[q].y, sa[i].y);
+                sb[i].x = fma(bl, v[q].x, sb[i].x);
+                sb[i].y = fma(bl, v[q].y, sb[i].y);
+            }
+        }
+    }
+    double* qj = P.V + (size_t)j * P.ld;
+    double* un = P.V + (size_t)(j + 1) * P.ld;
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+        const uint32_t gi = g0 + i * kDcThreads;
+        double2 q, o;
+        q.x = j > 0 ? (u[i].x - sa[i].x) * tinv : u[i].x;
+        q.y = j > 0 ? (u[i].y - sa[i].y) * tinv : u[i].y;
+        o.x = fma(-q.x, gco, w[i].x - sb[i].x);
+        o.y = fma(-q.y, gco, w[i].y - sb[i].y);
+        if (j > 0) {
+            o.x *= tinv;
+            o.y *= tinv;
+        }
+        if (2u * gi + 1u < n) {
+            if (j > 0) *reinterpret_cast<double2*>(qj + 2u * (size_t)gi) = q;
+            *reinterpret_cast<double2*>(un + 2u * (size_t)gi) = o;
+        } else if (2u * gi < n) {
+            if (j > 0) qj[2u * (size_t)gi] = q.x;
+            un[2u * (size_t)gi] = o.x;
+        }
+    }
+}
+
 // ---- launchers -------------------------------------------------------------------------
 
 // The shared-memory opt-in above 48 KB, once per kernel and device.
@@ -642,12 +840,46 @@ static int dc_grid(const Ctx& c, const void* fn, uint32_t n, int nv)
     return std::max(g, 1);
 }
 
+// Groups a thread of the direct passes (1 or 2, on at most two blocks per SM), or 0: the ring.
+// The grid is the same for both passes of a step.
+static int dc_direct(const Ctx& c, uint32_t n, int nv, int* grid)
+{
+    const uint32_t groups = (n + 1) / 2, per = (uint32_t)kDcThreads;
+    const uint32_t most = std::min<uint32_t>(
+        (uint32_t)std::min(2 * c.nsm, kDcMaxGrid),
+        (uint32_t)((kMaxRedValues * kMaxGrid) / std::max(nv, 1)));
+    const uint32_t blocks = (groups + per - 1) / per;
+    const int ng = (int)((blocks + most - 1) / most);
+    if (ng > kDcDirect) return 0;
+    *grid = (int)((blocks + (uint32_t)ng - 1) / (uint32_t)ng);
+    return ng;
+}
+
+static bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
 template <typename T>
 int dc_dots(Ctx& c, uint32_t n, int j, T* V, size_t ld, const T* w, const GmLayout& L,
             GmCtl* g)
 {
     if (j > kDcMaxK) return kErrInputPar;
     DcArgs<T> P{V, ld, w, n, j};
+    if constexpr (std::is_same<T, double>::value) {
+        int grid = 0;
+        const int ng = aligned16(V) && ld % 2 == 0 && (!w || aligned16(w))
+                           ? dc_direct(c, n, 2 * j + 2, &grid)
+                           : 0;
+        if (ng) {
+            ++c.launches;
+            auto go = [&](auto kern) {
+                return dc_launch(kern, grid, 0, c.stream, P, c.red, L, g, DcApply<double>{});
+            };
+            const int e = w ? (ng == 1 ? go(k_dc_dots_direct<true, 1, -1>) : go(k_dc_dots_direct<true, 2, -1>))
+                            : (ng == 1 ? go(k_dc_dots_direct<false, 1, -1>) : go(k_dc_dots_direct<false, 2, -1>));
+            if (e) return e;
+            FB_CUDA(cudaGetLastError());
+            return kOk;
+        }
+    }
     DcApply<T> none{};
     ++c.launches;
     int e;
@@ -667,11 +899,37 @@ int dc_dots(Ctx& c, uint32_t n, int j, T* V, size_t ld, const T* w, const GmLayo
     return kOk;
 }
 
+// The direct dots pass with the product in it (FP64, thread-per-row forms); kErrInputPar where
+// it does not apply and the caller launches the product and dc_dots.
+static int dc_direct_apply(Ctx& c, const CSRView<double>& A, int mode, const double* dinv, uint32_t n,
+                           int j, double* V, size_t ld, double* w, const GmLayout& L, GmCtl* g)
+{
+    int grid = 0;
+    const int ng = aligned16(V) && ld % 2 == 0 && aligned16(w) ? dc_direct(c, n, 2 * j + 2, &grid) : 0;
+    if (!ng) return kErrInputPar;
+    DcArgs<double> P{V, ld, w, n, j};
+    DcApply<double> Ap{A, dinv, w};
+    ++c.launches;
+    auto go = [&](auto kern) { return dc_launch(kern, grid, 0, c.stream, P, c.red, L, g, Ap); };
+    auto by = [&](auto M) {
+        constexpr int MODE = decltype(M)::value;
+        return ng == 1 ? go(k_dc_dots_direct<true, 1, MODE>) : go(k_dc_dots_direct<true, 2, MODE>);
+    };
+    const int e = mode == 0 ? by(std::integral_constant<int, 0>{})
+                            : mode == 1 ? by(std::integral_constant<int, 1>{})
+                                        : by(std::integral_constant<int, 2>{});
+    if (e) return e;
+    FB_CUDA(cudaGetLastError());
+    return kOk;
+}
+
 template <typename T>
 int dc_dots_apply(Ctx& c, const CSRView<T>& A, int mode, const T* dinv, uint32_t n, int j,
                   T* V, size_t ld, T* w, const GmLayout& L, GmCtl* g)
 {
     if (j > kDcMaxK) return kErrInputPar;
+    if constexpr (std::is_same<T, double>::value)
+        return dc_direct_apply(c, A, mode, dinv, n, j, V, ld, w, L, g);
     const int sh = stencil_vec_shape(A, V + (size_t)j * ld, w,
                                      mode == 0 ? (const void*)w : (const void*)dinv);
     if (!sh) return kErrInputPar;
@@ -697,12 +955,25 @@ int dc_dots_apply(Ctx& c, const CSRView<T>& A, int mode, const T* dinv, uint32_t
 
 template <typename T>
 int dc_update(Ctx& c, uint32_t n, int j, T* V, size_t ld, const T* w, const GmLayout& L,
-              const GmCtl* g, bool wlast)
+              const GmCtl* g, bool formed)
 {
     if (j > kDcMaxK) return kErrInputPar;
     DcArgs<T> P{V, ld, w, n, j};
     ++c.launches;
-    auto kern = wlast ? k_dc_update<T, true> : k_dc_update<T, false>;
+    if constexpr (std::is_same<T, double>::value) {
+        int grid = 0;
+        const int ng = aligned16(V) && ld % 2 == 0 && aligned16(w)
+                           ? dc_direct(c, n, 2 * j + 2, &grid)
+                           : 0;
+        if (ng) {
+            auto go = [&](auto kern) { return dc_launch(kern, grid, 0, c.stream, P, L, g, formed); };
+            const int e = ng == 1 ? go(k_dc_update_direct<1>) : go(k_dc_update_direct<2>);
+            if (e) return e;
+            FB_CUDA(cudaGetLastError());
+            return kOk;
+        }
+    }
+    auto kern = formed ? k_dc_update<T, true> : k_dc_update<T, false>;
     dc_optin((const void*)kern);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)dc_grid(c, (const void*)kern, n, 1));

@@ -72,11 +72,30 @@ __device__ __forceinline__ void gm_givens_serial(const GmLayout& L, int count, i
         return;
     }
     L.out[1] = 1.0;
-    for (int j = 1; j < count; ++j) {
-        t = C(j - 1);
-        C(j - 1) = S(j - 1) * C(j) + K(j - 1) * t;
-        C(j) = -S(j - 1) * t + K(j - 1) * C(j);
+    // the rotations one after another, eight at a time: their operands are loaded together,
+    // ahead of the chain through the running entry (one at a time, every rotation had waited
+    // for its own loads behind the previous one's stores)
+    double run = C(0);
+    for (int j0 = 1; j0 < count; j0 += 8) {
+        double cj[8], sj[8], kj[8], done[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (j0 + u < count) {
+                cj[u] = C(j0 + u);
+                sj[u] = S(j0 + u - 1);
+                kj[u] = K(j0 + u - 1);
+            }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (j0 + u < count) {
+                done[u] = sj[u] * cj[u] + kj[u] * run;
+                run = -sj[u] * run + kj[u] * cj[u];
+            }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (j0 + u < count) C(j0 + u - 1) = done[u];
     }
+    if (count > 0) C(count - 1) = run;
     t = C(count) * C(count);
     t += C(c1) * C(c1);
     t = sqrt(t);
@@ -100,12 +119,14 @@ __device__ __forceinline__ void gm_givens_serial(const GmLayout& L, int count, i
 
 template <typename T>
 int dc_dots(Ctx& c, uint32_t n, int j, T* V, size_t ld, const T* w, const GmLayout& L, GmCtl* g);
+// formed: the dots pass before it wrote w.
 template <typename T>
 int dc_update(Ctx& c, uint32_t n, int j, T* V, size_t ld, const T* w, const GmLayout& L,
-              const GmCtl* g, bool wlast);
+              const GmCtl* g, bool formed);
 // The dots pass of step j forming the product w = A M u itself (mode 0: A u, 1: A (D u),
-// 2: D (A u)) on stencil masks of the fixed 5- or 7-point shape; kErrInputPar when the
-// matrix or the vectors do not have that form (the caller then launches the product).
+// 2: D (A u)): FP32 on stencil masks of the fixed 5- or 7-point shape, FP64 on any
+// thread-per-row form of a system small enough for the direct passes; kErrInputPar
+// otherwise (the caller then launches the product).
 template <typename T>
 int dc_dots_apply(Ctx& c, const CSRView<T>& A, int mode, const T* dinv, uint32_t n, int j,
                   T* V, size_t ld, T* w, const GmLayout& L, GmCtl* g);

@@ -1891,10 +1891,17 @@ static int gm_cycle_device(SolverImpl& S, const GmLayout& L, T* V, uint32_t step
         const uint32_t j = k - 1;
         const T* u = V + j * ld;
         int e;
+        // FP64 systems small enough for the direct passes form the product there too
+        bool formed = fuse;
         if (fuse) {
             if ((e = dc_dots_apply<T>(c, AV, mode, dinv, n, (int)j, V, ld, wbuf, L, S.gmc)))
                 return e;
-        } else {
+        } else if (sizeof(T) == 8 && S.A->lanes == 1) {
+            e = dc_dots_apply<T>(c, AV, mode, dinv, n, (int)j, V, ld, wbuf, L, S.gmc);
+            if (e && e != kErrInputPar) return e;
+            formed = !e;
+        }
+        if (!formed) {
             if (mode == 0)
                 gm_apply_launch<T, 0>(c, *S.A, AV, u, dinv, wbuf, stop);
             else if (mode == 1)
@@ -1904,7 +1911,7 @@ static int gm_cycle_device(SolverImpl& S, const GmLayout& L, T* V, uint32_t step
             ++c.launches;
             if ((e = dc_dots<T>(c, n, (int)j, V, ld, wbuf, L, S.gmc))) return e;
         }
-        if ((e = dc_update<T>(c, n, (int)j, V, ld, wbuf, L, S.gmc, fuse))) return e;
+        if ((e = dc_update<T>(c, n, (int)j, V, ld, wbuf, L, S.gmc, formed))) return e;
     }
     if (dc) {
         int e;

@@ -193,3 +193,26 @@ def test_dcgs2_restart_48(gpu, prec):
     kw = dict(restart=48, maxRestart=48, minRestart=48, prec=prec)
     _agree(A, b, _run(gpu, A, b, "dcgs2", **kw), _run(gpu, A, b, "cgs2", **kw),
            tol=1e-8, xtol=1e-6 if prec == "FP64" else 1e-5)
+
+
+@pytest.mark.parametrize("n", [511, 512, 513, 151551, 151552, 151554, 303103, 303104, 303106])
+@pytest.mark.parametrize("lanes", [1, 2])
+def test_dcgs2_direct_passes(gpu, n, lanes):
+    """FP64 systems of up to two 16-byte groups a thread run without the ring, forming the product
+    in the dots pass (one thread per row) or taking it (lanes 2): at the sizes where the groups a
+    thread change on 148 SMs, one row below and past the last."""
+    capi, sol = gpu
+    A = _convection_1d(n, n)
+    b = A.matvec(np.random.default_rng(n).uniform(-1, 1, n))
+    out = []
+    for orth in ("DCGS2", "CGS2"):
+        s = sol.configure("gmres", maxIter=2000, relTol=1e-8, absTol=0.0, restart=30, pcd="jacobi",
+                          pcdWeight=2.0 / 3.0, pcdIter=1)
+        s.SetOrth(getattr(capi, "ORTH_" + orth))
+        M = sol.MAT(A)
+        M.SetLanes(lanes)
+        s.Setup(M)
+        x = np.zeros(n)
+        code = s.Solve(b, x)
+        out.append((code, s.GetIterations(), x, s.History()))
+    _agree(A, b, *out)
