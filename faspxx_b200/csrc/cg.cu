@@ -635,13 +635,14 @@ __global__ void __launch_bounds__(kBlock, (V4 ? 3 : (L > 1 ? 4 : (sizeof(T) == 4
         double2* pn2 = reinterpret_cast<double2*>(pNew);
         double2* q2 = reinterpret_cast<double2*>(q);
         constexpr int MID = SH / 2;
-        auto pat = [&](uint32_t h) { // the gathered p of rows 2h, 2h+1
-            const double2 zz = z2[h];
+        auto from = [&](const double2& zz, const double2& o) { // p of two rows
             const double a = JZ == 2 ? (double)zc * zz.x : zz.x;
             const double b = JZ == 2 ? (double)zc * zz.y : zz.y;
             if (!mode) return make_double2(a, b);
-            const double2 o = po2[h];
             return make_double2(fma((double)beta, o.x, a), fma((double)beta, o.y, b));
+        };
+        auto pat = [&](uint32_t h) { // the gathered p of rows 2h, 2h+1
+            return from(z2[h], mode ? po2[h] : zero);
         };
         auto masks = [&](uint32_t g, uint32_t& m0, uint32_t& m1) {
             if (A.gnz) {
@@ -690,8 +691,12 @@ __global__ void __launch_bounds__(kBlock, (V4 ? 3 : (L > 1 ? 4 : (sizeof(T) == 4
                 const uint32_t k0 = (w / cols) * C, k1 = min(k0 + C, nz);
                 uint32_t g = w % cols + k0 * cols;
                 double2 below = k0 > 0 ? pat(g - cols) : zero, cur = pat(g);
+                double2 above = k0 + 1 < nz ? pat(g + cols) : zero;
                 for (uint32_t k = k0; k < k1; ++k, g += cols) {
-                    const double2 above = k + 1 < nz ? pat(g + cols) : zero;
+                    // the plane after the next, one step ahead of its use
+                    const bool more = k + 2 < nz && k + 1 < k1;
+                    const double2 zN = more ? z2[g + 2 * cols] : zero;
+                    const double2 oN = more && mode ? po2[g + 2 * cols] : zero;
                     uint32_t m0, m1;
                     masks(g, m0, m1);
                     const uint32_t ga = g + (uint32_t)o1, gb = g + (uint32_t)o5;
@@ -708,6 +713,7 @@ __global__ void __launch_bounds__(kBlock, (V4 ? 3 : (L > 1 ? 4 : (sizeof(T) == 4
                     rows2(g, m0, m1, xs, cur);
                     below = cur;
                     cur = above;
+                    above = from(zN, oN);
                 }
             }
           }
