@@ -1,0 +1,401 @@
+// mg.cu -- the MG cycle with transfer operators as few launches per level as its data flow allows,
+// and Jacobi::Solve on small matrices in shared memory.
+//
+// A cycle whose smoothers and coarse solver run a fixed number of sweeps (minIter = maxIter) reads
+// no norm on the host. As separate kernels a level with two sweeps before and after took some 20
+// launches: NormInf(x) for MAT::Residual's shortcut, a residual and an update per sweep (the
+// Galerkin levels' rows are longer than one thread takes), vector resets, a product and an
+// addition per transfer. Coarse levels are nothing but launch and reduction latency: on B200 a
+// V(2,2) cycle took 330 us at 31^3 and 800 us at 127^3. Here a level takes one launch for
+// its first two sweeps (from x = 0), one a sweep after that, one residual, one restriction and
+// one prolongation that also corrects x; levels of up to 1,024 rows take one launch for all their
+// sweeps. NormInf(x), which a residual's shortcut test needs, is an atomic maximum of the bits
+// of |x| in the kernel that writes x: a maximum does not depend on order, so the test is exact
+// and reruns are the same.
+#include "solver.h"
+
+namespace fb {
+namespace {
+
+using Bits = unsigned long long;
+
+__device__ __forceinline__ double from_bits(const Bits* p)
+{
+    return __longlong_as_double((long long)*(const volatile Bits*)p);
+}
+
+// *out = max(*out, max over the block of m >= 0); every thread calls it.
+__device__ __forceinline__ void put_max(double m, Bits* out)
+{
+    __shared__ double sh[32];
+    m = warp_reduce(m, kMax);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = threadIdx.x < ((blockDim.x + 31) >> 5) ? sh[threadIdx.x] : 0.0;
+        m = warp_reduce(m, kMax);
+        if (threadIdx.x == 0 && m > 0.0) atomicMax(out, (Bits)__double_as_longlong(m));
+    }
+}
+
+// Rows of A on L lanes each (L = 1: one thread, block tiles where the view has them):
+// own(row, sum) on the row's first lane.
+template <int L, typename XV, typename OWN>
+__device__ __forceinline__ void rows_of(const CSRView<double>& A, XV xv, OWN own)
+{
+    if (L == 1) {
+        for_rows<double, false>(A, xv, own);
+        return;
+    }
+    const uint32_t lane = threadIdx.x & (L - 1);
+    const size_t stride = (size_t)gridDim.x * blockDim.x / L;
+    const size_t first = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / L;
+    for (size_t r0 = first - (threadIdx.x & 31) / L; r0 < A.nrow; r0 += stride) { // warp-uniform
+        const size_t row = r0 + (threadIdx.x & 31) / L;
+        double s = 0.0;
+        if (row < A.nrow) {
+            const uint32_t b = A.rowPtr[row], e = A.rowPtr[row + 1];
+            for (uint32_t k = b + lane; k < e; k += L)
+                s = fma(ld_stream(A.val + k), xv(ld_stream(A.colInd + k)), s);
+        }
+        s = group_sum<L>(s);
+        if (lane == 0 && row < A.nrow) own(row, s);
+    }
+}
+
+// One Jacobi sweep, xout = xin + dinv .* r with r = b - A xin, or r = b when NormInf(xin) (*in)
+// is below CLOSE_ZERO (MAT.cxx:455-476, Iter.cxx:83-92). TWO: the first two sweeps from
+// x = 0, whose first is dinv .* b, formed where it is gathered; *in is its NormInf.
+template <int L, bool TWO>
+__global__ void __launch_bounds__(kBlock) k_mg_sweep(CSRView<double> A, const double* __restrict__ b,
+                                                     const double* __restrict__ xin,
+                                                     const double* __restrict__ dinv,
+                                                     double* __restrict__ xout,
+                                                     const Bits* __restrict__ in, Bits* out)
+{
+    pdl_wait();
+    pdl_release();
+    const bool shortcut = from_bits(in) < kCloseZero;
+    double m = 0.0;
+    auto x0 = [&](size_t j) { return TWO ? b[j] * dinv[j] : xin[j]; };
+    auto own = [&](size_t i, double sum) {
+        const double xi = x0(i) + (b[i] - sum) * dinv[i];
+        xout[i] = xi;
+        m = fmax(m, fabs(xi));
+    };
+    if (shortcut)
+        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.nrow;
+             i += (size_t)gridDim.x * blockDim.x)
+            own(i, 0.0);
+    else
+        rows_of<L>(A, [&](uint32_t j) { return x0(j); }, own);
+    put_max(m, out);
+}
+
+// The first sweep from x = 0: x = dinv .* b.
+__global__ void __launch_bounds__(kBlock) k_mg_first(uint32_t n, const double* __restrict__ b,
+                                                     const double* __restrict__ dinv,
+                                                     double* __restrict__ x, Bits* out)
+{
+    pdl_wait();
+    pdl_release();
+    double m = 0.0;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (size_t)gridDim.x * blockDim.x) {
+        const double xi = b[i] * dinv[i];
+        x[i] = xi;
+        m = fmax(m, fabs(xi));
+    }
+    put_max(m, out);
+}
+
+// bc = R r, and NormInf(dinv .* bc), the coarse level's first sweep.
+template <int L>
+__global__ void __launch_bounds__(kBlock) k_mg_restrict(CSRView<double> R, const double* __restrict__ r,
+                                                        double* __restrict__ bc,
+                                                        const double* __restrict__ dinv, Bits* out)
+{
+    pdl_wait();
+    pdl_release();
+    double m = 0.0;
+    rows_of<L>(R, [&](uint32_t j) { return r[j]; }, [&](size_t i, double s) {
+        bc[i] = s;
+        m = fmax(m, fabs(s * dinv[i]));
+    });
+    put_max(m, out);
+}
+
+// x += P e.
+template <int L>
+__global__ void __launch_bounds__(kBlock) k_mg_correct(CSRView<double> P, const double* __restrict__ e,
+                                                       double* __restrict__ x, Bits* out)
+{
+    pdl_wait();
+    pdl_release();
+    double m = 0.0;
+    rows_of<L>(P, [&](uint32_t j) { return e[j]; }, [&](size_t i, double s) {
+        const double xi = x[i] + s;
+        x[i] = xi;
+        m = fmax(m, fabs(xi));
+    });
+    put_max(m, out);
+}
+
+// A whole Jacobi::Solve (Iter.cxx:56-112) on at most 1,024 rows, thread per row, with the
+// matrix and x in shared memory: a sweep of a 27-row coarsest level waits for shared memory and
+// one or two block barriers instead of global loads (40 sweeps: 105 -> 12 us on B200). Rows are
+// summed left to right as row_apply sums them. zero: x is taken as 0 and not read.
+template <typename T>
+__global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
+                                                       const uint32_t* __restrict__ rowPtr,
+                                                       const uint32_t* __restrict__ colInd,
+                                                       const T* __restrict__ val,
+                                                       const T* __restrict__ b, T* __restrict__ x,
+                                                       const T* __restrict__ dinv,
+                                                       fasp_gpu_params prm, int zero, Bits* out)
+{
+    extern __shared__ __align__(16) unsigned char small[];
+    __shared__ double sh[32];
+    T* sv = reinterpret_cast<T*>(small);
+    T* sx = sv + nnz;
+    uint16_t* sc = reinterpret_cast<uint16_t*>(sx + n);
+    const uint32_t t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+    for (uint32_t k = t; k < nnz; k += blockDim.x) { // the matrix: no predecessor writes it
+        sv[k] = val[k];
+        sc[k] = (uint16_t)colInd[k];
+    }
+    const bool row = t < n;
+    const uint32_t r0 = row ? rowPtr[t] : 0u, r1 = row ? rowPtr[t + 1] : 0u;
+    const T di = row ? dinv[t] : T(0);
+    pdl_wait();
+    pdl_release();
+    const T bi = row ? b[t] : T(0);
+    T xi = row && !zero ? x[t] : T(0);
+    if (row) sx[t] = xi;
+    // the block's sum or maximum of v, the same on every thread; its barriers order sx
+    auto all = [&](double v, int op) {
+        v = warp_reduce(v, op);
+        __syncthreads();
+        if (lane == 0) sh[wid] = v;
+        __syncthreads();
+        return __shfl_sync(0xffffffffu, warp_reduce(lane < nw ? sh[lane] : 0.0, op), 0);
+    };
+    double xinf = all((double)fabs(xi), kMax), denAbs = 1.0;
+    for (uint32_t it = 0; it < prm.maxIter; ++it) {
+        T s = T(0);
+        if (!(xinf < kCloseZero))
+            for (uint32_t k = r0; k < r1; ++k) s = fma(sv[k], sx[sc[k]], s);
+        const T r = bi - s;
+        if (it >= prm.minIter) {
+            const double resAbs = sqrt(all((double)(row ? r * r : T(0)), kSum));
+            if (it == prm.minIter) denAbs = (kCloseZero > resAbs) ? kCloseZero : resAbs;
+            if (resAbs / denAbs < prm.relTol || resAbs < prm.absTol) break;
+        }
+        __syncthreads(); // every row's sum has read the old x
+        if (row) {
+            xi = xi + r * di;
+            sx[t] = xi;
+        }
+        xinf = all((double)fabs(xi), kMax);
+    }
+    if (row) x[t] = xi;
+    if (out && t == 0 && xinf > 0.0) atomicMax(out, (Bits)__double_as_longlong(xinf));
+}
+
+constexpr size_t kSmallBytes = 200 * 1024; // shared memory of k_jacobi_small at most
+
+size_t small_bytes(const Mat& A, size_t elem)
+{
+    return (size_t)A.nnz * (elem + 2) + (size_t)A.nrow * elem;
+}
+
+template <typename F>
+void by_lanes(int lanes, F&& go)
+{
+    switch (lanes) {
+        case 1: go(std::integral_constant<int, 1>()); break;
+        case 2: go(std::integral_constant<int, 2>()); break;
+        case 4: go(std::integral_constant<int, 4>()); break;
+        case 8: go(std::integral_constant<int, 8>()); break;
+        case 16: go(std::integral_constant<int, 16>()); break;
+        default: go(std::integral_constant<int, 32>()); break;
+    }
+}
+
+// kern(view of A, args...) on one resident wave, rows on `lanes` lanes, in block tiles where A
+// takes them.
+template <typename... P, typename... X>
+int launch_rows(Ctx& c, const Mat& A, int lanes, void (*kern)(CSRView<double>, P...), X... args)
+{
+    CSRView<double> V = A.v64();
+    size_t smem = lanes == 1 ? with_tiles(V, kBlock) : 0;
+    if (smem && !tiles_fit((const void*)kern, smem)) V.tiles = 0, smem = 0;
+    const int g = std::min(c.grid((long long)A.nrow * lanes, kBlock),
+                           resident_grid(c, (const void*)kern, kBlock, smem));
+    ++c.launches;
+    FB_CUDA(launch_pdl(kern, dim3((unsigned)g), dim3(kBlock), smem, c.stream, V, args...));
+    return kOk;
+}
+
+// Lanes for a transfer operator's rows: a matrix without stored values for it (a grid operator)
+// keeps one thread per row.
+int transfer_lanes(const Mat& A) { return A.grid ? 1 : lanes_for(A.meanRowLen); }
+
+} // namespace
+
+bool jacobi_small_fits(const Mat& A, size_t elem)
+{
+    return !A.grid && A.val && A.nrow == A.mcol && A.nrow <= 1024 && small_bytes(A, elem) <= kSmallBytes;
+}
+
+template <typename T>
+int jacobi_small(Ctx& c, const Mat& A, const T* val, const T* b, T* x, const T* dinv,
+                 const fasp_gpu_params& prm, bool zero, unsigned long long* xinf)
+{
+    const size_t smem = small_bytes(A, sizeof(T));
+    const auto kern = k_jacobi_small<T>;
+    FB_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kSmallBytes));
+    ++c.launches;
+    FB_CUDA(launch_pdl(kern, dim3(1), dim3((A.nrow + 31u) & ~31u), smem, c.stream, A.nrow, A.nnz,
+                       (const uint32_t*)A.rowPtr, (const uint32_t*)A.colInd, val, b, x, dinv, prm,
+                       zero ? 1 : 0, xinf));
+    return kOk;
+}
+template int jacobi_small<double>(Ctx&, const Mat&, const double*, const double*, double*,
+                                  const double*, const fasp_gpu_params&, bool, unsigned long long*);
+template int jacobi_small<float>(Ctx&, const Mat&, const float*, const float*, float*, const float*,
+                                 const fasp_gpu_params&, bool, unsigned long long*);
+
+// NormInf slots that one cycle writes: one per kernel that writes x, and one per restriction.
+static double cycle_slots(const SolverImpl& S)
+{
+    double total = 0.0, visits = 1.0;
+    for (size_t l = 0; l < S.mgP.size(); ++l) {
+        total += visits * (2.0 * S.mgSmooth[l].prm.maxIter + 4.0);
+        if (l + 1 < S.mgP.size()) visits *= std::max(1u, S.cfg.mgCycles);
+        else total += visits * (S.mgCoarse[l].prm.maxIter + 2.0);
+    }
+    return total;
+}
+
+bool SolverImpl::mg_fixed_cycle() const
+{
+    if (mgP.empty() || cfg.mgCycles == 0) return false;
+    auto fixed = [](const Pcd& p) {
+        return p.type == 1 && p.prm.minIter == p.prm.maxIter && p.prm.maxIter >= 1 &&
+               (p.A->val || p.A->grid);
+    };
+    for (size_t l = 0; l < mgP.size(); ++l)
+        if (!fixed(mgSmooth[l]) || (l + 1 == mgP.size() && !fixed(mgCoarse[l])) ||
+            !(mgP[l]->val || mgP[l]->grid) || !(mgR[l]->val || mgR[l]->grid))
+            return false;
+    return cycle_slots(*this) <= kMgSlots;
+}
+
+// prm.maxIter sweeps of p on b and x. in: NormInf(x), or with zero (x is taken as 0 and not
+// read) NormInf(dinv .* b) where it is known, else null. *end: NormInf of the new x.
+static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, const Bits* in,
+                  Bits** end)
+{
+    Ctx& c = S.c;
+    const Mat& A = *p.A;
+    const int lanes = A.grid ? 1 : A.lanes;
+    int e;
+    if (jacobi_small_fits(A, 8)) {
+        *end = S.mgInf + S.mgInfUsed++;
+        return jacobi_small<double>(c, A, A.val, b, x, p.dinv, p.prm, zero, *end);
+    }
+    uint32_t left = p.prm.maxIter;
+    double *cur = x, *nxt = p.work;
+    auto next_slot = [&]() { return *end = S.mgInf + S.mgInfUsed++; };
+    if (zero) {
+        const bool two = in && left >= 2;
+        left -= two ? 2 : 1;
+        if (left % 2) std::swap(cur, nxt); // so that the last sweep writes x
+        if (two) {
+            Bits* out = next_slot();
+            by_lanes(lanes, [&](auto L) {
+                e = launch_rows(c, A, lanes, k_mg_sweep<decltype(L)::value, true>, b,
+                                (const double*)nullptr, (const double*)p.dinv, cur, in, out);
+            });
+            if (e) return e;
+        } else {
+            Bits* out = next_slot();
+            ++c.launches;
+            const int g = std::min(c.grid(A.nrow, kBlock),
+                                   resident_grid(c, (const void*)k_mg_first, kBlock));
+            FB_CUDA(launch_pdl(k_mg_first, dim3((unsigned)g), dim3(kBlock), 0, c.stream, A.nrow, b,
+                               (const double*)p.dinv, cur, out));
+        }
+        in = *end;
+    }
+    for (; left > 0; --left) {
+        Bits* out = next_slot();
+        by_lanes(lanes, [&](auto L) {
+            e = launch_rows(c, A, lanes, k_mg_sweep<decltype(L)::value, false>, b, (const double*)cur,
+                            (const double*)p.dinv, nxt, in, out);
+        });
+        if (e) return e;
+        in = out;
+        std::swap(cur, nxt);
+    }
+    return cur == x ? (int)kOk : v_copy(c, A.nrow, (const double*)cur, x);
+}
+
+// One cycle from level l (MG.cxx:105-152 with this level's operators): pre-smoothing,
+// residual, restriction, the coarse solver or the next level's cycles, correction,
+// post-smoothing. zero, in, end as in smooth().
+static int cycle(SolverImpl& S, uint32_t l, const double* b, double* x, bool zero, const Bits* in,
+                 Bits** end)
+{
+    Ctx& c = S.c;
+    const uint32_t NL = (uint32_t)S.mgP.size();
+    const Mat &A = *S.mgA[l], &R = *S.mgR[l], &P = *S.mgP[l];
+    double* r = l == 0 ? S.w[0] : S.mgRes[l];
+    int e;
+    Bits* s = nullptr;
+    if ((e = smooth(S, S.mgSmooth[l], b, x, zero, in, &s)) ||
+        (e = m_residual(c, A, b, (const double*)x, r, reinterpret_cast<const double*>(s))))
+        return e;
+    Pcd& next = l + 1 == NL ? S.mgCoarse[l] : S.mgSmooth[l + 1];
+    Bits* first = S.mgInf + S.mgInfUsed++;
+    const int rl = transfer_lanes(R), pl = transfer_lanes(P);
+    by_lanes(rl, [&](auto L) {
+        e = launch_rows(c, R, rl, k_mg_restrict<decltype(L)::value>, (const double*)r, S.mgB[l],
+                        (const double*)next.dinv, first);
+    });
+    if (e) return e;
+    Bits* coarse = nullptr;
+    if (l + 1 == NL) {
+        if ((e = smooth(S, next, S.mgB[l], S.mgX[l], true, first, &coarse))) return e;
+    } else {
+        for (uint32_t i = 0; i < S.cfg.mgCycles; ++i)
+            if ((e = cycle(S, l + 1, S.mgB[l], S.mgX[l], i == 0, i == 0 ? first : coarse, &coarse)))
+                return e;
+    }
+    s = S.mgInf + S.mgInfUsed++;
+    by_lanes(pl, [&](auto L) {
+        e = launch_rows(c, P, pl, k_mg_correct<decltype(L)::value>, (const double*)S.mgX[l], x, s);
+    });
+    if (e) return e;
+    return smooth(S, S.mgSmooth[l], b, x, false, s, end);
+}
+
+int SolverImpl::mg_cycle_fixed(const double* b, double* x, bool zero)
+{
+    int e;
+    if (!mgInf && (e = dev_alloc(&mgInf, sizeof(Bits) * kMgSlots, c.stream))) return e;
+    FB_CUDA(cudaMemsetAsync(mgInf, 0, sizeof(Bits) * kMgSlots, c.stream));
+    mgInfUsed = 0;
+    const Bits* in = nullptr;
+    if (!zero) {
+        double* xinf = reinterpret_cast<double*>(mgInf + mgInfUsed++);
+        if ((e = v_norminf(c, n, (const double*)x, xinf))) return e;
+        in = reinterpret_cast<const Bits*>(xinf);
+    }
+    Bits* end = nullptr;
+    return cycle(*this, 0, b, x, zero, in, &end);
+}
+
+} // namespace fb

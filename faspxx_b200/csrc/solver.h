@@ -52,6 +52,8 @@ struct Pcd {
     template <typename T>
     int  solve(Ctx& c, const T* b, T* x, std::vector<double>* hist = nullptr,
                double* norm2 = nullptr, double* normInf = nullptr);
+    // solve with x = 0 as the initial guess, whatever x holds
+    int  solve_from_zero(Ctx& c, const double* b, double* x);
 };
 
 // The vectors one precision of a host-orchestrated solver works on.
@@ -103,12 +105,20 @@ struct SolverImpl {
     std::vector<double*>     mgRes;
     int  mg_setup_transfers();
     void mg_cycle_transfer(const double* b, double* x);
+    // the same cycle when every smoother and the coarse solver run a fixed number of sweeps
+    // (mg.cu); zero: x is taken as 0 and not read. mgInf: the cycle's NormInf slots
+    static constexpr uint32_t kMgSlots = 1024;
+    unsigned long long* mgInf = nullptr;
+    uint32_t            mgInfUsed = 0;
+    bool mg_fixed_cycle() const;
+    int  mg_cycle_fixed(const double* b, double* x, bool zero);
     // MG as a preconditioner: when no step of its solve reads a norm on the host (minIter =
     // maxIter for the MG object, its smoothers and its coarse solver), the whole solve is a
-    // fixed kernel sequence; it is captured once per (b, x) pair and replayed as a graph
+    // fixed kernel sequence; it is captured once per (b, x) pair and start and replayed as a graph
     struct MgGraph {
         const double*   b;
         double*         x;
+        bool            zero;
         cudaGraphExec_t exec;
     };
     std::vector<MgGraph> mgGraphs;
@@ -157,7 +167,7 @@ struct SolverImpl {
     Space<double> sp64() { return Space<double>{&w, V, Z}; }
     Space<float>  sp32() { return Space<float>{&w32, V32, Z32}; }
     int jacobi(const double* b, double* x, fasp_gpu_info* info);
-    int mg(const double* b, double* x, fasp_gpu_info* info);
+    int mg(const double* b, double* x, fasp_gpu_info* info, bool zero = false);
     void mg_cycle(const double* b, double* x);
 
     // helpers
@@ -169,6 +179,14 @@ struct SolverImpl {
         hist[k] = v * histScale;
     }
 };
+
+// Jacobi::Solve on a matrix of at most 1,024 rows in one launch (mg.cu): whether it fits, and
+// the solve (val: the values in T; zero: x is taken as 0; xinf, optional, a zeroed slot that gets
+// NormInf(x)).
+bool jacobi_small_fits(const Mat& A, size_t elem);
+template <typename T>
+int jacobi_small(Ctx& c, const Mat& A, const T* val, const T* b, T* x, const T* dinv,
+                 const fasp_gpu_params& prm, bool zero, unsigned long long* xinf);
 
 } // namespace fb
 

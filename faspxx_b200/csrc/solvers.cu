@@ -204,7 +204,7 @@ int Pcd::setup(Ctx& c, const Mat* M, int t, double w, const fasp_gpu_params& p)
 }
 
 // type 2 (MG preconditioner): one MG::Solve on the preconditioner's own solver object
-static int pcd_mg_apply(SolverImpl* s, const double* b, double* x);
+static int pcd_mg_apply(SolverImpl* s, const double* b, double* x, bool zero = false);
 static void pcd_mg_free(SolverImpl* s);
 
 void Pcd::destroy()
@@ -262,6 +262,16 @@ int Pcd::solve(Ctx& c, const T* b, T* x, std::vector<double>* hist, double* norm
     double resAbs = 1.0, resRel = 1.0, denAbs = 1.0;
     const CSRView<T> V = pcd_view<T>(*A);
     const bool fusable = A->lanes == 1 && (V.val || V.gnz) && (const void*)b != (const void*)x;
+    if (!hist && !norm2 && !normInf && (const void*)b != (const void*)x &&
+        (A->lanes == 1 || sizeof(T) == 8) && jacobi_small_fits(*A, sizeof(T))) {
+        numIter = prm.maxIter; // the convergence test runs on the device
+        const T* val;
+        if constexpr (std::is_same<T, float>::value)
+            val = A->val32;
+        else
+            val = A->val;
+        return jacobi_small<T>(c, *A, val, b, x, dinv, prm, false, nullptr);
+    }
     if (fusable && !hist && !norm2 && !normInf && n <= kJacobiBlockRows) {
         // nothing reads the norms back: the whole solve in one single-block launch
         ++c.launches;
@@ -354,6 +364,13 @@ template int Pcd::solve<double>(Ctx&, const double*, double*, std::vector<double
                                 double*);
 template int Pcd::solve<float>(Ctx&, const float*, float*, std::vector<double>*, double*,
                                double*);
+
+int Pcd::solve_from_zero(Ctx& c, const double* b, double* x)
+{
+    if (type == 2 && mg->mg_fixed_cycle()) return pcd_mg_apply(mg, b, x, true);
+    v_set(c, A->nrow, 0.0, x);
+    return solve(c, b, x);
+}
 
 // ---- setup -------------------------------------------------------------------------------
 
@@ -600,6 +617,8 @@ void SolverImpl::destroy()
     for (double* p : mgB) dev_free(p);
     for (double* p : mgX) dev_free(p);
     for (double* p : mgRes) dev_free(p);
+    dev_free(mgInf);
+    mgInf = nullptr;
     mgRes.clear();
     for (Mat* m : mgOwn) {
         m_free(*m);
@@ -657,8 +676,7 @@ int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
     uint32_t numIter = 0;
 
     if ((e = apply_residual(c, *A, b, x, rk))) return e;
-    v_set(c, n, 0.0, zk);
-    if ((e = pcd.solve(c, rk, zk))) return e;
+    if ((e = pcd.solve_from_zero(c, rk, zk))) return e;
     v_copy(c, n, zk, pk);
     v_dot(c, n, zk, rk, d + SL_T0);
     tmpa = fetch(d + SL_T0);
@@ -746,8 +764,7 @@ int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
         }
         if (numIter < P.maxIter) {
             resAbsOld = resAbs;
-            v_set(c, n, 0.0, zk);
-            if ((e = pcd.solve(c, rk, zk))) return e;
+            if ((e = pcd.solve_from_zero(c, rk, zk))) return e;
             v_dot(c, n, zk, rk, d + SL_T0);
             tmpb = fetch(d + SL_T0);
             beta = tmpb / tmpa;
@@ -2270,22 +2287,26 @@ void SolverImpl::mg_cycle(const double* b, double* x)
     }
 }
 
-static int pcd_mg_apply(SolverImpl* s, const double* b, double* x)
+static int pcd_mg_apply(SolverImpl* s, const double* b, double* x, bool zero)
 {
     fasp_gpu_info info{};
     const fasp_gpu_config& k = s->cfg;
     const bool fixed = k.prm.minIter == k.prm.maxIter && k.mgSmoothPrm.minIter == k.mgSmoothPrm.maxIter &&
                        k.mgCoarsePrm.minIter == k.mgCoarsePrm.maxIter;
-    if (!fixed) return s->mg(b, x, &info);
+    if (!fixed) return s->mg(b, x, &info, zero);
     for (const auto& g : s->mgGraphs)
-        if (g.b == b && g.x == x) {
+        if (g.b == b && g.x == x && g.zero == zero) {
             FB_CUDA(cudaGraphLaunch(g.exec, s->c.stream));
             return kOk;
         }
     cudaStream_t st = s->c.stream;
+    if (!s->mgInf && s->mg_fixed_cycle()) { // before the capture, which takes no allocation
+        const int ea = dev_alloc(&s->mgInf, sizeof(*s->mgInf) * SolverImpl::kMgSlots, st);
+        if (ea) return ea;
+    }
     FB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     s->capturing = true;
-    const int e = s->mg(b, x, &info);
+    const int e = s->mg(b, x, &info, zero);
     s->capturing = false;
     cudaGraph_t graph = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(st, &graph);
@@ -2293,7 +2314,7 @@ static int pcd_mg_apply(SolverImpl* s, const double* b, double* x)
     if (!e && ce == cudaSuccess && graph &&
         cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
         cudaGraphDestroy(graph);
-        s->mgGraphs.push_back({b, x, exec});
+        s->mgGraphs.push_back({b, x, zero, exec});
         FB_CUDA(cudaGraphLaunch(exec, st));
         return kOk;
     }
@@ -2407,17 +2428,23 @@ void SolverImpl::mg_cycle_transfer(const double* b, double* x)
     --mgLevel;
 }
 
-int SolverImpl::mg(const double* b, double* x, fasp_gpu_info* info)
+int SolverImpl::mg(const double* b, double* x, fasp_gpu_info* info, bool zero)
 {
     const fasp_gpu_params& P = cfg.prm;
     double* r = w[0];
     double* d = c.dslot;
     double resAbs = 1.0, resRel = 1.0, denAbs = 1.0;
     uint32_t numIter = 0;
+    int e;
     mgLevel = -1;
+    const bool fixed = mg_fixed_cycle() && b != x;
+    if (zero && (!fixed || P.maxIter == 0 || P.minIter == 0)) { // x is read: make it the zero it stands for
+        v_set(c, n, 0.0, x);
+        zero = false;
+    }
     while (numIter < P.maxIter) {
-        m_residual(c, *A, b, x, r, nullptr);
-        if (numIter >= P.minIter) {
+        if (numIter >= P.minIter) { // the residual is read by this test alone
+            m_residual(c, *A, b, x, r, nullptr);
             v_norm2(c, n, r, d + SL_T1);
             resAbs = fetch(d + SL_T1);
             if (numIter == P.minIter) denAbs = (kCloseZero > resAbs) ? kCloseZero : resAbs;
@@ -2425,10 +2452,14 @@ int SolverImpl::mg(const double* b, double* x, fasp_gpu_info* info)
             rec(numIter, resAbs);
             if (resRel < P.relTol || resAbs < P.absTol) break;
         }
-        if (mgP.empty())
+        if (fixed) {
+            if ((e = mg_cycle_fixed(b, x, zero))) return e;
+        } else if (mgP.empty()) {
             mg_cycle(b, x);
-        else
+        } else {
             mg_cycle_transfer(b, x);
+        }
+        zero = false;
         ++numIter;
     }
     info->numIter = numIter;

@@ -300,3 +300,34 @@ def test_two_grid_cycle_against_textbook_numpy(gpu):
             assert np.allclose(h, res, rtol=1e-9, atol=0.0), (h, res)
             rates = np.array(res[1:]) / np.array(res[:-1])
             assert np.max(rates) < 0.2, rates
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-24])
+@pytest.mark.parametrize("sweeps,coarse,cycles", [(1, 1, 1), (2, 3, 1), (3, 40, 2), (2, 2, 3)])
+@pytest.mark.parametrize("dim,nf,L", [(3, 31, 3), (3, 23, 1), (2, 63, 2)])
+def test_fixed_cycles_match_tested_ones(gpu, O, dim, nf, L, sweeps, coarse, cycles, scale):
+    """A fixed number of sweeps (minIter = maxIter) runs the short launch sequence; the same
+    sweeps with a convergence test that never stops run kernel by kernel. Both are the same
+    cycle: solutions after two cycles agree to 1e-12 (each is a few hundred rounded sums away
+    from the other), MG alone and under CG, also where every x is below NormInf's 1e-20."""
+    A = P.poisson3d(nf) if dim == 3 else P.poisson2d(nf)
+    b = scale * np.random.default_rng(5).uniform(-1, 1, A.nrow)
+    M, f, Ps = gpu.MAT(A), nf, []
+    for _ in range(L):
+        Ps.append(gpu.MAT(_interp(f, dim)))
+        f = (f - 1) // 2
+    out = []
+    for tested in (False, True):
+        def prm(k):
+            return dict(maxIter=k, minIter=0 if tested else k, weight=2.0 / 3.0, relTol=0.0, absTol=0.0)
+        kw = dict(mgLevels=L, mgCycles=cycles, mgSmooth=prm(sweeps), mgCoarse=prm(coarse))
+        for alg, extra in (("mg", dict(maxIter=2, minIter=2)),
+                           ("cg", dict(maxIter=3, minIter=3, pcd="mg", pcdIter=1, pcdMinIter=1))):
+            s = gpu.configure(alg, relTol=0.0, absTol=0.0, **kw, **extra)
+            s.transfers = {l: (Pm, None, None) for l, Pm in enumerate(Ps)}
+            s.Setup(M)
+            x = np.zeros(A.nrow)
+            s.Solve(b, x)
+            out.append(x)
+    for k in (0, 1):
+        assert np.max(np.abs(out[k] - out[k + 2])) <= 1e-12 * np.max(np.abs(out[k + 2]))
