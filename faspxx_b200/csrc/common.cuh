@@ -575,6 +575,30 @@ __device__ __forceinline__ T row_apply(const CSRView<T>& A, size_t row, XV xv)
     return row_dot<T, PAT>(A, row, b, e, xv);
 }
 
+// Two rows of a stencil-mask view (or grid operator) of at most 8 offsets on one thread, each
+// row's sum as row_apply forms it: both masks, then both rows' gathers, then the FMAs, so a
+// thread has twice the loads in flight.
+template <typename T, typename XV>
+__device__ __forceinline__ void mask_rows2(const CSRView<T>& A, size_t r0, size_t r1, XV xv, T& s0,
+                                           T& s1)
+{
+    const uint32_t m0 = A.gnz ? grid_mask(A, (uint32_t)r0) : (uint32_t)__ldcs(A.mask + r0);
+    const uint32_t m1 = A.gnz ? grid_mask(A, (uint32_t)r1) : (uint32_t)__ldcs(A.mask + r1);
+    T a[8], b[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) { // the masks have no bits at or above ulen
+        a[u] = (m0 >> u) & 1u ? xv((uint32_t)((long long)r0 + A.udelta[u])) : T(0);
+        b[u] = (m1 >> u) & 1u ? xv((uint32_t)((long long)r1 + A.udelta[u])) : T(0);
+    }
+    s0 = T(0);
+    s1 = T(0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        if ((m0 >> u) & 1u) s0 = fma(A.uval[u], a[u], s0);
+        if ((m1 >> u) & 1u) s1 = fma(A.uval[u], b[u], s1);
+    }
+}
+
 // Every row of A once, own(row, sum) on the thread that owns it: thread t of the grid owns
 // rows t, t + S, t + 2S, ... (S = the grid's threads) in that order. Views launched with
 // block tiles (A.tiles, see with_tiles) stream them; call it with every thread of the block.
@@ -586,9 +610,16 @@ __device__ __forceinline__ void for_rows(const CSRView<T>& A, XV xv, OWN own)
         return;
     }
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t row = (size_t)blockIdx.x * blockDim.x + threadIdx.x; row < A.nrow;
-         row += stride)
-        own(row, row_apply<T, PAT>(A, row, xv));
+    size_t row = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (!PAT && (A.mask || A.gnz) && A.ulen <= 8) {
+        for (; row + stride < A.nrow; row += 2 * stride) {
+            T s0, s1;
+            mask_rows2<T>(A, row, row + stride, xv, s0, s1);
+            own(row, s0);
+            own(row + stride, s1);
+        }
+    }
+    for (; row < A.nrow; row += stride) own(row, row_apply<T, PAT>(A, row, xv));
 }
 
 // Block tiles for a plain CSR view (no row classes, stencil masks, grid form or 16-bit

@@ -67,7 +67,7 @@ __device__ __forceinline__ void rows_of(const CSRView<double>& A, XV xv, OWN own
 // is below CLOSE_ZERO (MAT.cxx:455-476, Iter.cxx:83-92). TWO: the first two sweeps from
 // x = 0, whose first is dinv .* b, formed where it is gathered; *in is its NormInf.
 template <int L, bool TWO>
-__global__ void __launch_bounds__(kBlock) k_mg_sweep(CSRView<double> A, const double* __restrict__ b,
+__global__ void __launch_bounds__(kBlock, 5) k_mg_sweep(CSRView<double> A, const double* __restrict__ b,
                                                      const double* __restrict__ xin,
                                                      const double* __restrict__ dinv,
                                                      double* __restrict__ xout,
@@ -160,9 +160,10 @@ __global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
     T* sx = sv + nnz;
     uint16_t* sc = reinterpret_cast<uint16_t*>(sx + n);
     const uint32_t t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = blockDim.x >> 5;
+#pragma unroll 8
     for (uint32_t k = t; k < nnz; k += blockDim.x) { // the matrix: no predecessor writes it
-        sv[k] = val[k];
-        sc[k] = (uint16_t)colInd[k];
+        sv[k] = __ldg(val + k);
+        sc[k] = (uint16_t)__ldg(colInd + k);
     }
     const bool row = t < n;
     const uint32_t r0 = row ? rowPtr[t] : 0u, r1 = row ? rowPtr[t + 1] : 0u;
@@ -184,7 +185,21 @@ __global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
     for (uint32_t it = 0; it < prm.maxIter; ++it) {
         T s = T(0);
         if (!(xinf < kCloseZero))
-            for (uint32_t k = r0; k < r1; ++k) s = fma(sv[k], sx[sc[k]], s);
+            for (uint32_t k = r0; k < r1; k += 8) { // eight entries' loads, then their FMAs
+                uint32_t c[8];
+                T v[8], g[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const bool in = k + u < r1;
+                    c[u] = in ? sc[k + u] : 0u;
+                    v[u] = in ? sv[k + u] : T(0);
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) g[u] = sx[c[u]];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (k + u < r1) s = fma(v[u], g[u], s);
+            }
         const T r = bi - s;
         if (it >= prm.minIter) {
             const double resAbs = sqrt(all((double)(row ? r * r : T(0)), kSum));
