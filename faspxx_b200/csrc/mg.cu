@@ -9,34 +9,22 @@
 // V(2,2) cycle took 330 us at 31^3 and 800 us at 127^3. Here a level takes one launch for
 // its first two sweeps (from x = 0), one a sweep after that, one residual, one restriction and
 // one prolongation that also corrects x; levels of up to 1,024 rows take one launch for all their
-// sweeps. NormInf(x), which a residual's shortcut test needs, is an atomic maximum of the bits
-// of |x| in the kernel that writes x: a maximum does not depend on order, so the test is exact
-// and reruns are the same.
+// sweeps. Whether NormInf(x) is below CLOSE_ZERO, which a residual's shortcut tests, is a mark that
+// the kernel writing x leaves when any |x| is not: the same decision without a reduction.
 #include "solver.h"
 
 namespace fb {
 namespace {
 
-using Bits = unsigned long long;
-
-__device__ __forceinline__ double from_bits(const Bits* p)
+// Marks *out (0.0 before the cycle) when any thread of the block saw an |x| that is not below
+// CLOSE_ZERO: all that a residual's shortcut asks of NormInf(x) (a NaN counts as below, as in
+// VEC::NormInf). Every thread calls it.
+__device__ __forceinline__ void mark_above(bool above, double* out)
 {
-    return __longlong_as_double((long long)*(const volatile Bits*)p);
+    if (__syncthreads_or(above) && threadIdx.x == 0) *out = 1.0;
 }
 
-// *out = max(*out, max over the block of m >= 0); every thread calls it.
-__device__ __forceinline__ void put_max(double m, Bits* out)
-{
-    __shared__ double sh[32];
-    m = warp_reduce(m, kMax);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        m = threadIdx.x < ((blockDim.x + 31) >> 5) ? sh[threadIdx.x] : 0.0;
-        m = warp_reduce(m, kMax);
-        if (threadIdx.x == 0 && m > 0.0) atomicMax(out, (Bits)__double_as_longlong(m));
-    }
-}
+__device__ __forceinline__ bool above_zero(double x) { return fabs(x) >= kCloseZero; }
 
 // Rows of A on L lanes each (L = 1: one thread, block tiles where the view has them):
 // own(row, sum) on the row's first lane.
@@ -65,23 +53,23 @@ __device__ __forceinline__ void rows_of(const CSRView<double>& A, XV xv, OWN own
 
 // One Jacobi sweep, xout = xin + dinv .* r with r = b - A xin, or r = b when NormInf(xin) (*in)
 // is below CLOSE_ZERO (MAT.cxx:455-476, Iter.cxx:83-92). TWO: the first two sweeps from
-// x = 0, whose first is dinv .* b, formed where it is gathered; *in is its NormInf.
+// x = 0, whose first is dinv .* b, formed where it is gathered; *in is its mark.
 template <int L, bool TWO>
 __global__ void __launch_bounds__(kBlock, 5) k_mg_sweep(CSRView<double> A, const double* __restrict__ b,
                                                      const double* __restrict__ xin,
                                                      const double* __restrict__ dinv,
                                                      double* __restrict__ xout,
-                                                     const Bits* __restrict__ in, Bits* out)
+                                                     const double* __restrict__ in, double* out)
 {
     pdl_wait();
     pdl_release();
-    const bool shortcut = from_bits(in) < kCloseZero;
-    double m = 0.0;
+    const bool shortcut = *in < kCloseZero;
+    bool above = false;
     auto x0 = [&](size_t j) { return TWO ? b[j] * dinv[j] : xin[j]; };
     auto own = [&](size_t i, double sum) {
         const double xi = x0(i) + (b[i] - sum) * dinv[i];
         xout[i] = xi;
-        m = fmax(m, fabs(xi));
+        above = above || above_zero(xi);
     };
     if (shortcut)
         for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.nrow;
@@ -89,56 +77,56 @@ __global__ void __launch_bounds__(kBlock, 5) k_mg_sweep(CSRView<double> A, const
             own(i, 0.0);
     else
         rows_of<L>(A, [&](uint32_t j) { return x0(j); }, own);
-    put_max(m, out);
+    mark_above(above, out);
 }
 
 // The first sweep from x = 0: x = dinv .* b.
 __global__ void __launch_bounds__(kBlock) k_mg_first(uint32_t n, const double* __restrict__ b,
                                                      const double* __restrict__ dinv,
-                                                     double* __restrict__ x, Bits* out)
+                                                     double* __restrict__ x, double* out)
 {
     pdl_wait();
     pdl_release();
-    double m = 0.0;
+    bool above = false;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x) {
         const double xi = b[i] * dinv[i];
         x[i] = xi;
-        m = fmax(m, fabs(xi));
+        above = above || above_zero(xi);
     }
-    put_max(m, out);
+    mark_above(above, out);
 }
 
-// bc = R r, and NormInf(dinv .* bc), the coarse level's first sweep.
+// bc = R r, and the mark of dinv .* bc, the coarse level's first sweep.
 template <int L>
 __global__ void __launch_bounds__(kBlock) k_mg_restrict(CSRView<double> R, const double* __restrict__ r,
                                                         double* __restrict__ bc,
-                                                        const double* __restrict__ dinv, Bits* out)
+                                                        const double* __restrict__ dinv, double* out)
 {
     pdl_wait();
     pdl_release();
-    double m = 0.0;
+    bool above = false;
     rows_of<L>(R, [&](uint32_t j) { return r[j]; }, [&](size_t i, double s) {
         bc[i] = s;
-        m = fmax(m, fabs(s * dinv[i]));
+        above = above || above_zero(s * dinv[i]);
     });
-    put_max(m, out);
+    mark_above(above, out);
 }
 
 // x += P e.
 template <int L>
 __global__ void __launch_bounds__(kBlock) k_mg_correct(CSRView<double> P, const double* __restrict__ e,
-                                                       double* __restrict__ x, Bits* out)
+                                                       double* __restrict__ x, double* out)
 {
     pdl_wait();
     pdl_release();
-    double m = 0.0;
+    bool above = false;
     rows_of<L>(P, [&](uint32_t j) { return e[j]; }, [&](size_t i, double s) {
         const double xi = x[i] + s;
         x[i] = xi;
-        m = fmax(m, fabs(xi));
+        above = above || above_zero(xi);
     });
-    put_max(m, out);
+    mark_above(above, out);
 }
 
 // A whole Jacobi::Solve (Iter.cxx:56-112) on at most 1,024 rows, thread per row, with the
@@ -152,7 +140,7 @@ __global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
                                                        const T* __restrict__ val,
                                                        const T* __restrict__ b, T* __restrict__ x,
                                                        const T* __restrict__ dinv,
-                                                       fasp_gpu_params prm, int zero, Bits* out)
+                                                       fasp_gpu_params prm, int zero, double* out)
 {
     extern __shared__ __align__(16) unsigned char small[];
     __shared__ double sh[32];
@@ -173,18 +161,19 @@ __global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
     const T bi = row ? b[t] : T(0);
     T xi = row && !zero ? x[t] : T(0);
     if (row) sx[t] = xi;
-    // the block's sum or maximum of v, the same on every thread; its barriers order sx
-    auto all = [&](double v, int op) {
-        v = warp_reduce(v, op);
+    // the block's sum of v, the same on every thread
+    auto all = [&](double v) {
+        v = warp_reduce(v, kSum);
         __syncthreads();
         if (lane == 0) sh[wid] = v;
         __syncthreads();
-        return __shfl_sync(0xffffffffu, warp_reduce(lane < nw ? sh[lane] : 0.0, op), 0);
+        return __shfl_sync(0xffffffffu, warp_reduce(lane < nw ? sh[lane] : 0.0, kSum), 0);
     };
-    double xinf = all((double)fabs(xi), kMax), denAbs = 1.0;
+    double denAbs = 1.0;
+    bool above = __syncthreads_or(above_zero((double)xi)); // orders the writes of sx too
     for (uint32_t it = 0; it < prm.maxIter; ++it) {
         T s = T(0);
-        if (!(xinf < kCloseZero))
+        if (above)
             for (uint32_t k = r0; k < r1; k += 8) { // eight entries' loads, then their FMAs
                 uint32_t c[8];
                 T v[8], g[8];
@@ -202,7 +191,7 @@ __global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
             }
         const T r = bi - s;
         if (it >= prm.minIter) {
-            const double resAbs = sqrt(all((double)(row ? r * r : T(0)), kSum));
+            const double resAbs = sqrt(all((double)(row ? r * r : T(0))));
             if (it == prm.minIter) denAbs = (kCloseZero > resAbs) ? kCloseZero : resAbs;
             if (resAbs / denAbs < prm.relTol || resAbs < prm.absTol) break;
         }
@@ -211,10 +200,10 @@ __global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
             xi = xi + r * di;
             sx[t] = xi;
         }
-        xinf = all((double)fabs(xi), kMax);
+        above = __syncthreads_or(above_zero((double)xi));
     }
     if (row) x[t] = xi;
-    if (out && t == 0 && xinf > 0.0) atomicMax(out, (Bits)__double_as_longlong(xinf));
+    if (out && t == 0 && above) *out = 1.0;
 }
 
 constexpr size_t kSmallBytes = 200 * 1024; // shared memory of k_jacobi_small at most
@@ -265,7 +254,7 @@ bool jacobi_small_fits(const Mat& A, size_t elem)
 
 template <typename T>
 int jacobi_small(Ctx& c, const Mat& A, const T* val, const T* b, T* x, const T* dinv,
-                 const fasp_gpu_params& prm, bool zero, unsigned long long* xinf)
+                 const fasp_gpu_params& prm, bool zero, double* mark)
 {
     const size_t smem = small_bytes(A, sizeof(T));
     const auto kern = k_jacobi_small<T>;
@@ -274,15 +263,15 @@ int jacobi_small(Ctx& c, const Mat& A, const T* val, const T* b, T* x, const T* 
     ++c.launches;
     FB_CUDA(launch_pdl(kern, dim3(1), dim3((A.nrow + 31u) & ~31u), smem, c.stream, A.nrow, A.nnz,
                        (const uint32_t*)A.rowPtr, (const uint32_t*)A.colInd, val, b, x, dinv, prm,
-                       zero ? 1 : 0, xinf));
+                       zero ? 1 : 0, mark));
     return kOk;
 }
 template int jacobi_small<double>(Ctx&, const Mat&, const double*, const double*, double*,
-                                  const double*, const fasp_gpu_params&, bool, unsigned long long*);
+                                  const double*, const fasp_gpu_params&, bool, double*);
 template int jacobi_small<float>(Ctx&, const Mat&, const float*, const float*, float*, const float*,
-                                 const fasp_gpu_params&, bool, unsigned long long*);
+                                 const fasp_gpu_params&, bool, double*);
 
-// NormInf slots that one cycle writes: one per kernel that writes x, and one per restriction.
+// Marks that one cycle writes: one per kernel that writes x, and one per restriction.
 static double cycle_slots(const SolverImpl& S)
 {
     double total = 0.0, visits = 1.0;
@@ -308,10 +297,10 @@ bool SolverImpl::mg_fixed_cycle() const
     return cycle_slots(*this) <= kMgSlots;
 }
 
-// prm.maxIter sweeps of p on b and x. in: NormInf(x), or with zero (x is taken as 0 and not
-// read) NormInf(dinv .* b) where it is known, else null. *end: NormInf of the new x.
-static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, const Bits* in,
-                  Bits** end)
+// prm.maxIter sweeps of p on b and x. in: the mark of x, or with zero (x is taken as 0 and not
+// read) that of dinv .* b where it is known, else null. *end: the mark of the new x.
+static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, const double* in,
+                  double** end)
 {
     Ctx& c = S.c;
     const Mat& A = *p.A;
@@ -329,14 +318,14 @@ static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, 
         left -= two ? 2 : 1;
         if (left % 2) std::swap(cur, nxt); // so that the last sweep writes x
         if (two) {
-            Bits* out = next_slot();
+            double* out = next_slot();
             by_lanes(lanes, [&](auto L) {
                 e = launch_rows(c, A, lanes, k_mg_sweep<decltype(L)::value, true>, b,
                                 (const double*)nullptr, (const double*)p.dinv, cur, in, out);
             });
             if (e) return e;
         } else {
-            Bits* out = next_slot();
+            double* out = next_slot();
             ++c.launches;
             const int g = std::min(c.grid(A.nrow, kBlock),
                                    resident_grid(c, (const void*)k_mg_first, kBlock));
@@ -346,7 +335,7 @@ static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, 
         in = *end;
     }
     for (; left > 0; --left) {
-        Bits* out = next_slot();
+        double* out = next_slot();
         by_lanes(lanes, [&](auto L) {
             e = launch_rows(c, A, lanes, k_mg_sweep<decltype(L)::value, false>, b, (const double*)cur,
                             (const double*)p.dinv, nxt, in, out);
@@ -361,27 +350,27 @@ static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, 
 // One cycle from level l (MG.cxx:105-152 with this level's operators): pre-smoothing,
 // residual, restriction, the coarse solver or the next level's cycles, correction,
 // post-smoothing. zero, in, end as in smooth().
-static int cycle(SolverImpl& S, uint32_t l, const double* b, double* x, bool zero, const Bits* in,
-                 Bits** end)
+static int cycle(SolverImpl& S, uint32_t l, const double* b, double* x, bool zero, const double* in,
+                 double** end)
 {
     Ctx& c = S.c;
     const uint32_t NL = (uint32_t)S.mgP.size();
     const Mat &A = *S.mgA[l], &R = *S.mgR[l], &P = *S.mgP[l];
     double* r = l == 0 ? S.w[0] : S.mgRes[l];
     int e;
-    Bits* s = nullptr;
+    double* s = nullptr;
     if ((e = smooth(S, S.mgSmooth[l], b, x, zero, in, &s)) ||
-        (e = m_residual(c, A, b, (const double*)x, r, reinterpret_cast<const double*>(s))))
+        (e = m_residual(c, A, b, (const double*)x, r, (const double*)s)))
         return e;
     Pcd& next = l + 1 == NL ? S.mgCoarse[l] : S.mgSmooth[l + 1];
-    Bits* first = S.mgInf + S.mgInfUsed++;
+    double* first = S.mgInf + S.mgInfUsed++;
     const int rl = transfer_lanes(R), pl = transfer_lanes(P);
     by_lanes(rl, [&](auto L) {
         e = launch_rows(c, R, rl, k_mg_restrict<decltype(L)::value>, (const double*)r, S.mgB[l],
                         (const double*)next.dinv, first);
     });
     if (e) return e;
-    Bits* coarse = nullptr;
+    double* coarse = nullptr;
     if (l + 1 == NL) {
         if ((e = smooth(S, next, S.mgB[l], S.mgX[l], true, first, &coarse))) return e;
     } else {
@@ -400,16 +389,16 @@ static int cycle(SolverImpl& S, uint32_t l, const double* b, double* x, bool zer
 int SolverImpl::mg_cycle_fixed(const double* b, double* x, bool zero)
 {
     int e;
-    if (!mgInf && (e = dev_alloc(&mgInf, sizeof(Bits) * kMgSlots, c.stream))) return e;
-    FB_CUDA(cudaMemsetAsync(mgInf, 0, sizeof(Bits) * kMgSlots, c.stream));
+    if (!mgInf && (e = dev_alloc(&mgInf, sizeof(double) * kMgSlots, c.stream))) return e;
+    FB_CUDA(cudaMemsetAsync(mgInf, 0, sizeof(double) * kMgSlots, c.stream));
     mgInfUsed = 0;
-    const Bits* in = nullptr;
+    const double* in = nullptr;
     if (!zero) {
-        double* xinf = reinterpret_cast<double*>(mgInf + mgInfUsed++);
+        double* xinf = mgInf + mgInfUsed++; // NormInf itself
         if ((e = v_norminf(c, n, (const double*)x, xinf))) return e;
-        in = reinterpret_cast<const Bits*>(xinf);
+        in = xinf;
     }
-    Bits* end = nullptr;
+    double* end = nullptr;
     return cycle(*this, 0, b, x, zero, in, &end);
 }
 

@@ -106,10 +106,11 @@ struct SolverImpl {
     int  mg_setup_transfers();
     void mg_cycle_transfer(const double* b, double* x);
     // the same cycle when every smoother and the coarse solver run a fixed number of sweeps
-    // (mg.cu); zero: x is taken as 0 and not read. mgInf: the cycle's NormInf slots
+    // (mg.cu); zero: x is taken as 0 and not read. mgInf: the cycle's marks, one per kernel that
+    // writes an x: 0.0 when NormInf(x) is below CLOSE_ZERO
     static constexpr uint32_t kMgSlots = 1024;
-    unsigned long long* mgInf = nullptr;
-    uint32_t            mgInfUsed = 0;
+    double*  mgInf = nullptr;
+    uint32_t mgInfUsed = 0;
     bool mg_fixed_cycle() const;
     int  mg_cycle_fixed(const double* b, double* x, bool zero);
     // MG as a preconditioner: when no step of its solve reads a norm on the host (minIter =
@@ -181,12 +182,12 @@ struct SolverImpl {
 };
 
 // Jacobi::Solve on a matrix of at most 1,024 rows in one launch (mg.cu): whether it fits, and
-// the solve (val: the values in T; zero: x is taken as 0; xinf, optional, a zeroed slot that gets
-// NormInf(x)).
+// the solve (val: the values in T; zero: x is taken as 0; mark, optional, 0.0 before, becomes 1.0
+// unless NormInf(x) is below CLOSE_ZERO).
 bool jacobi_small_fits(const Mat& A, size_t elem);
 template <typename T>
 int jacobi_small(Ctx& c, const Mat& A, const T* val, const T* b, T* x, const T* dinv,
-                 const fasp_gpu_params& prm, bool zero, unsigned long long* xinf);
+                 const fasp_gpu_params& prm, bool zero, double* mark);
 
 } // namespace fb
 
