@@ -72,8 +72,8 @@ constexpr double kSmallDbl = -1e+60;
 constexpr double kKsmChkRatio = 0.95;
 constexpr unsigned kMaxStagNum = 20;
 
-// A scalar operand: a host value, or (m * *p) / (m / *p when inv) read on the device, so
-// that one kernel can consume another's reduction without a host round trip.
+// A scalar operand: a host value, or m * *p (m / *p when inv is 1, *p / m when it is 2) read
+// on the device, so that one kernel can consume another's reduction without a host round trip.
 struct Scal {
     double        v;
     const double* p;
@@ -82,12 +82,13 @@ struct Scal {
     static Scal h(double x) { return Scal{x, nullptr, 1.0, 0}; }
     static Scal d(const double* q, double mul = 1.0) { return Scal{0.0, q, mul, 0}; }
     static Scal dinv(const double* q, double mul = 1.0) { return Scal{0.0, q, mul, 1}; }
+    static Scal over(const double* q, double den) { return Scal{0.0, q, den, 2}; }
 };
 
 __device__ __forceinline__ double eval(const Scal& s)
 {
     if (!s.p) return s.v;
-    return s.inv ? s.m / *s.p : s.m * *s.p;
+    return s.inv == 2 ? *s.p / s.m : (s.inv ? s.m / *s.p : s.m * *s.p);
 }
 
 constexpr int kSlots = 256;

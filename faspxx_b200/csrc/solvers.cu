@@ -22,6 +22,7 @@ static const double kNaN = std::numeric_limits<double>::quiet_NaN();
 // scalar slots of the solver context
 enum {
     SL_T0 = 0, SL_T1, SL_T2, SL_T3, SL_T4, SL_T5, SL_T6, SL_T7,
+    SL_TA0 = 8, SL_TA1, SL_TB, SL_TR, // cg_generic: (z, r) by turns, (ax, p), ||r||
     SL_XINF = 16,  // NormInf of a residual's x (MAT::Residual shortcut)
     SL_ONE = 17,   // constant 1: disables the shortcut (MAT::Apply + XPAY paths)
     SL_XINF2 = 18, // the fused Jacobi sweeps' second NormInf slot (ping-pong with SL_XINF)
@@ -662,6 +663,33 @@ void SolverImpl::destroy()
 
 // ---- CG (src/CG.cxx:53-249) ---------------------------------------------------------------
 
+// alpha = *tmpa / *tmpb, x += alpha p, r -= alpha ax and ||r|| (CG.cxx:104-133) in one pass,
+// with the operations of v_axpy and v_norm2 one after another; nothing but the norm's slot
+// changes when |*tmpb| <= 1e-40 (the host finishes that branch).
+__global__ void __launch_bounds__(kBlock) k_cg_step(uint32_t n, const double* __restrict__ tmpa,
+                                                    const double* __restrict__ tmpb,
+                                                    const double* __restrict__ p,
+                                                    const double* __restrict__ ax,
+                                                    double* __restrict__ x, double* __restrict__ r,
+                                                    Scratch s, double* dnorm)
+{
+    pdl_wait();
+    pdl_release();
+    const double tb = *tmpb, alpha = *tmpa / tb;
+    const bool go = fabs(tb) > kCloseZero * kCloseZero;
+    double t = 0.0;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; go && i < n;
+         i += (size_t)gridDim.x * blockDim.x) {
+        x[i] = fma(alpha, p[i], x[i]);
+        const double ri = fma(-alpha, ax[i], r[i]);
+        r[i] = ri;
+        t = fma(ri, ri, t);
+    }
+    double acc[1] = {t};
+    const int ops[1] = {kSum};
+    grid_reduce<1>(acc, ops, s, [=] __device__(const double* v) { *dnorm = sqrt(v[0]); });
+}
+
 int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
 {
     const fasp_gpu_params& P = cfg.prm;
@@ -672,14 +700,16 @@ int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
     const double solStagTol = 1e-4 * P.relTol, solZeroTol = kCloseZero;
     unsigned stagStep = 0, moreStep = 0;
     double resAbs = 1.0, resRel = 1.0, denAbs = 1.0, ratio = 0.0, resAbsOld = 1.0;
-    double alpha = 0.0, beta, tmpa, tmpb;
+    double alpha = 0.0, tmpa, tmpb;
     uint32_t numIter = 0;
 
     if ((e = apply_residual(c, *A, b, x, rk))) return e;
     if ((e = pcd.solve_from_zero(c, rk, zk))) return e;
     v_copy(c, n, zk, pk);
-    v_dot(c, n, zk, rk, d + SL_T0);
-    tmpa = fetch(d + SL_T0);
+    // (z, r) stays on the device, in SL_TA0 and SL_TA1 by turns; one wait an iteration reads it
+    // with (ax, p) and ||r||
+    int turn = 0;
+    v_dot(c, n, zk, rk, d + SL_TA0);
 
     while (numIter < P.maxIter) {
         if (numIter == P.minIter) {
@@ -693,8 +723,17 @@ int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
         }
         ++numIter;
         m_spmv(c, *A, pk, ax);
-        v_dot(c, n, ax, pk, d + SL_T0);
-        tmpb = fetch(d + SL_T0);
+        v_dot(c, n, ax, pk, d + SL_TB);
+        ++c.launches;
+        FB_CUDA(launch_pdl(k_cg_step, dim3((unsigned)c.grid(n, kBlock)), dim3(kBlock), 0, c.stream, n,
+                           (const double*)(d + SL_TA0 + turn), (const double*)(d + SL_TB),
+                           (const double*)pk, (const double*)ax, x, rk, c.red, d + SL_TR));
+        FB_CUDA(cudaMemcpyAsync(c.hslot, d + SL_TA0, 4 * sizeof(double), cudaMemcpyDeviceToHost,
+                                c.stream));
+        FB_CUDA(cudaStreamSynchronize(c.stream));
+        tmpa = c.hslot[turn];
+        tmpb = c.hslot[2];
+        const double rnorm = c.hslot[3];
         if (std::fabs(tmpb) > kCloseZero * kCloseZero)
             alpha = tmpa / tmpb;
         else {
@@ -707,12 +746,9 @@ int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
             rec(numIter, resAbs);
             break;
         }
-        v_axpy(c, n, Scal::h(alpha), pk, x);
-        v_axpy(c, n, Scal::h(-alpha), ax, rk);
         if (numIter >= P.minIter) {
             bool stop = false;
-            v_norm2(c, n, rk, d + SL_T1);
-            resAbs = fetch(d + SL_T1);
+            resAbs = rnorm;
             resRel = resAbs / denAbs;
             ratio = resAbs / resAbsOld;
             if (numIter >= P.savIter && resAbs < resAbsOld) v_copy(c, n, x, sv);
@@ -765,11 +801,9 @@ int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
         if (numIter < P.maxIter) {
             resAbsOld = resAbs;
             if ((e = pcd.solve_from_zero(c, rk, zk))) return e;
-            v_dot(c, n, zk, rk, d + SL_T0);
-            tmpb = fetch(d + SL_T0);
-            beta = tmpb / tmpa;
-            tmpa = tmpb;
-            v_xpay(c, n, Scal::h(beta), zk, pk);
+            turn ^= 1;
+            v_dot(c, n, zk, rk, d + SL_TA0 + turn);
+            v_xpay(c, n, Scal::over(d + SL_TA0 + turn, tmpa), zk, pk); // beta = (z, r) / tmpa
         }
     }
     info->numIter = numIter;
