@@ -190,10 +190,19 @@ int fasp_gpu_free(void* p)
     return kOk;
 }
 
+// cudaMemcpy of pageable memory returns once the last piece is staged, and cudaMemset at once: the
+// legacy stream may still be writing, and the library's streams do not wait for it. A product
+// started right after a 3.2 MB copy read the old last entries.
+static int landed()
+{
+    FB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    return kOk;
+}
+
 int fasp_gpu_memcpy_h2d(void* dst, const void* src, size_t bytes)
 {
     FB_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
-    return kOk;
+    return landed();
 }
 
 int fasp_gpu_memcpy_d2h(void* dst, const void* src, size_t bytes)
@@ -205,7 +214,7 @@ int fasp_gpu_memcpy_d2h(void* dst, const void* src, size_t bytes)
 int fasp_gpu_memset(void* dst, int value, size_t bytes)
 {
     FB_CUDA(cudaMemset(dst, value, bytes));
-    return kOk;
+    return landed();
 }
 
 int fasp_gpu_synchronize(void)
@@ -434,7 +443,7 @@ int fasp_gpu_mat_diag(fasp_gpu_mat A, double* diag)
 {
     if (!A || !diag) return kErrInputPar;
     FB_CUDA(cudaMemcpy(diag, A->M.diag, (size_t)A->M.nrow * 8, cudaMemcpyDeviceToDevice));
-    return kOk;
+    return landed();
 }
 
 int fasp_gpu_mat_autotune(fasp_gpu_mat A, int* lanes)
