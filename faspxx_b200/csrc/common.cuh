@@ -423,27 +423,51 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, uint3
     return false;
 }
 
-// Rows of a plain CSR view in block tiles; own(row, sum) on the row's thread. Block b takes
-// tiles b, b + G, b + 2G, ... (G = gridDim.x), so thread t of the grid owns rows t, t + S,
-// t + 2S, ... (S = the grid's threads) in that order, as the row-at-a-time loops do. Every
+__device__ __forceinline__ double rounded_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double rounded_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float rounded_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float rounded_add(float a, float b) { return __fadd_rn(a, b); }
+
+// How a row's sum takes its entries: one FMA each from 0 (products), or from the row's own
+// start with every product rounded before it is added (MAT::MultTransposeAdd).
+struct RowFma {
+    static constexpr bool kSep = false;
+    template <typename T>
+    __device__ __forceinline__ T start(size_t) const { return T(0); }
+};
+template <typename F>
+struct RowSep {
+    static constexpr bool kSep = true;
+    F from;
+    template <typename T>
+    __device__ __forceinline__ T start(size_t row) const { return from(row); }
+};
+
+// Rows of a plain CSR view in block tiles; own(row, sum) on the row's first thread. L threads own
+// a row (L = 1: one), so a tile has 256 / L rows. Block b takes tiles b, b + G, b + 2G, ...
+// (G = gridDim.x); for L = 1, thread t of the grid owns rows t, t + S, t + 2S, ... (S = the
+// grid's threads) in that order, as the row-at-a-time loops do. Sums with FMAs are those of
+// row_dot (L = 1) and of the lane kernels (L > 1: lane l takes entries l, l + L, ..., then
+// a shuffle tree); separately rounded sums go left to right whatever L. Every
 // thread of the block calls it (it synchronises the block). A tile whose entries do not fit
 // a stage (only possible when the caller ignored the span check of with_tiles) is summed
 // from global memory.
-template <typename T, bool PAT, typename XV, typename OWN>
+template <typename T, bool PAT, int L = 1, typename XV, typename OWN, typename ACC = RowFma>
 __device__ __forceinline__ void csr_tile_rows(const CSRView<T>& A, TileSmem<T>& sm, XV xv,
-                                              OWN own)
+                                              OWN own, ACC acc = ACC())
 {
+    constexpr uint32_t R = kTileRows / L; // rows of a tile
     constexpr uint32_t CAP = TileShape<T>::cap;
     const size_t n = A.nrow;
-    const size_t ntiles = (n + kTileRows - 1) / kTileRows;
+    const size_t ntiles = (n + R - 1) / R;
     const uint32_t tid = threadIdx.x;
     const size_t mine =
         blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const unsigned long long pol = tid == 0 ? l2_evict_first() : 0ull;
     auto issue = [&](size_t k) { // thread 0: tile k of this block into stage k % stages
         const int s = (int)(k % kTileStages);
-        const size_t r0 = (blockIdx.x + k * gridDim.x) * kTileRows;
-        const size_t rows = n - r0 < kTileRows ? n - r0 : kTileRows;
+        const size_t r0 = (blockIdx.x + k * gridDim.x) * R;
+        const size_t rows = n - r0 < R ? n - r0 : R;
         const uint32_t beg = A.rowPtr[r0], end = A.rowPtr[r0 + rows];
         const uint32_t a = beg & ~3u, ar = (uint32_t)(((size_t)end + 3) & ~size_t(3));
         const bool ok = ar - a <= CAP;
@@ -480,33 +504,100 @@ __device__ __forceinline__ void csr_tile_rows(const CSRView<T>& A, TileSmem<T>& 
             atomicAdd(&fb_tile_timeouts, 1u);
             sm.bad = 1;
         }
-        const size_t row = (blockIdx.x + k * gridDim.x) * kTileRows + tid;
-        if (landed && row < n) {
-            const TileStage<T>& st = sm.st[s];
-            const uint32_t b = st.rp[tid], e = st.rp[tid + 1];
-            T sum = T(0);
-            if (sm.ok[s]) {
-                const uint32_t a = sm.a[s];
+        const uint32_t lr = tid / L;
+        const size_t row = (blockIdx.x + k * gridDim.x) * R + lr;
+        if constexpr (L == 1) {
+            if (landed && row < n) {
+                const TileStage<T>& st = sm.st[s];
+                const uint32_t b = st.rp[tid], e = st.rp[tid + 1];
+                T sum = acc.template start<T>(row);
+                if (sm.ok[s]) {
+                    const uint32_t a = sm.a[s];
 #pragma unroll 2
-                for (uint32_t k4 = b; k4 < e; k4 += 4) {
-                    uint32_t cc[4];
+                    for (uint32_t k4 = b; k4 < e; k4 += 4) {
+                        uint32_t cc[4];
+                        T v[4], xs[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const bool in = k4 + u < e;
+                            cc[u] = in ? st.c[k4 + u - a] : 0u;
+                            v[u] = PAT ? T(in ? 1 : 0) : (in ? st.v[k4 + u - a] : T(0));
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) xs[u] = k4 + u < e ? xv(cc[u]) : T(0);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (k4 + u < e)
+                                sum = !ACC::kSep ? fma(v[u], xs[u], sum)
+                                                 : rounded_add(sum, PAT ? xs[u]
+                                                                        : rounded_mul(xs[u], v[u]));
+                    }
+                } else if (!ACC::kSep) {
+                    sum = row_dot<T, PAT>(A, row, b, e, xv);
+                } else {
+                    for (uint32_t q = b; q < e; ++q)
+                        sum = rounded_add(sum, PAT ? xv(A.colInd[q])
+                                                   : rounded_mul(xv(A.colInd[q]), A.val[q]));
+                }
+                own(row, sum);
+            }
+        } else {
+            // every lane takes part in the shuffles, rows past the end as empty ones
+            const TileStage<T>& st = sm.st[s];
+            const bool have = __all_sync(0xffffffffu, landed) && row < n;
+            const bool staged = sm.ok[s] != 0;
+            const uint32_t a = sm.a[s];
+            if constexpr (!ACC::kSep) {
+                const uint32_t b = have ? st.rp[lr] : 0u, e = have ? st.rp[lr + 1] : 0u;
+                const uint32_t lane = tid & (L - 1);
+                auto col = [&](uint32_t q) { return staged ? st.c[q - a] : A.colInd[q]; };
+                auto val = [&](uint32_t q) {
+                    return PAT ? T(1) : (staged ? st.v[q - a] : A.val[q]);
+                };
+                T sum = T(0);
+                for (uint32_t q = b + lane; q < e; q += 4 * L) {
                     T v[4], xs[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        const bool in = k4 + u < e;
-                        cc[u] = in ? st.c[k4 + u - a] : 0u;
-                        v[u] = PAT ? T(in ? 1 : 0) : (in ? st.v[k4 + u - a] : T(0));
+                        const bool in = q + u * L < e;
+                        v[u] = in ? val(q + u * L) : T(0);
+                        xs[u] = in ? xv(col(q + u * L)) : T(0);
                     }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) xs[u] = k4 + u < e ? xv(cc[u]) : T(0);
-#pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        if (k4 + u < e) sum = fma(v[u], xs[u], sum);
+                        if (q + u * L < e) sum = PAT ? sum + xs[u] : fma(v[u], xs[u], sum);
                 }
+                sum = group_sum<L>(sum);
+                if (have && lane == 0) own(row, sum);
             } else {
-                sum = row_dot<T, PAT>(A, row, b, e, xv);
+                // the tile's products in place, entry by entry over all threads (every gather
+                // of the tile in flight at once), then one thread a row adds its own in order
+                TileStage<T>& sw = sm.st[s];
+                const size_t r0 = row - lr;
+                const uint32_t rows = (uint32_t)(n - r0 < R ? n - r0 : R);
+                if (staged && __all_sync(0xffffffffu, landed)) {
+                    const uint32_t end = st.rp[rows] - a;
+#pragma unroll 4
+                    for (uint32_t q = st.rp[0] - a + tid; q < end; q += kTileRows) {
+                        const T x = xv(sw.c[q]);
+                        sw.v[q] = PAT ? x : rounded_mul(x, sw.v[q]);
+                    }
+                }
+                __syncthreads();
+                if (tid < rows && landed) {
+                    const uint32_t b1 = st.rp[tid], e1 = st.rp[tid + 1];
+                    T sum = acc.template start<T>(r0 + tid);
+                    if (staged) {
+#pragma unroll 4
+                        for (uint32_t q = b1 - a; q < e1 - a; ++q) sum = rounded_add(sum, sw.v[q]);
+                    } else {
+                        for (uint32_t q = b1; q < e1; ++q)
+                            sum = rounded_add(sum, PAT ? xv(A.colInd[q])
+                                                       : rounded_mul(xv(A.colInd[q]), A.val[q]));
+                    }
+                    own(r0 + tid, sum);
+                }
             }
-            own(row, sum);
         }
         __syncthreads(); // stage s is free again
         if (sm.bad) { // every thread sees it after the barrier: leave together
@@ -628,16 +719,22 @@ __device__ __forceinline__ void for_rows(const CSRView<T>& A, XV xv, OWN own)
 // dynamic shared memory its kernel must be launched with (0, view unmarked, otherwise).
 // Launchers then call tiles_fit with the kernel, which unmarks the view again when the
 // kernel's static shared memory and the stages together exceed 48 KB.
+// span: the most entries of a tile of the kernel's rows (Mat::span for lanes > 1).
 template <typename T>
-inline size_t with_tiles(CSRView<T>& V, int block)
+inline size_t with_tiles(CSRView<T>& V, int block, uint32_t span)
 {
     auto al = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
     const bool ok = V.nrow > 0 && !V.cls && !V.mask && !V.gnz && !V.cd16 &&
-                    V.tileSpan > 0 && V.tileSpan <= TileShape<T>::cap &&
+                    span > 0 && span <= TileShape<T>::cap &&
                     block == (int)kTileRows && al(V.rowPtr) && al(V.colInd) &&
                     (!V.val || al(V.val));
     V.tiles = ok ? 1u : 0u;
     return ok ? sizeof(TileSmem<T>) : 0;
+}
+template <typename T>
+inline size_t with_tiles(CSRView<T>& V, int block)
+{
+    return with_tiles(V, block, V.tileSpan);
 }
 
 // This translation unit's count of tile waits that ran out.

@@ -233,6 +233,13 @@ struct Mat {
     bool      cd16On = false;    // the thread-per-row kernels use cd16 (opt-in: measured
                                  // slower than the 32-bit colInd on B200)
     uint32_t  tileSpan = 0;      // most entries of a 256-row tile (m_inspect), 0 unknown
+    uint32_t  laneSpan[6] = {};  // the same of a tile of 256 >> k rows (2^k lanes a row)
+    uint32_t  span(int L) const
+    {
+        int k = 0;
+        while (k < 5 && (1 << k) < L) ++k;
+        return laneSpan[k];
+    }
     double    diagValue = 0.0;
     uint32_t  maxRowLen = 0;
     double    meanRowLen = 0;

@@ -8,6 +8,7 @@
 // L = 32 the warp-per-row vector kernel; L is chosen from the mean row length or timed.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 #include "internal.h"
@@ -63,6 +64,11 @@ __global__ void __launch_bounds__(kBlock) k_spmv(CSRView<T> A, const T* __restri
         for_rows<T, PAT>(A, [&](uint32_t j) { return x[j]; }, [&](size_t r, T s) { y[r] = s; });
         return;
     }
+    if (A.tiles) { // L threads a row, the entries through shared memory: the same sums
+        csr_tile_rows<T, PAT, L>(A, *reinterpret_cast<TileSmem<T>*>(fb_tile_smem),
+                                 [&](uint32_t j) { return x[j]; }, [&](size_t r, T s) { y[r] = s; });
+        return;
+    }
     const int lane = threadIdx.x & (L - 1);
     const size_t warpRows = 32 / L;
     const size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -102,6 +108,12 @@ __global__ void __launch_bounds__(kBlock) k_residual(CSRView<T> A, const T* __re
         }
         return;
     }
+    if (A.tiles && !shortcut) {
+        csr_tile_rows<T, false, L>(A, *reinterpret_cast<TileSmem<T>*>(fb_tile_smem),
+                                   [&](uint32_t j) { return x[j]; },
+                                   [&](size_t row, T s) { r[row] = b[row] - s; });
+        return;
+    }
     const int lane = threadIdx.x & (L - 1);
     const size_t warpRows = 32 / L;
     const size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -138,7 +150,7 @@ int lanes_for(double mean)
 }
 
 template <typename T>
-static int launch_spmv(Ctx& c, CSRView<T> A, int L, const T* x, T* y)
+static int launch_spmv(Ctx& c, CSRView<T> A, int L, uint32_t span, const T* x, T* y)
 {
     if (A.nrow == 0) return kOk;
     const int need = spmv_grid(c, A.nrow, L);
@@ -159,7 +171,7 @@ static int launch_spmv(Ctx& c, CSRView<T> A, int L, const T* x, T* y)
             return kOk;
         }
     }
-    const size_t tiles = L == 1 ? with_tiles(A, kBlock) : 0;
+    const size_t tiles = with_tiles(A, kBlock, span);
     auto go = [&](auto kern) {
         CSRView<T> V = A;
         size_t smem = tiles;
@@ -191,12 +203,39 @@ static int launch_spmv(Ctx& c, CSRView<T> A, int L, const T* x, T* y)
 
 int m_spmv(Ctx& c, const Mat& A, const double* x, double* y)
 {
-    return launch_spmv<double>(c, A.v64(), A.lanes, x, y);
+    return launch_spmv<double>(c, A.v64(), A.lanes, A.span(A.lanes), x, y);
 }
 
 int m_spmv32(Ctx& c, const Mat& A, const float* x, float* y)
 {
-    return launch_spmv<float>(c, A.v32(), A.lanes, x, y);
+    return launch_spmv<float>(c, A.v32(), A.lanes, A.span(A.lanes), x, y);
+}
+
+// *mark = 1.0 when some |x_i| is not below CLOSE_ZERO (NormInf(x) >= CLOSE_ZERO, a NaN counting
+// as below as in VEC::NormInf), else 0.0: all that MAT::Residual's shortcut asks. Every block
+// looks at the same kBlock entries spread over x; where one of them decides, the first block
+// writes the mark and nobody reads or reduces anything else. Only a (nearly) zero x is read on,
+// up to each block's first such entry. NormInf itself read all of it: 11 of the 100 us of a
+// residual at 160^3, now 5.
+template <typename T>
+__global__ void __launch_bounds__(kBlock) k_mark_above(uint32_t n, const T* __restrict__ x, Scratch s,
+                                                       double* mark)
+{
+    auto above = [&](size_t i) { return (double)fabs(x[i]) >= kCloseZero; };
+    if (__syncthreads_or(n && above((size_t)threadIdx.x * n / kBlock))) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *mark = 1.0;
+        return;
+    }
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    bool found = false;
+    // the bound is the same for the whole block, which votes together
+    for (size_t i0 = (size_t)blockIdx.x * blockDim.x; i0 < n && !found; i0 += stride) {
+        const size_t i = i0 + threadIdx.x;
+        found = __syncthreads_or(i < n && above(i));
+    }
+    double acc[1] = {found ? 1.0 : 0.0};
+    const int ops[1] = {kMax};
+    grid_reduce<1>(acc, ops, s, [=] __device__(const double* t) { *mark = t[0]; });
 }
 
 template <typename T>
@@ -206,10 +245,11 @@ static int residual_t(Ctx& c, const Mat& A, CSRView<T> V, const T* b, const T* x
     if (A.nrow == 0) return kOk;
     if (!V.val && !V.gnz) return kErrMatData; // MAT::Residual reads values (MAT.cxx:466)
     if (!xinf) {
-        double* slot = c.dslot + kSlotResidualXinf;
-        int e = v_norminf(c, A.mcol, x, slot);
-        if (e) return e;
-        xinf = slot;
+        double* mark = c.dslot + kSlotResidualXinf;
+        ++c.launches;
+        k_mark_above<T><<<c.grid(A.mcol, kBlock), kBlock, 0, c.stream>>>(A.mcol, x, c.red, mark);
+        FB_CUDA(cudaGetLastError());
+        xinf = mark;
     }
     const int need = spmv_grid(c, A.nrow, A.lanes);
     if (A.lanes == 1) {
@@ -228,7 +268,7 @@ static int residual_t(Ctx& c, const Mat& A, CSRView<T> V, const T* b, const T* x
             return kOk;
         }
     }
-    const size_t tiles = A.lanes == 1 ? with_tiles(V, kBlock) : 0;
+    const size_t tiles = with_tiles(V, kBlock, A.span(A.lanes));
     auto go = [&](auto kern) {
         CSRView<T> W = V;
         size_t smem = tiles;
@@ -362,10 +402,25 @@ int m_sampled_outer(Ctx& c, const Mat& A, const double* lam, const double* x, do
 // reference's bit for bit wherever its loop bounds are right (structurally symmetric A).
 // Pattern-only matrices count every stored entry as 1, as MAT::Apply does; a grid operator
 // walks its stencil points in ascending offset, which is its CSR order.
-template <bool GRID, bool PAT>
-__global__ void k_mult_transpose_add(CSRView<double> T, const double* __restrict__ v1,
-                                     const double* __restrict__ v2, double* __restrict__ v)
+// Rows of some 8 to 50 entries stream through block tiles of 256 / L rows (csr_tile_rows with
+// separately rounded sums): thread per row straight from global memory reads words 12 len
+// bytes apart. On B200 a 571,000-row matrix of 23 entries a row took 63 us that way and takes
+// 47 us; seven-entry rows took 73 us thread per row (160^3), 76 us through tiles and 105 us
+// with evict-first loads four entries at a time, and keep the plain loop.
+template <bool GRID, bool PAT, int L>
+__global__ void __launch_bounds__(kBlock) k_mult_transpose_add(CSRView<double> T,
+                                                               const double* __restrict__ v1,
+                                                               const double* __restrict__ v2,
+                                                               double* __restrict__ v)
 {
+    if (!GRID && T.tiles) {
+        auto from = [&](size_t i) { return v2[i]; };
+        csr_tile_rows<double, PAT, L>(T, *reinterpret_cast<TileSmem<double>*>(fb_tile_smem),
+                                      [&](uint32_t j) { return v1[j]; },
+                                      [&](size_t i, double s) { v[i] = s; },
+                                      RowSep<decltype(from)>{from});
+        return;
+    }
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < T.nrow;
          i += (size_t)gridDim.x * blockDim.x) {
         double acc = v2[i];
@@ -387,14 +442,37 @@ __global__ void k_mult_transpose_add(CSRView<double> T, const double* __restrict
 int m_mult_transpose_add(Ctx& c, const Mat& T, const double* v1, const double* v2, double* v)
 {
     if (T.nrow == 0) return kOk;
-    const int g = std::max(1, std::min(ceil_div(T.nrow, kBlock), c.nsm * 8));
     CSRView<double> V = T.view<double>(T.val, nullptr);
+    V.cd16 = nullptr;
+    // the fewest threads a row whose tiles fit a stage; rows short enough for one (a
+    // 7-point stencil) go straight from global memory
+    int L = 1;
+    while (L < 8 && T.span(L) > TileShape<double>::cap) L *= 2;
+    const size_t tiles = T.grid || L == 1 ? 0 : with_tiles(V, kBlock, T.span(L));
+    if (!tiles) L = 1;
+    auto go = [&](auto kern) {
+        CSRView<double> W = V;
+        size_t smem = tiles;
+        if (smem && !tiles_fit((const void*)kern, smem)) W.tiles = 0, smem = 0;
+        const int g = std::max(1, std::min(ceil_div((long long)T.nrow * L, kBlock),
+                                           resident_grid(c, (const void*)kern, kBlock, smem)));
+        kern<<<g, kBlock, smem, c.stream>>>(W, v1, v2, v);
+    };
+    auto by = [&](auto PAT) {
+        constexpr bool P = decltype(PAT)::value;
+        switch (L) {
+            case 1: go(k_mult_transpose_add<false, P, 1>); break;
+            case 2: go(k_mult_transpose_add<false, P, 2>); break;
+            case 4: go(k_mult_transpose_add<false, P, 4>); break;
+            default: go(k_mult_transpose_add<false, P, 8>); break;
+        }
+    };
     if (T.grid)
-        k_mult_transpose_add<true, false><<<g, kBlock, 0, c.stream>>>(V, v1, v2, v);
+        go(k_mult_transpose_add<true, false, 1>);
     else if (!T.val)
-        k_mult_transpose_add<false, true><<<g, kBlock, 0, c.stream>>>(V, v1, v2, v);
+        by(std::true_type{});
     else
-        k_mult_transpose_add<false, false><<<g, kBlock, 0, c.stream>>>(V, v1, v2, v);
+        by(std::false_type{});
     FB_CUDA(cudaGetLastError());
     return kOk;
 }

@@ -29,7 +29,7 @@ constexpr uint32_t kRcSample = 8192; // rows looked at first: twice the classes 
 struct Inspect {
     unsigned           bad;     // CheckCSR fails
     unsigned           maxLen;  // longest row
-    unsigned           span;    // most entries of a 256-row tile, widened to multiples of 4
+    unsigned           span[6]; // most entries of a tile of 256 >> k rows, widened to multiples of 4
     unsigned           far16;   // some entry is more than 32,767 columns from its row
     unsigned           noDiag;  // some row stores no diagonal entry
     unsigned           classes; // distinct rows met by the class pass
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(kBlock) k_inspect(uint32_t nrow, uint32_t mcol
 {
     __shared__ uint32_t cs[kInspectChunk];
     bool bad = false, far = false, noDiag = false;
-    unsigned maxLen = 0, span = 0;
+    unsigned maxLen = 0, span[6] = {};
     unsigned long long dmin = ~0ull, dmax = 0ull;
     const size_t ntiles = ((size_t)nrow + kTileRows - 1) / kTileRows;
     for (size_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -74,8 +74,15 @@ __global__ void __launch_bounds__(kBlock) k_inspect(uint32_t nrow, uint32_t mcol
             }
         }
         if (T0 > T1 || T1 > nnz) T1 = T0; // a row of the tile is flagged: nothing to scan
-        const unsigned long long w = (((unsigned long long)T1 + 3) & ~3ull) - (T0 & ~3u);
-        span = max(span, (unsigned)(w < 0xffffffffull ? w : 0xffffffffull));
+#pragma unroll
+        for (int k = 0; k < 6; ++k) // the tile's parts of 256 >> k rows that begin at this row
+            if (in && (threadIdx.x & ((kTileRows >> k) - 1)) == 0) {
+                const size_t r1 = row + (kTileRows >> k) < t1 ? row + (kTileRows >> k) : t1;
+                const uint32_t p0 = rowPtr[row], p1 = rowPtr[r1];
+                const unsigned long long w =
+                    p1 < p0 ? 0ull : (((unsigned long long)p1 + 3) & ~3ull) - (p0 & ~3u);
+                span[k] = max(span[k], (unsigned)(w < 0xffffffffull ? w : 0xffffffffull));
+            }
         maxLen = max(maxLen, e - b);
         bool found = false;
         uint32_t dp = 0;
@@ -116,7 +123,8 @@ __global__ void __launch_bounds__(kBlock) k_inspect(uint32_t nrow, uint32_t mcol
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         maxLen = max(maxLen, __shfl_down_sync(0xffffffffu, maxLen, o));
-        span = max(span, __shfl_down_sync(0xffffffffu, span, o));
+#pragma unroll
+        for (int k = 0; k < 6; ++k) span[k] = max(span[k], __shfl_down_sync(0xffffffffu, span[k], o));
         dmin = min(dmin, __shfl_down_sync(0xffffffffu, dmin, o));
         dmax = max(dmax, __shfl_down_sync(0xffffffffu, dmax, o));
     }
@@ -127,7 +135,8 @@ __global__ void __launch_bounds__(kBlock) k_inspect(uint32_t nrow, uint32_t mcol
     }
     if ((threadIdx.x & 31) == 0) {
         atomicMax(&out->maxLen, maxLen);
-        atomicMax(&out->span, span);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) atomicMax(&out->span[k], span[k]);
         atomicMin(&out->dmin, dmin);
         atomicMax(&out->dmax, dmax);
     }
@@ -516,7 +525,8 @@ int m_inspect(Mat& T, bool classes, cudaStream_t s)
     } while (what == kCollision && ++attempt < 3); // three shared hashes: the CSR form stays
     T.rcOn = what == kBuilt;
     T.maxRowLen = h.maxLen;
-    T.tileSpan = h.span;
+    T.tileSpan = h.span[0];
+    std::memcpy(T.laneSpan, h.span, sizeof(T.laneSpan));
     T.near16 = !h.far16;
     T.diagConst = false;
     if (T.val && nrow == T.mcol && !h.noDiag && h.dmin == h.dmax) {

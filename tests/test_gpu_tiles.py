@@ -133,3 +133,63 @@ def test_gmres_solve_bit_exact(gpu, alg, prec):
     assert np.array_equal(out[0][2], out[1][2])
     assert np.array_equal(out[0][3], out[1][3])
     assert gpu.tile_timeouts() == 0
+
+
+@pytest.mark.parametrize("mean,lanes", [(20, 4), (27, 4), (45, 8), (100, 16), (200, 32), (24, 2)])
+@pytest.mark.parametrize("n", [1, 7, 63, 64, 65, 5000])
+def test_lane_tiles(gpu, n, mean, lanes):
+    """Tiles of 256 / lanes rows, and matrices whose tiles do not fit a stage (24 entries on two
+    lanes): MAT::Apply and MAT::Residual within the rounding of a row's sum, MAT::MultTransposeAdd
+    equal to its sequential definition. The last tile is partial, rows may be empty, entries start
+    off 16-byte boundaries."""
+    rng = np.random.default_rng(100 * mean + n)
+    lens = rng.integers(0, 2 * mean, n)
+    lens[rng.random(n) < 0.1] = 0
+    lens[n // 2] = mean
+    rp = np.zeros(n + 1, np.uint32)
+    rp[1:] = np.cumsum(lens)
+    A = P.CSRMatrix(n, n, rp, rng.integers(0, n, rp[-1]).astype(np.uint32),
+                    rng.uniform(-1, 1, rp[-1]))
+    x, b = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    M = gpu.MAT(A)
+    M.SetLanes(lanes)
+    dx, db, y, r, v = (gpu.DVec.from_numpy(t) for t in (x, b, b, b, b))
+    M.Apply(dx, y)
+    M.Residual(db, dx, r)
+    rp, ci = A.rowPtr.astype(np.int64), A.colInd.astype(np.int64)
+    want = np.zeros(n)
+    for i in range(n):  # lane l takes entries l, l + L, ...; then the halving tree
+        s = np.zeros(lanes)
+        for k in range(rp[i], rp[i + 1]):
+            s[(k - rp[i]) % lanes] += A.values[k] * x[ci[k]]
+        want[i] = s.sum()
+    scale = np.array([np.abs(A.values[rp[i]:rp[i + 1]] * x[ci[rp[i]:rp[i + 1]]]).sum()
+                      for i in range(n)]) + 1e-300
+    # |error| <= (entries + 2) ulp of the absolute sum, on both sides
+    assert np.all(np.abs(y.numpy() - want) <= 2 * (2 * mean + 2) * 2.3e-16 * scale)
+    assert np.all(np.abs(r.numpy() - (b - want)) <= 2 * (2 * mean + 3) * 2.3e-16 * (scale + np.abs(b)))
+    M.MultTransposeAdd(dx, db, v)
+    acc = b.copy()  # entries in CSR order: each column's in ascending rows
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    for i, c, a in zip(rows, ci, A.values):
+        acc[c] += a * x[i]
+    assert np.array_equal(v.numpy(), acc)
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 400000])
+@pytest.mark.parametrize("where", ["none", "first", "last", "nan"])
+def test_residual_shortcut(gpu, n, where):
+    """r = b exactly when every |x| is below 1e-20, NaNs counting as below: decided wherever the
+    one larger entry is."""
+    A = P.CSRMatrix(n, n, np.arange(n + 1, dtype=np.uint32), np.arange(n, dtype=np.uint32),
+                    np.full(n, 3e20) * (1 + np.arange(n) / n))
+    x = np.full(n, 9.9e-21)
+    if where == "nan":
+        x[0] = np.nan
+    elif where != "none":
+        x[0 if where == "first" else -1] = 1e-20
+    b = np.linspace(1, 2, n)
+    M, r = gpu.MAT(A), gpu.DVec(n)
+    M.Residual(gpu.DVec.from_numpy(b), gpu.DVec.from_numpy(x), r)
+    want = b if where in ("none", "nan") else b - A.values * x
+    assert np.allclose(r.numpy(), want, rtol=1e-15, atol=0)
