@@ -12,6 +12,7 @@
 #include <utility>
 
 #include "bicgstab.cuh"
+#include "plane_walk.cuh"
 
 namespace fb {
 
@@ -132,13 +133,15 @@ __device__ void bi_checks(BiCtl* c, const double* red, int phase)
 // product is the same bits, the partial sums group the rows by W). JAC = 2 (reliable
 // updates on a matrix whose diagonal varies): ptmp = A (D pj), the right-preconditioned
 // product, so that the recursive residual stays b - A x (the reference's order keeps it so
-// only when D commutes with A).
-template <typename T, int L, int JAC, int SH = 0>
+// only when D commutes with A). JAC = 3: D is one value for all rows, read from the control
+// block instead of a vector in each of the three kernels (the same bits).
+template <typename T, int L, int JAC, int SH = 0, bool WALK = false>
 __global__ void __launch_bounds__(kBlock) bi_p(CSRView<T> A, T* __restrict__ p0,
                                                T* __restrict__ p1, T* __restrict__ t0,
                                                T* __restrict__ t1, const T* __restrict__ rj,
                                                const T* __restrict__ r0s,
-                                               const T* __restrict__ dinv, BiCtl* c, Scratch s)
+                                               const T* __restrict__ dinv, BiCtl* c, Scratch s,
+                                               PlaneWalk walk)
 {
     pdl_wait();
     pdl_release();
@@ -149,14 +152,14 @@ __global__ void __launch_bounds__(kBlock) bi_p(CSRView<T> A, T* __restrict__ p0,
     const T* __restrict__ tOld = par ? t1 : t0;
     T* __restrict__ pNew = par ? p0 : p1;
     T* __restrict__ tNew = par ? t0 : t1;
-    const T beta = (T)c->beta, nomega = (T)(-c->omega);
+    const T beta = (T)c->beta, nomega = (T)(-c->omega), zc = (T)c->zc;
     auto pat = [&](size_t j) { // the updated pj at j
         const T tmp = fma(T(1), pOld[j], nomega * tOld[j]);
         return fma(T(1), rj[j], beta * tmp);
     };
     T a0 = 0, a1 = 0, a2 = 0;
     auto own = [&](size_t row, T ap) {
-        const T pt = JAC == 1 ? ap * dinv[row] : ap;
+        const T pt = JAC == 1 ? ap * dinv[row] : JAC == 3 ? ap * zc : ap;
         tNew[row] = pt;
         const T r = rj[row], r0 = r0s[row];
         a0 = fma(pt, r0, a0);
@@ -164,7 +167,22 @@ __global__ void __launch_bounds__(kBlock) bi_p(CSRView<T> A, T* __restrict__ p0,
         a2 = fma(r, r, a2);
     };
     auto xv = [&](uint32_t j) { return JAC == 2 ? pat(j) * dinv[j] : pat(j); };
-    if constexpr (SH != 0) {
+    if constexpr (WALK) {
+        struct Raw {
+            T r, p, t;
+        };
+        plane_rows<Raw, T>(
+            A, walk, reinterpret_cast<T*>(fb_tile_smem),
+            [&](uint32_t j) { return Raw{rj[j], pOld[j], tOld[j]}; },
+            [&](const Raw& v) {
+                const T tmp = fma(T(1), v.p, nomega * v.t);
+                return fma(T(1), v.r, beta * tmp);
+            },
+            [&](size_t row, T p, T ap) {
+                pNew[row] = p;
+                own(row, ap);
+            });
+    } else if constexpr (SH != 0) {
         using VT = Vec16<T>;
         using V = typename VT::V;
         constexpr int W = VT::W;
@@ -233,31 +251,39 @@ __global__ void __launch_bounds__(kBlock) bi_p(CSRView<T> A, T* __restrict__ p0,
 // sj = rj - alpha ptmp (on the fly for the gathers, stored for the owned rows),
 // stmp = D (A sj), omega = (stmp, sj) / (stmp, stmp)  (BiCGStab.cxx:103-113). SH as bi_p,
 // with sj's groups formed from rj and ptmp by the same FMA.
-template <typename T, int L, int JAC, int SH = 0>
+template <typename T, int L, int JAC, int SH = 0, bool WALK = false>
 __global__ void __launch_bounds__(kBlock) bi_s(CSRView<T> A, const T* __restrict__ rj,
                                                const T* __restrict__ t0,
                                                const T* __restrict__ t1,
                                                const T* __restrict__ dinv, T* __restrict__ sj,
-                                               T* __restrict__ stmp, BiCtl* c, Scratch s)
+                                               T* __restrict__ stmp, BiCtl* c, Scratch s,
+                                               PlaneWalk walk)
 {
     pdl_wait();
     pdl_release();
     if (c->status != kRun) return;
     const T* __restrict__ ptmp = c->par ? t1 : t0;
     static_assert(SH == 0 || JAC != 2, "right preconditioning runs the row kernels");
-    const T nalpha = (T)(-c->alpha);
+    const T nalpha = (T)(-c->alpha), zc = (T)c->zc;
     auto sv = [&](uint32_t j) { return fma(T(1), rj[j], nalpha * ptmp[j]); };
     auto gv = [&](uint32_t j) { return JAC == 2 ? sv(j) * dinv[j] : sv(j); };
     T a0 = 0, a1 = 0;
-    auto own = [&](size_t row, T as) {
-        const T sjv = sv((uint32_t)row);
+    auto own = [&](size_t row, T sjv, T as) {
         sj[row] = sjv;
-        const T st = JAC == 1 ? as * dinv[row] : as;
+        const T st = JAC == 1 ? as * dinv[row] : JAC == 3 ? as * zc : as;
         stmp[row] = st;
         a0 = fma(st, sjv, a0);
         a1 = fma(st, st, a1);
     };
-    if constexpr (SH != 0) {
+    if constexpr (WALK) {
+        struct Raw {
+            T r, t;
+        };
+        plane_rows<Raw, T>(
+            A, walk, reinterpret_cast<T*>(fb_tile_smem),
+            [&](uint32_t j) { return Raw{rj[j], ptmp[j]}; },
+            [&](const Raw& v) { return fma(T(1), v.r, nalpha * v.t); }, own);
+    } else if constexpr (SH != 0) {
         using VT = Vec16<T>;
         using V = typename VT::V;
         constexpr int W = VT::W;
@@ -281,12 +307,12 @@ __global__ void __launch_bounds__(kBlock) bi_s(CSRView<T> A, const T* __restrict
             stencil_group<T, SH>(A, g, nw, act, sg, c, sm);
             if (act)
 #pragma unroll
-                for (int j = 0; j < W; ++j) own((size_t)W * g + j, sm[j]);
+                for (int j = 0; j < W; ++j) own((size_t)W * g + j, sv((uint32_t)(W * g + j)), sm[j]);
         }
     } else if (L == 1) {
         for (size_t row = (size_t)blockIdx.x * blockDim.x + threadIdx.x; row < A.nrow;
              row += (size_t)gridDim.x * blockDim.x)
-            own(row, row_apply<T, false>(A, row, gv));
+            own(row, sv((uint32_t)row), row_apply<T, false>(A, row, gv));
     } else {
         const int lane = threadIdx.x & (L - 1);
         const size_t warpRows = 32 / L;
@@ -300,7 +326,7 @@ __global__ void __launch_bounds__(kBlock) bi_s(CSRView<T> A, const T* __restrict
                 for (uint32_t k = A.rowPtr[row] + lane; k < A.rowPtr[row + 1]; k += L)
                     sum = fma(A.val[k], gv(A.colInd[k]), sum);
             sum = group_sum<L>(sum);
-            if (lane == 0 && row < A.nrow) own(row, sum);
+            if (lane == 0 && row < A.nrow) own(row, sv((uint32_t)row), sum);
         }
     }
     double a[2] = {(double)a0, (double)a1};
@@ -349,6 +375,7 @@ __global__ void __launch_bounds__(kBlock) bi_x(uint32_t n, T* __restrict__ x, T*
     if (c->status != kRun) return;
     const T* __restrict__ pj = c->par ? p1 : p0;
     const T alpha = (T)c->alpha, omega = (T)c->omega, nomega = (T)(-c->omega);
+    const T zc = (T)c->zc;
     BiXSums<T> a;
     uint32_t i0 = 0;
     if (VEC) {
@@ -360,13 +387,13 @@ __global__ void __launch_bounds__(kBlock) bi_x(uint32_t n, T* __restrict__ x, T*
             T p[W], sv[W], d[W], xi[W], st[W], r0[W], r[W];
             *(VT*)p = ((const VT*)pj)[iv];
             *(VT*)sv = ((const VT*)sj)[iv];
-            if (JAC) *(VT*)d = ((const VT*)dinv)[iv];
+            if (JAC == 1) *(VT*)d = ((const VT*)dinv)[iv];
             *(VT*)xi = ((const VT*)x)[iv];
             *(VT*)st = ((const VT*)stmp)[iv];
             *(VT*)r0 = ((const VT*)r0s)[iv];
 #pragma unroll
             for (int e = 0; e < W; ++e)
-                bi_x_elem<T, JAC>(alpha, omega, nomega, p[e], sv[e], JAC ? d[e] : T(1), xi[e],
+                bi_x_elem<T, JAC>(alpha, omega, nomega, p[e], sv[e], JAC == 1 ? d[e] : zc, xi[e],
                                   st[e], r0[e], r[e], a);
             ((VT*)x)[iv] = *(VT*)xi;
             ((VT*)rj)[iv] = *(VT*)r;
@@ -376,7 +403,7 @@ __global__ void __launch_bounds__(kBlock) bi_x(uint32_t n, T* __restrict__ x, T*
     for (uint32_t i = i0 + blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += gridDim.x * blockDim.x) {
         T xi = x[i], r;
-        bi_x_elem<T, JAC>(alpha, omega, nomega, pj[i], sj[i], JAC ? dinv[i] : T(1), xi, stmp[i],
+        bi_x_elem<T, JAC>(alpha, omega, nomega, pj[i], sj[i], JAC == 1 ? dinv[i] : zc, xi, stmp[i],
                           r0s[i], r, a);
         x[i] = xi;
         rj[i] = r;
@@ -423,11 +450,13 @@ CSRView<float> bi_view<float>(const Mat& A) { return A.v32(); }
 // A launch that may overlap the previous kernel's tail (programmatic dependent launch): the
 // kernels wait for it to complete (pdl_wait) before their first memory access.
 template <typename... P, typename... A>
-static void bi_launch(void (*kern)(P...), int grid, cudaStream_t s, bool pdl, A&&... args)
+static void bi_launch(void (*kern)(P...), int grid, size_t smem, cudaStream_t s, bool pdl,
+                      A&&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -447,59 +476,75 @@ int BiEngine<T>::launch_iter()
     const int needV = c->grid(n, kBlock);
     auto fit = [&](const void* k, int need) { return std::min(need, resident_grid(*c, k, kBlock)); };
     T *p0 = pj2[0], *p1 = pj2[1], *t0 = ptmp2[0], *t1 = ptmp2[1];
-#define BI_SPMV(KP, KS, LL, JJ)                                                            \
+#define BI_PAIR(KP, KS, GP, GS, SMEM, WP, WS)                                              \
     do {                                                                                   \
-        bi_launch(KP<T, LL, JJ>, fit((const void*)KP<T, LL, JJ>, needS), c->stream, pdl, V,  \
-                  p0, p1, t0, t1, (const T*)rj, (const T*)r0s, dinv, ctl, c->red);          \
-        bi_launch(KS<T, LL, JJ>, fit((const void*)KS<T, LL, JJ>, needS), c->stream, pdl, V,  \
-                  (const T*)rj, (const T*)t0, (const T*)t1, dinv, sj, stmp, ctl, c->red);   \
+        bi_launch(KP, GP, SMEM, c->stream, pdl, V, p0, p1, t0, t1, (const T*)rj,            \
+                  (const T*)r0s, dinv, ctl, c->red, WP);                                    \
+        bi_launch(KS, GS, SMEM, c->stream, pdl, V, (const T*)rj, (const T*)t0,              \
+                  (const T*)t1, dinv, sj, stmp, ctl, c->red, WS);                           \
     } while (0)
+#define BI_SPMV(LL, JJ)                                                                    \
+    BI_PAIR((bi_p<T, LL, JJ>), (bi_s<T, LL, JJ>), fit((const void*)bi_p<T, LL, JJ>, needS), \
+            fit((const void*)bi_s<T, LL, JJ>, needS), 0, PlaneWalk(), PlaneWalk())
     // 16-byte row groups on 5- and 7-point stencil masks (bi_p / bi_s with SH)
     auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     const int sh = L == 1 && al16(p1) && al16(t1) && al16(r0s) && al16(sj) && al16(stmp)
                        ? stencil_vec_shape(V, p0, rj, t0)
                        : 0;
 #define BI_SPMV_SH(JJ, SS)                                                                 \
-    do {                                                                                   \
-        bi_launch(bi_p<T, 1, JJ, SS>, fit((const void*)bi_p<T, 1, JJ, SS>, needV),         \
-                  c->stream, pdl, V, p0, p1, t0, t1, (const T*)rj, (const T*)r0s, dinv, ctl, \
-                  c->red);                                                                 \
-        bi_launch(bi_s<T, 1, JJ, SS>, fit((const void*)bi_s<T, 1, JJ, SS>, needV),         \
-                  c->stream, pdl, V, (const T*)rj, (const T*)t0, (const T*)t1, dinv, sj,    \
-                  stmp, ctl, c->red);                                                      \
-    } while (0)
+    BI_PAIR((bi_p<T, 1, JJ, SS>), (bi_s<T, 1, JJ, SS>),                                    \
+            fit((const void*)bi_p<T, 1, JJ, SS>, needV),                                    \
+            fit((const void*)bi_s<T, 1, JJ, SS>, needV), 0, PlaneWalk(), PlaneWalk())
+    // plane walks, FP64 (FP32 keeps the order of its FP32 partial sums)
+    bool walked = false;
+#define BI_WALK(JJ)                                                                        \
+    if constexpr (sizeof(T) == 8) {                                                        \
+        const WalkLaunch wp = walk_launch(*c, V, (const void*)bi_p<T, 1, JJ, 0, true>);     \
+        const WalkLaunch ws = walk_launch(*c, V, (const void*)bi_s<T, 1, JJ, 0, true>);     \
+        walked = L == 1 && wp.grid && ws.grid;                                             \
+        if (walked)                                                                        \
+            BI_PAIR((bi_p<T, 1, JJ, 0, true>), (bi_s<T, 1, JJ, 0, true>), wp.grid, ws.grid, \
+                    wp.smem, wp.w, ws.w);                                                  \
+    }
 #define BI_LANES(JJ)                                                                       \
-    switch (sh ? -sh : L) {                                                                \
+    BI_WALK(JJ)                                                                            \
+    if (!walked) switch (sh ? -sh : L) {                                                   \
         case -5: BI_SPMV_SH(JJ, 5); break;                                                 \
         case -7: BI_SPMV_SH(JJ, 7); break;                                                 \
-        case 1: BI_SPMV(bi_p, bi_s, 1, JJ); break;                                         \
-        case 2: BI_SPMV(bi_p, bi_s, 2, JJ); break;                                         \
-        case 4: BI_SPMV(bi_p, bi_s, 4, JJ); break;                                         \
-        case 8: BI_SPMV(bi_p, bi_s, 8, JJ); break;                                         \
-        case 16: BI_SPMV(bi_p, bi_s, 16, JJ); break;                                       \
-        default: BI_SPMV(bi_p, bi_s, 32, JJ); break;                                       \
+        case 1: BI_SPMV(1, JJ); break;                                                     \
+        case 2: BI_SPMV(2, JJ); break;                                                     \
+        case 4: BI_SPMV(4, JJ); break;                                                     \
+        case 8: BI_SPMV(8, JJ); break;                                                     \
+        case 16: BI_SPMV(16, JJ); break;                                                   \
+        default: BI_SPMV(32, JJ); break;                                                   \
     }
     // 16-byte groups when every vector bi_x touches starts on a 16-byte boundary
     const bool vx = (((uintptr_t)x | (uintptr_t)rj | (uintptr_t)p0 | (uintptr_t)p1 |
                       (uintptr_t)sj | (uintptr_t)stmp | (uintptr_t)r0s |
-                      (uintptr_t)(jacobi ? dinv : p0)) & 15) == 0;
+                      (uintptr_t)(jacobi && !constDiag ? dinv : p0)) & 15) == 0;
     auto launch_x = [&](auto kern) {
-        bi_launch(kern, fit((const void*)kern, needV), c->stream, pdl, n, x, rj, (const T*)p0,
+        bi_launch(kern, fit((const void*)kern, needV), 0, c->stream, pdl, n, x, rj, (const T*)p0,
                   (const T*)p1, (const T*)sj, (const T*)stmp, (const T*)r0s, dinv, ctl, c->red);
     };
     if (jacobi && rightPcd) { // A (D v): the row kernels (no stencil groups)
         switch (L) {
-            case 1: BI_SPMV(bi_p, bi_s, 1, 2); break;
-            case 2: BI_SPMV(bi_p, bi_s, 2, 2); break;
-            case 4: BI_SPMV(bi_p, bi_s, 4, 2); break;
-            case 8: BI_SPMV(bi_p, bi_s, 8, 2); break;
-            case 16: BI_SPMV(bi_p, bi_s, 16, 2); break;
-            default: BI_SPMV(bi_p, bi_s, 32, 2); break;
+            case 1: BI_SPMV(1, 2); break;
+            case 2: BI_SPMV(2, 2); break;
+            case 4: BI_SPMV(4, 2); break;
+            case 8: BI_SPMV(8, 2); break;
+            case 16: BI_SPMV(16, 2); break;
+            default: BI_SPMV(32, 2); break;
         }
         if (vx)
             launch_x(bi_x<T, 1, 1>);
         else
             launch_x(bi_x<T, 1, 0>);
+    } else if (jacobi && constDiag) {
+        BI_LANES(3)
+        if (vx)
+            launch_x(bi_x<T, 3, 1>);
+        else
+            launch_x(bi_x<T, 3, 0>);
     } else if (jacobi) {
         BI_LANES(1)
         if (vx)
@@ -514,6 +559,8 @@ int BiEngine<T>::launch_iter()
             launch_x(bi_x<T, 0, 0>);
     }
 #undef BI_LANES
+#undef BI_WALK
+#undef BI_PAIR
 #undef BI_SPMV_SH
 #undef BI_SPMV
     if (!capturing) c->launches += 3;
@@ -536,6 +583,7 @@ int BiEngine<T>::launch_resume()
 template <typename T>
 int BiEngine<T>::push_ctl()
 {
+    hctl->zc = zc;
     FB_CUDA(cudaMemcpyAsync(ctl, hctl, sizeof(BiCtl), cudaMemcpyHostToDevice, c->stream));
     return kOk;
 }

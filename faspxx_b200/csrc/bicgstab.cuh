@@ -27,6 +27,7 @@ struct BiCtl {
     // recursive residual has fallen below delta x its largest value since the last refresh
     int      reliable;
     double   delta, rmax;
+    double   zc;        // the constant diagInv when the Jacobi diagonal is one value
     // which of the two direction buffers (pj, ptmp) holds the current iteration's values:
     // bi_p reads the other pair and flips it in its finalize
     int      par;
@@ -48,6 +49,10 @@ struct BiEngine {
     const Mat* A = nullptr;
     int        jacobi = 0;
     const T*   dinv = nullptr;
+    // a constant diagInv (every diagonal entry equal), set with zc before init: no kernel
+    // reads the vector, 3 of the 20 vectors an iteration moves
+    bool       constDiag = false;
+    double     zc = 0.0;
     T *x = nullptr, *rj = nullptr, *r0s = nullptr, *sj = nullptr, *stmp = nullptr;
     T *pj2[2] = {nullptr, nullptr}, *ptmp2[2] = {nullptr, nullptr}; // chosen by ctl->par
     T* pj(int par) const { return pj2[par & 1]; } // the direction of iteration par

@@ -485,10 +485,14 @@ int SolverImpl::setup(fasp_gpu_mat Mh)
                     bi32->pdl = cfg.overlapLaunch != 0;
                     bi32->rightPcd = cfg.precision == FASP_GPU_MIXED_RELIABLE && cfg.pcd == 1 &&
                                      !A->diagConst;
+                    bi32->constDiag = cfg.pcd == 1 && A->diagConst;
+                    bi32->zc = (1.0 / A->diagValue) * pcd.weight;
                     if ((e = bi32->init(&c, A, cfg.pcd, pcd.dinv32, cfg.useGraph != 0))) return e;
                 } else {
                     bi64 = new BiEngine<double>();
                     bi64->pdl = cfg.overlapLaunch != 0;
+                    bi64->constDiag = cfg.pcd == 1 && A->diagConst;
+                    bi64->zc = (1.0 / A->diagValue) * pcd.weight;
                     if ((e = bi64->init(&c, A, cfg.pcd, pcd.dinv, cfg.useGraph != 0))) return e;
                 }
             } else if (cfg.precision == FASP_GPU_MIXED_RELIABLE) {
