@@ -583,6 +583,8 @@ int BiEngine<T>::launch_resume()
 template <typename T>
 int BiEngine<T>::push_ctl()
 {
+    hctl->hst = hstatus;
+    *hstatus = hctl->status;
     hctl->zc = zc;
     FB_CUDA(cudaMemcpyAsync(ctl, hctl, sizeof(BiCtl), cudaMemcpyHostToDevice, c->stream));
     return kOk;
@@ -622,12 +624,12 @@ int BiEngine<T>::init(Ctx* ctx, const Mat* M, int jac, const T* dinvv, bool grap
     std::memset(hctl, 0, sizeof(BiCtl));
     hctl->histScale = 1.0;
     if (useGraph) {
+        itersPerGraph = 4;
         cudaGraph_t g;
         FB_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         capturing = true;
         for (int i = 0; i < itersPerGraph; ++i) launch_iter();
         capturing = false;
-        cudaMemcpyAsync(hstatus, &ctl->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
         FB_CUDA(cudaStreamEndCapture(c->stream, &g));
         FB_CUDA(cudaGraphInstantiate(&gexec, g, 0));
         cudaGraphDestroy(g);
@@ -663,8 +665,6 @@ int BiEngine<T>::run(unsigned* launches)
                 int e = launch_iter();
                 if (e) return e;
             }
-            FB_CUDA(cudaMemcpyAsync(hstatus, &ctl->status, sizeof(int), cudaMemcpyDeviceToHost,
-                                    c->stream));
             FB_CUDA(cudaStreamSynchronize(c->stream));
             if (launches) *launches += 3 * itersPerGraph;
             if (*hstatus != kRun) return kOk;
@@ -673,7 +673,6 @@ int BiEngine<T>::run(unsigned* launches)
     cudaEvent_t ev[2];
     FB_CUDA(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
     FB_CUDA(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
-    *hstatus = kRun;
     int cur = 0;
     FB_CUDA(cudaGraphLaunch(gexec, c->stream));
     FB_CUDA(cudaEventRecord(ev[cur], c->stream));

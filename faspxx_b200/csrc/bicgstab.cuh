@@ -13,6 +13,7 @@ enum BiReason { kBiNone = 0, kBiSave = 1, kBiStag = 2, kBiCheck = 3, kBiRefresh 
 // memory so that the finalize thread of each fused kernel runs the reference's control flow.
 struct BiCtl {
     int      status, reason, code, phase;
+    int*     hst;       // page-locked copy of status, stored when it changes
     int      bench;     // 1: kernel timing, the finalize steps do nothing
     unsigned numIter, minIter, maxIter, savIter, restart, stagStep, moreStep;
     double   relTol, absTol, solStagTol;
@@ -58,8 +59,10 @@ struct BiEngine {
     T* pj(int par) const { return pj2[par & 1]; } // the direction of iteration par
     BiCtl*     ctl = nullptr;     // device
     BiCtl*     hctl = nullptr;    // pinned host copy
-    int*       hstatus = nullptr; // pinned, written at the end of every graph launch
+    int*       hstatus = nullptr; // pinned, BiCtl::hst
     cudaGraphExec_t gexec = nullptr;
+    // 8 between the plain launches' waits, 4 a graph: up to two graphs of empty kernels run
+    // after the last iteration, and a graph boundary costs less than 1 us
     int        itersPerGraph = 8;
     bool       useGraph = true;
     bool       pdl = true; // programmatic dependent launch between the iteration's kernels

@@ -1710,6 +1710,8 @@ int CGEngine<T>::launch_resume()
 template <typename T>
 int CGEngine<T>::push_ctl()
 {
+    hctl->hst = hstatus;
+    *hstatus = hctl->status;
     hctl->zc = zc;
     hctl->onered = onered() ? 1 : 0;
     FB_CUDA(cudaMemcpyAsync(ctl, hctl, sizeof(CGCtl), cudaMemcpyHostToDevice, c->stream));
@@ -1751,14 +1753,13 @@ int CGEngine<T>::init(Ctx* ctx, const Mat* M, int jac, const T* dinvv, bool grap
     FB_CUDA(cudaMemsetAsync(P0, 0, bytes, c->stream));
     FB_CUDA(cudaMemsetAsync(P1, 0, bytes, c->stream));
     if (useGraph) {
-        // itersPerGraph iterations + a status read-back, captured once; kernels read every
-        // scalar from the control block, so the graph never needs updating.
+        // itersPerGraph iterations, captured once; kernels read every scalar from the control
+        // block, so the graph never needs updating.
         cudaGraph_t g;
         FB_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         capturing = true;
         for (int i = 0; i < itersPerGraph; ++i) launch_iter();
         capturing = false;
-        cudaMemcpyAsync(hstatus, &ctl->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
         FB_CUDA(cudaStreamEndCapture(c->stream, &g));
         FB_CUDA(cudaGraphInstantiate(&gexec, g, 0));
         cudaGraphDestroy(g);
@@ -1970,8 +1971,6 @@ int CGEngine<T>::run(unsigned* launches)
                 int e = launch_iter();
                 if (e) return e;
             }
-            FB_CUDA(cudaMemcpyAsync(hstatus, &ctl->status, sizeof(int), cudaMemcpyDeviceToHost,
-                                    c->stream));
             FB_CUDA(cudaStreamSynchronize(c->stream));
             if (launches) *launches += 2 * itersPerGraph;
             if (*hstatus != kRun && *hstatus != kRefresh) return kOk;
@@ -1980,7 +1979,6 @@ int CGEngine<T>::run(unsigned* launches)
     cudaEvent_t ev[2];
     FB_CUDA(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
     FB_CUDA(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
-    *hstatus = kRun;
     int cur = 0;
     FB_CUDA(cudaGraphLaunch(gexec, c->stream));
     FB_CUDA(cudaEventRecord(ev[cur], c->stream));
@@ -1996,7 +1994,7 @@ int CGEngine<T>::run(unsigned* launches)
             err = kErrCuda;
             break;
         }
-        // hstatus was written by the graph that ev[cur] follows (stream order)
+        // stores of the status by the graph that ev[cur] follows have arrived
         if (*hstatus != kRun && *hstatus != kRefresh) break;
         cur ^= 1;
     }

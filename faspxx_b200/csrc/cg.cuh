@@ -22,6 +22,7 @@ struct GridBar {
 
 struct CGCtl {
     int      status, reason, code, phase;
+    int*     hst;       // page-locked copy of status, stored when it changes
     int      pmode;     // 0: p = z (first iteration or restart), 1: p = z + beta p
     int      par;       // which of the two p buffers holds the current direction
     int      pzero;     // the host zeroed p (a restart): next p = z
@@ -91,7 +92,7 @@ struct CGEngine {
     T *x = nullptr, *r = nullptr, *z = nullptr, *q = nullptr, *P0 = nullptr, *P1 = nullptr;
     CGCtl*     ctl = nullptr;    // device
     CGCtl*     hctl = nullptr;   // pinned host copy
-    int*       hstatus = nullptr;// pinned, written at the end of every graph launch
+    int*       hstatus = nullptr;// pinned, CGCtl::hst
     cudaGraphExec_t gexec = nullptr;
     int        itersPerGraph = 16;
     bool       useGraph = true;

@@ -137,7 +137,9 @@ __device__ __forceinline__ void grid_reduce(double (&acc)[NV], const int (&ops)[
 // shared memory with one parallel read (issued before the partials are summed, so the two
 // overlap), thread 0 runs fin(ctl_in_shared_memory, totals), and the block writes it back.
 // Only the last block touches the control block after the ticket: every other block has
-// read what it needs before its own reduction.
+// read what it needs before its own reduction. A change of Ctl::status is also stored to the
+// page-locked word Ctl::hst, set when the control block is sent: a graph of iterations then
+// needs no copy of it at its end, which had kept the next graph waiting for 8 to 10 us.
 template <int NV, typename Ctl, typename Fin>
 __device__ __forceinline__ void grid_reduce_ctl(double (&acc)[NV], const int (&ops)[NV],
                                                 Scratch s, Ctl* gctl, Fin fin)
@@ -159,7 +161,12 @@ __device__ __forceinline__ void grid_reduce_ctl(double (&acc)[NV], const int (&o
     double tot[NV];
     sum_partials<NV>(s.partials, ops, tot);
     block_reduce<NV>(tot, ops); // ends with a barrier: sc is complete
-    if (threadIdx.x == 0) fin(reinterpret_cast<Ctl*>(sc), tot);
+    if (threadIdx.x == 0) {
+        Ctl* cs = reinterpret_cast<Ctl*>(sc);
+        const int was = cs->status;
+        fin(cs, tot);
+        if (cs->status != was) *(volatile int*)cs->hst = cs->status;
+    }
     __syncthreads();
     for (int w = threadIdx.x; w < kWords; w += blockDim.x) __stcg(g + w, sc[w]);
 }
