@@ -828,6 +828,51 @@ __global__ void __launch_bounds__(kBlock, (V4 ? 3 : (L > 1 ? 4 : (sizeof(T) == 4
     }
 }
 
+// cg_spmv (FP64, p formed where it is gathered) on plain CSR in block tiles, for a
+// few rounds of blocks: the matrix does not change during a solve, so a block has its entries
+// copied while the previous kernel is still reducing, and its rows wait only for the gathers.
+// See launch_spmv_kernel for where it pays.
+template <int JZ>
+__global__ void __launch_bounds__(kBlock, 4)
+    cg_spmv_tiles(CSRView<double> A, const double* __restrict__ z, double* P0, double* P1,
+                  double* __restrict__ q, CGCtl* c, Scratch s)
+{
+    TileSmem<double>& sm = *reinterpret_cast<TileSmem<double>*>(fb_tile_smem);
+    const CsrTiles<double, false> tiles(A, sm);
+    if (threadIdx.x == 0) tiles.begin();
+    pdl_wait();
+    pdl_release();
+    const int status = c->status;
+    const int mode = c->pmode, par = c->par;
+    const double zc = c->zc, beta = c->beta;
+    if (status != kRun) {
+        if (threadIdx.x == 0) tiles.drain();
+        return;
+    }
+    const double* __restrict__ pOld = par ? P1 : P0;
+    double* __restrict__ pNew = par ? P0 : P1;
+    double acc = 0.0;
+    auto pat = [&](size_t j) { // the new p at j
+        const double zi = JZ == 2 ? zc * z[j] : z[j];
+        return mode ? fma(beta, pOld[j], zi) : zi;
+    };
+    csr_tile_rows<double, false, 1, true>(
+        A, sm, [&](uint32_t j) { return pat(j); },
+        [&](size_t row, double sum) {
+            const double pi = pat(row);
+            pNew[row] = pi;
+            q[row] = sum;
+            acc = fma(sum, pi, acc);
+        });
+    if (sm.bad) acc = (double)NAN; // rows are missing: no direction to go on with
+    double a[1] = {acc};
+    const int ops[1] = {kSum};
+    grid_reduce_ctl<1>(a, ops, s, c, [=] __device__(CGCtl* cs, const double* t) {
+        cs->par = par ^ 1;
+        if (!cs->bench) cg_after_spmv(cs, t[0]);
+    });
+}
+
 template <typename T, int JAC>
 __global__ void __launch_bounds__(kBlock, 4) cg_update(uint32_t n, T* __restrict__ x,
                                                     T* __restrict__ r, T* __restrict__ z,
@@ -1557,6 +1602,13 @@ static MarchPlan march_plan(const V& A, int sh, int grid, int rpg)
     return mp;
 }
 
+// FP64 plain CSR runs cg_spmv_tiles where matrix and vectors together stay in L2 and the tiles'
+// four blocks an SM need fewer than 1.5 times the rounds of the row kernel's five. An iteration
+// on a seven-point matrix, row kernel and tiles: 40^3 12.7 and 12.3 us, 50^3 15.5 and 14.6, 64^3
+// 19.0 and 17.5, 80^3 25.4 and 24.2, 90^3 32.1 and 30.4; 56^3 (one round against two) 15.9 and
+// 16.4, 70^3 (two against three) 20.7 and 21.0, 100^3 (124 MB) 40.5 and 40.4.
+constexpr unsigned long long kTileBytes = 110ull << 20;
+
 // The two fused kernels, each on one resident wave (grid from the occupancy limit).
 template <typename T>
 void CGEngine<T>::launch_spmv_kernel()
@@ -1566,15 +1618,31 @@ void CGEngine<T>::launch_spmv_kernel()
     const int jm = jmode();
     const T* zz = jm == 1 ? z : r;
     const int sh = stencil_shape(V);
-    // The fused iteration kernels walk CSR rows one at a time, without block tiles: with its
-    // p, q, x updates per row a tile's block barrier stalls every warp on the slowest one,
-    // and on B200 the 128^3 CSR solves measured slower with tiles (mixed 16.3 against 14.9
-    // ms, FP64 28.9 against 25.0 ms) although the product alone is faster.
+    // Large CSR systems are walked one row at a time, without block tiles: a tile's barrier
+    // stalls every warp on the slowest one, and the 128^3 solves measured slower with tiles
+    // (mixed 16.3 against 14.9 ms, FP64 28.9 against 25.0 ms) although the product alone is
+    // faster.
     auto go = [&](auto kern) {
         const int g = std::min(need, resident_grid(*c, (const void*)kern, kBlock));
         launch_overlapped(kern, g, c->stream, pdl, V, zz, P0, P1, q, x, ctl, c->red,
                           march_plan(V, sh, g, sizeof(T) == 4 ? 4 : 2));
     };
+    if constexpr (sizeof(T) == 8) {
+        CSRView<T> W = V;
+        const size_t smem = A->lanes == 1 && !recurrence ? with_tiles(W, kBlock) : 0;
+        if (smem && A->nnz * 12ull + A->nrow * 48ull <= kTileBytes) {
+            auto kern = jm == 2 ? cg_spmv_tiles<2> : cg_spmv_tiles<0>;
+            auto rows = jm == 2 ? cg_spmv<T, 1, 0, 2> : cg_spmv<T, 1, 0, 0>;
+            const int tiles = (int)((A->nrow + kTileRows - 1) / kTileRows);
+            const int g = std::min(tiles, resident_grid(*c, (const void*)kern, kBlock, smem));
+            const int gr = std::min(tiles, resident_grid(*c, (const void*)rows, kBlock));
+            const int roundsT = (tiles + g - 1) / g, roundsR = (tiles + gr - 1) / gr;
+            if (2 * roundsT < 3 * roundsR && tiles_fit((const void*)kern, smem)) {
+                launch_overlapped_smem(kern, g, smem, c->stream, pdl, W, zz, P0, P1, q, ctl, c->red);
+                return;
+            }
+        }
+    }
     auto al = [](const void* p, uintptr_t a) { return ((uintptr_t)p & (a - 1)) == 0; };
     // vector rows (stencil masks, see cg_spmv): four per thread for the FP32 recurrences,
     // two for FP64 on the 5- and 7-point shapes
@@ -2111,5 +2179,7 @@ int to32(Ctx& c, uint32_t n, const double* s, float* d)
     FB_CUDA(cudaGetLastError());
     return kOk;
 }
+
+unsigned tile_timeouts_cg() { return tile_timeouts(); }
 
 } // namespace fb

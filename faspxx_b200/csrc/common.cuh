@@ -450,28 +450,29 @@ struct RowSep {
     __device__ __forceinline__ T start(size_t row) const { return from(row); }
 };
 
-// Rows of a plain CSR view in block tiles; own(row, sum) on the row's first thread. L threads own
-// a row (L = 1: one), so a tile has 256 / L rows. Block b takes tiles b, b + G, b + 2G, ...
-// (G = gridDim.x); for L = 1, thread t of the grid owns rows t, t + S, t + 2S, ... (S = the
-// grid's threads) in that order, as the row-at-a-time loops do. Sums with FMAs are those of
-// row_dot (L = 1) and of the lane kernels (L > 1: lane l takes entries l, l + L, ..., then
-// a shuffle tree); separately rounded sums go left to right whatever L. Every
-// thread of the block calls it (it synchronises the block). A tile whose entries do not fit
-// a stage (only possible when the caller ignored the span check of with_tiles) is summed
-// from global memory.
-template <typename T, bool PAT, int L = 1, typename XV, typename OWN, typename ACC = RowFma>
-__device__ __forceinline__ void csr_tile_rows(const CSRView<T>& A, TileSmem<T>& sm, XV xv,
-                                              OWN own, ACC acc = ACC())
-{
-    constexpr uint32_t R = kTileRows / L; // rows of a tile
-    constexpr uint32_t CAP = TileShape<T>::cap;
-    const size_t n = A.nrow;
-    const size_t ntiles = (n + R - 1) / R;
-    const uint32_t tid = threadIdx.x;
-    const size_t mine =
-        blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-    const unsigned long long pol = tid == 0 ? l2_evict_first() : 0ull;
-    auto issue = [&](size_t k) { // thread 0: tile k of this block into stage k % stages
+// The first tiles of this block, on their way before csr_tile_rows<..., BEGUN = true> (thread 0
+// copies; the matrix must be complete, whatever else the kernel still waits for). A kernel that
+// returns without the rows calls csr_tiles_drain first.
+template <typename T, bool PAT, int L = 1>
+struct CsrTiles {
+    static constexpr uint32_t R = kTileRows / L; // rows of a tile
+    static constexpr uint32_t CAP = TileShape<T>::cap;
+    const CSRView<T>& A;
+    TileSmem<T>& sm;
+    const unsigned long long pol;
+    __device__ __forceinline__ CsrTiles(const CSRView<T>& A_, TileSmem<T>& sm_)
+        : A(A_), sm(sm_), pol(threadIdx.x == 0 ? l2_evict_first() : 0ull)
+    {
+    }
+    __device__ __forceinline__ size_t mine() const // tiles of this block
+    {
+        const size_t ntiles = ((size_t)A.nrow + R - 1) / R;
+        return blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    }
+    // thread 0: tile k of this block into stage k % stages
+    __device__ __forceinline__ void issue(size_t k) const
+    {
+        const size_t n = A.nrow;
         const int s = (int)(k % kTileStages);
         const size_t r0 = (blockIdx.x + k * gridDim.x) * R;
         const size_t rows = n - r0 < R ? n - r0 : R;
@@ -494,15 +495,43 @@ __device__ __forceinline__ void csr_tile_rows(const CSRView<T>& A, TileSmem<T>& 
                 bulk_copy_g2s(sm.st[s].v, A.val + a, (ar - a) * (uint32_t)sizeof(T),
                               &sm.full[s], pol);
         }
-    };
-    if (tid == 0) {
+    }
+    __device__ __forceinline__ void begin() const // thread 0
+    {
         sm.bad = 0;
         for (int s = 0; s < kTileStages; ++s)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.full[s]))
                          : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (size_t k = 0; k < (size_t)kTileStages && k < mine; ++k) issue(k);
+        const size_t m = mine();
+        for (size_t k = 0; k < (size_t)kTileStages && k < m; ++k) issue(k);
     }
+    __device__ __forceinline__ void drain() const // thread 0, after begin(): before an early exit
+    {
+        const size_t m = mine();
+        for (size_t k = 0; k < (size_t)kTileStages && k < m; ++k) mbar_wait_bounded(&sm.full[k], 0);
+    }
+};
+
+// Rows of a plain CSR view in block tiles; own(row, sum) on the row's first thread. L threads own
+// a row (L = 1: one), so a tile has 256 / L rows. Block b takes tiles b, b + G, b + 2G, ...
+// (G = gridDim.x); for L = 1, thread t of the grid owns rows t, t + S, t + 2S, ... (S = the
+// grid's threads) in that order, as the row-at-a-time loops do. Sums with FMAs are those of
+// row_dot (L = 1) and of the lane kernels (L > 1: lane l takes entries l, l + L, ..., then
+// a shuffle tree); separately rounded sums go left to right whatever L. Every
+// thread of the block calls it (it synchronises the block). A tile whose entries do not fit
+// a stage (only possible when the caller ignored the span check of with_tiles) is summed
+// from global memory.
+template <typename T, bool PAT, int L = 1, bool BEGUN = false, typename XV, typename OWN,
+          typename ACC = RowFma>
+__device__ __forceinline__ void csr_tile_rows(const CSRView<T>& A, TileSmem<T>& sm, XV xv,
+                                              OWN own, ACC acc = ACC())
+{
+    constexpr uint32_t R = kTileRows / L; // rows of a tile
+    const CsrTiles<T, PAT, L> tiles(A, sm);
+    const size_t n = A.nrow, mine = tiles.mine();
+    const uint32_t tid = threadIdx.x;
+    if (!BEGUN && tid == 0) tiles.begin();
     __syncthreads();
     for (size_t k = 0; k < mine; ++k) {
         const int s = (int)(k % kTileStages);
@@ -614,7 +643,7 @@ __device__ __forceinline__ void csr_tile_rows(const CSRView<T>& A, TileSmem<T>& 
                                       (uint32_t)((j / kTileStages) & 1));
             return;
         }
-        if (tid == 0 && k + kTileStages < mine) issue(k + kTileStages);
+        if (tid == 0 && k + kTileStages < mine) tiles.issue(k + kTileStages);
     }
 }
 

@@ -410,6 +410,8 @@ int dmalloc(void** p, size_t bytes, cudaStream_t s);
 // landed).
 unsigned tile_timeouts_spmv();
 unsigned tile_timeouts_solvers();
+unsigned tile_timeouts_cg();
+unsigned tile_timeouts_mg();
 // v = A^T v1 + v2 on T = m_transpose(A), in MAT::MultTransposeAdd's order (MAT.cxx:541-606)
 int m_mult_transpose_add(Ctx& c, const Mat& T, const double* v1, const double* v2, double* v);
 int lanes_for(double meanRowLen);                                         // SpMV mapping

@@ -402,4 +402,6 @@ int SolverImpl::mg_cycle_fixed(const double* b, double* x, bool zero)
     return cycle(*this, 0, b, x, zero, in, &end);
 }
 
+unsigned tile_timeouts_mg() { return tile_timeouts(); }
+
 } // namespace fb

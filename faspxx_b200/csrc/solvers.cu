@@ -2667,6 +2667,9 @@ int SolverImpl::solve(const double* b, double* x, fasp_gpu_info* info)
     return e;
 }
 
-unsigned tile_timeouts_solvers() { return tile_timeouts() + tile_timeouts_dcgs2(); }
+unsigned tile_timeouts_solvers()
+{
+    return tile_timeouts() + tile_timeouts_dcgs2() + tile_timeouts_cg() + tile_timeouts_mg();
+}
 
 } // namespace fb

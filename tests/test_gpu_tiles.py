@@ -193,3 +193,34 @@ def test_residual_shortcut(gpu, n, where):
     M.Residual(gpu.DVec.from_numpy(b), gpu.DVec.from_numpy(x), r)
     want = b if where in ("none", "nan") else b - A.values * x
     assert np.allclose(r.numpy(), want, rtol=1e-15, atol=0)
+
+
+@pytest.mark.parametrize("pcd", [None, "jacobi"])
+@pytest.mark.parametrize("kind,n", [("var", 3), ("var", 8), ("var", 50), ("var", 64), ("var", 80),
+                                    ("poisson", 20), ("poisson", 64)])
+def test_cg_tiles(gpu, kind, n, pcd):
+    """The first iterations of FP64 CG on plain CSR (one block, one and several tiles a block, a
+    ragged last tile; varying and constant diagonals) against two lanes a row, which walk the rows
+    without tiles. The two differ in the order of the sums: less than 1e-13 of a sum of 5e5
+    terms, carried through four steps by recurrences that cancel at most tenfold each: 1e-9 of a
+    residual norm, 1e-11 of max|x|."""
+    rng = np.random.default_rng(n)
+    A = P.poisson3d(n) if kind == "poisson" else P.vardiff3d(n, rng.uniform(0.5, 2.0, (n, n, n)))
+    b, x0 = rng.uniform(-1, 1, A.nrow), rng.uniform(-1, 1, A.nrow)
+    got = []
+    for lanes in (1, 2):
+        M = gpu.MAT(A)
+        M.SetRowClass(CSR)
+        M.SetCol16(False)
+        M.SetLanes(lanes)
+        s = gpu.configure("cg", maxIter=4, relTol=1e-30, absTol=0.0, pcd=pcd, pcdWeight=2.0 / 3.0,
+                          pcdIter=1)
+        s.Setup(M)
+        x = x0.copy()
+        s.Solve(b, x)
+        assert s.GetIterations() == 4
+        got.append((x, s.History()[:5]))
+    (x1, h1), (x2, h2) = got
+    assert np.all(np.abs(h1 - h2) <= 1e-9 * h2)
+    assert np.max(np.abs(x1 - x2)) <= 1e-11 * np.max(np.abs(x2))
+    assert gpu.tile_timeouts() == 0
