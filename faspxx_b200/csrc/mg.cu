@@ -26,11 +26,36 @@ __device__ __forceinline__ void mark_above(bool above, double* out)
 
 __device__ __forceinline__ bool above_zero(double x) { return fabs(x) >= kCloseZero; }
 
-// Rows of A on L lanes each (L = 1: one thread, block tiles where the view has them):
-// own(row, sum) on the row's first lane.
+__device__ __forceinline__ TileSmem<double>& tile_smem()
+{
+    return *reinterpret_cast<TileSmem<double>*>(fb_tile_smem);
+}
+
+// First in a kernel, before it waits for its predecessor: no kernel of a cycle writes a matrix, so
+// the block's first tiles are copied while the predecessor still runs. rows_of() takes them, a
+// kernel without rows_of() calls no_rows().
+template <int L>
+__device__ __forceinline__ void tiles_first(const CSRView<double>& A)
+{
+    if (A.tiles && threadIdx.x == 0) CsrTiles<double, false, L>(A, tile_smem()).begin();
+}
+
+template <int L>
+__device__ __forceinline__ void no_rows(const CSRView<double>& A)
+{
+    if (A.tiles && threadIdx.x == 0) CsrTiles<double, false, L>(A, tile_smem()).drain();
+}
+
+// Rows of A on L lanes each, in block tiles where the view has them (see tiles_first; both ways
+// the same sums): own(row, sum) on the row's first lane. A sweep of the 27-point level of 63^3
+// rows took 27.5 us row by row, 22.6 in tiles (cold).
 template <int L, typename XV, typename OWN>
 __device__ __forceinline__ void rows_of(const CSRView<double>& A, XV xv, OWN own)
 {
+    if (A.tiles) {
+        csr_tile_rows<double, false, L, true>(A, tile_smem(), xv, own);
+        return;
+    }
     if (L == 1) {
         for_rows<double, false>(A, xv, own);
         return;
@@ -61,6 +86,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_mg_sweep(CSRView<double> A, const
                                                      double* __restrict__ xout,
                                                      const double* __restrict__ in, double* out)
 {
+    tiles_first<L>(A);
     pdl_wait();
     pdl_release();
     const bool shortcut = *in < kCloseZero;
@@ -71,13 +97,37 @@ __global__ void __launch_bounds__(kBlock, 5) k_mg_sweep(CSRView<double> A, const
         xout[i] = xi;
         above = above || above_zero(xi);
     };
-    if (shortcut)
+    if (shortcut) {
+        no_rows<L>(A);
         for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.nrow;
              i += (size_t)gridDim.x * blockDim.x)
             own(i, 0.0);
-    else
+    } else {
         rows_of<L>(A, [&](uint32_t j) { return x0(j); }, own);
+    }
     mark_above(above, out);
+}
+
+// r = b - A x, or r = b by the same shortcut (MAT.cxx:455-476).
+template <int L>
+__global__ void __launch_bounds__(kBlock) k_mg_residual(CSRView<double> A,
+                                                        const double* __restrict__ b,
+                                                        const double* __restrict__ x,
+                                                        double* __restrict__ r,
+                                                        const double* __restrict__ in)
+{
+    tiles_first<L>(A);
+    pdl_wait();
+    pdl_release();
+    auto own = [&](size_t i, double s) { r[i] = b[i] - s; };
+    if (*in < kCloseZero) {
+        no_rows<L>(A);
+        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.nrow;
+             i += (size_t)gridDim.x * blockDim.x)
+            own(i, 0.0);
+    } else {
+        rows_of<L>(A, [&](uint32_t j) { return x[j]; }, own);
+    }
 }
 
 // The first sweep from x = 0: x = dinv .* b.
@@ -103,6 +153,7 @@ __global__ void __launch_bounds__(kBlock) k_mg_restrict(CSRView<double> R, const
                                                         double* __restrict__ bc,
                                                         const double* __restrict__ dinv, double* out)
 {
+    tiles_first<L>(R);
     pdl_wait();
     pdl_release();
     bool above = false;
@@ -118,6 +169,7 @@ template <int L>
 __global__ void __launch_bounds__(kBlock) k_mg_correct(CSRView<double> P, const double* __restrict__ e,
                                                        double* __restrict__ x, double* out)
 {
+    tiles_first<L>(P);
     pdl_wait();
     pdl_release();
     bool above = false;
@@ -132,9 +184,14 @@ __global__ void __launch_bounds__(kBlock) k_mg_correct(CSRView<double> P, const 
 // A whole Jacobi::Solve (Iter.cxx:56-112) on at most 1,024 rows, thread per row, with the
 // matrix and x in shared memory: a sweep of a 27-row coarsest level waits for shared memory and
 // one or two block barriers instead of global loads (40 sweeps: 105 -> 12 us on B200). Rows are
-// summed left to right as row_apply sums them. zero: x is taken as 0 and not read.
-template <typename T>
-__global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
+// summed left to right as row_apply sums them. zero: x is taken as 0 and not read. RE: the first
+// RE entries of a row stay in registers over the sweeps, whose only loads are then the gathers,
+// all in flight at once: 40 sweeps of 27 rows 27 us instead of 35 (cold, with the launch). One warp
+// only: with the four warps of 125 rows 40 sweeps took 5 us more than from shared memory.
+constexpr int kSmallRegs = 32;
+
+template <typename T, int RE>
+__global__ void __launch_bounds__(RE ? kSmallRegs : 1024) k_jacobi_small(uint32_t n, uint32_t nnz,
                                                        const uint32_t* __restrict__ rowPtr,
                                                        const uint32_t* __restrict__ colInd,
                                                        const T* __restrict__ val,
@@ -161,6 +218,17 @@ __global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
     const T bi = row ? b[t] : T(0);
     T xi = row && !zero ? x[t] : T(0);
     if (row) sx[t] = xi;
+    T rv[RE ? RE : 1];
+    uint32_t rc[RE ? RE : 1];
+    const uint32_t re = min(r1 - r0, (uint32_t)RE);
+    if (RE) {
+        __syncthreads(); // the entries are in shared memory
+#pragma unroll
+        for (int u = 0; u < RE; ++u) {
+            rv[u] = (uint32_t)u < re ? sv[r0 + u] : T(0);
+            rc[u] = (uint32_t)u < re ? sc[r0 + u] : 0u;
+        }
+    }
     // the block's sum of v, the same on every thread
     auto all = [&](double v) {
         v = warp_reduce(v, kSum);
@@ -173,8 +241,16 @@ __global__ void __launch_bounds__(1024) k_jacobi_small(uint32_t n, uint32_t nnz,
     bool above = __syncthreads_or(above_zero((double)xi)); // orders the writes of sx too
     for (uint32_t it = 0; it < prm.maxIter; ++it) {
         T s = T(0);
+        if (RE && above) {
+            T g[RE ? RE : 1];
+#pragma unroll
+            for (int u = 0; u < RE; ++u) g[u] = sx[rc[u]];
+#pragma unroll
+            for (int u = 0; u < RE; ++u)
+                if ((uint32_t)u < re) s = fma(rv[u], g[u], s);
+        }
         if (above)
-            for (uint32_t k = r0; k < r1; k += 8) { // eight entries' loads, then their FMAs
+            for (uint32_t k = r0 + re; k < r1; k += 8) { // eight entries' loads, then their FMAs
                 uint32_t c[8];
                 T v[8], g[8];
 #pragma unroll
@@ -232,7 +308,7 @@ template <typename... P, typename... X>
 int launch_rows(Ctx& c, const Mat& A, int lanes, void (*kern)(CSRView<double>, P...), X... args)
 {
     CSRView<double> V = A.v64();
-    size_t smem = lanes == 1 ? with_tiles(V, kBlock) : 0;
+    size_t smem = with_tiles(V, kBlock, A.span(lanes));
     if (smem && !tiles_fit((const void*)kern, smem)) V.tiles = 0, smem = 0;
     const int g = std::min(c.grid((long long)A.nrow * lanes, kBlock),
                            resident_grid(c, (const void*)kern, kBlock, smem));
@@ -257,7 +333,7 @@ int jacobi_small(Ctx& c, const Mat& A, const T* val, const T* b, T* x, const T* 
                  const fasp_gpu_params& prm, bool zero, double* mark)
 {
     const size_t smem = small_bytes(A, sizeof(T));
-    const auto kern = k_jacobi_small<T>;
+    const auto kern = A.nrow <= kSmallRegs ? k_jacobi_small<T, 32> : k_jacobi_small<T, 0>;
     FB_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kSmallBytes));
     ++c.launches;
@@ -359,9 +435,16 @@ static int cycle(SolverImpl& S, uint32_t l, const double* b, double* x, bool zer
     double* r = l == 0 ? S.w[0] : S.mgRes[l];
     int e;
     double* s = nullptr;
-    if ((e = smooth(S, S.mgSmooth[l], b, x, zero, in, &s)) ||
-        (e = m_residual(c, A, b, (const double*)x, r, (const double*)s)))
-        return e;
+    if ((e = smooth(S, S.mgSmooth[l], b, x, zero, in, &s))) return e;
+    CSRView<double> V = A.v64();
+    if (with_tiles(V, kBlock, A.span(A.lanes)))
+        by_lanes(A.lanes, [&](auto L) {
+            e = launch_rows(c, A, A.lanes, k_mg_residual<decltype(L)::value>, b, (const double*)x, r,
+                            (const double*)s);
+        });
+    else // stencils keep their row groups
+        e = m_residual(c, A, b, (const double*)x, r, (const double*)s);
+    if (e) return e;
     Pcd& next = l + 1 == NL ? S.mgCoarse[l] : S.mgSmooth[l + 1];
     double* first = S.mgInf + S.mgInfUsed++;
     const int rl = transfer_lanes(R), pl = transfer_lanes(P);

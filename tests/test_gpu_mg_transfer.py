@@ -331,3 +331,26 @@ def test_fixed_cycles_match_tested_ones(gpu, O, dim, nf, L, sweeps, coarse, cycl
             out.append(x)
     for k in (0, 1):
         assert np.max(np.abs(out[k] - out[k + 2])) <= 1e-12 * np.max(np.abs(out[k + 2]))
+
+
+@pytest.mark.parametrize("n", [1, 5, 27, 31, 32, 33, 125])
+def test_small_jacobi(gpu, n):
+    """Forty Jacobi sweeps of a small system in one launch (rows of up to 32 entries in registers
+    for at most 32 rows) against numpy: each sweep rounds a row of at most 33 products, the
+    iteration contracts, so 40 x 35 ulp of max|x| bounds the difference."""
+    rng = np.random.default_rng(n)
+    D = rng.uniform(-1, 1, (n, n)) * (rng.random((n, n)) < 0.8)
+    if n > 33:
+        D *= rng.random((n, n)) < 0.2
+    np.fill_diagonal(D, 0.0)
+    np.fill_diagonal(D, 2.0 * np.abs(D).sum(1) + 1.0)
+    rp = np.concatenate([[0], np.cumsum((D != 0).sum(1))]).astype(np.uint32)
+    A = P.CSRMatrix(n, n, rp, np.nonzero(D)[1].astype(np.uint32), D[D != 0])
+    b, x = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    s = gpu.configure("jacobi", maxIter=40, minIter=40, weight=0.8, relTol=0.0, absTol=0.0)
+    s.Setup(gpu.MAT(A))
+    got = x.copy()
+    s.Solve(b, got)
+    for _ in range(40):
+        x = x + (b - D @ x) * (0.8 / np.diag(D))
+    assert np.max(np.abs(got - x)) <= 40 * 35 * 2.3e-16 * max(1.0, np.max(np.abs(x)))
