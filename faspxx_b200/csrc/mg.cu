@@ -76,13 +76,27 @@ __device__ __forceinline__ void rows_of(const CSRView<double>& A, XV xv, OWN own
     }
 }
 
+// Jacobi's weight / diag: one number where the diagonal is one value (the same bits), else the
+// vector. Reading it had been a quarter of a sweep's bytes on a constant stencil.
+struct DiagInv {
+    const double* v;
+    double c;
+    __device__ __forceinline__ double operator[](size_t i) const { return v ? v[i] : c; }
+};
+
+DiagInv diag_inv(const Pcd& p)
+{
+    if (p.A->diagConst) return {nullptr, (1.0 / p.A->diagValue) * p.weight};
+    return {p.dinv, 0.0};
+}
+
 // One Jacobi sweep, xout = xin + dinv .* r with r = b - A xin, or r = b when NormInf(xin) (*in)
 // is below CLOSE_ZERO (MAT.cxx:455-476, Iter.cxx:83-92). TWO: the first two sweeps from
 // x = 0, whose first is dinv .* b, formed where it is gathered; *in is its mark.
 template <int L, bool TWO>
 __global__ void __launch_bounds__(kBlock, 5) k_mg_sweep(CSRView<double> A, const double* __restrict__ b,
                                                      const double* __restrict__ xin,
-                                                     const double* __restrict__ dinv,
+                                                     DiagInv dinv,
                                                      double* __restrict__ xout,
                                                      const double* __restrict__ in, double* out)
 {
@@ -132,7 +146,7 @@ __global__ void __launch_bounds__(kBlock) k_mg_residual(CSRView<double> A,
 
 // The first sweep from x = 0: x = dinv .* b.
 __global__ void __launch_bounds__(kBlock) k_mg_first(uint32_t n, const double* __restrict__ b,
-                                                     const double* __restrict__ dinv,
+                                                     DiagInv dinv,
                                                      double* __restrict__ x, double* out)
 {
     pdl_wait();
@@ -151,7 +165,7 @@ __global__ void __launch_bounds__(kBlock) k_mg_first(uint32_t n, const double* _
 template <int L>
 __global__ void __launch_bounds__(kBlock) k_mg_restrict(CSRView<double> R, const double* __restrict__ r,
                                                         double* __restrict__ bc,
-                                                        const double* __restrict__ dinv, double* out)
+                                                        DiagInv dinv, double* out)
 {
     tiles_first<L>(R);
     pdl_wait();
@@ -397,7 +411,7 @@ static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, 
             double* out = next_slot();
             by_lanes(lanes, [&](auto L) {
                 e = launch_rows(c, A, lanes, k_mg_sweep<decltype(L)::value, true>, b,
-                                (const double*)nullptr, (const double*)p.dinv, cur, in, out);
+                                (const double*)nullptr, diag_inv(p), cur, in, out);
             });
             if (e) return e;
         } else {
@@ -406,7 +420,7 @@ static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, 
             const int g = std::min(c.grid(A.nrow, kBlock),
                                    resident_grid(c, (const void*)k_mg_first, kBlock));
             FB_CUDA(launch_pdl(k_mg_first, dim3((unsigned)g), dim3(kBlock), 0, c.stream, A.nrow, b,
-                               (const double*)p.dinv, cur, out));
+                               diag_inv(p), cur, out));
         }
         in = *end;
     }
@@ -414,7 +428,7 @@ static int smooth(SolverImpl& S, Pcd& p, const double* b, double* x, bool zero, 
         double* out = next_slot();
         by_lanes(lanes, [&](auto L) {
             e = launch_rows(c, A, lanes, k_mg_sweep<decltype(L)::value, false>, b, (const double*)cur,
-                            (const double*)p.dinv, nxt, in, out);
+                            diag_inv(p), nxt, in, out);
         });
         if (e) return e;
         in = out;
@@ -450,7 +464,7 @@ static int cycle(SolverImpl& S, uint32_t l, const double* b, double* x, bool zer
     const int rl = transfer_lanes(R), pl = transfer_lanes(P);
     by_lanes(rl, [&](auto L) {
         e = launch_rows(c, R, rl, k_mg_restrict<decltype(L)::value>, (const double*)r, S.mgB[l],
-                        (const double*)next.dinv, first);
+                        diag_inv(next), first);
     });
     if (e) return e;
     double* coarse = nullptr;
