@@ -22,7 +22,7 @@ static const double kNaN = std::numeric_limits<double>::quiet_NaN();
 // scalar slots of the solver context
 enum {
     SL_T0 = 0, SL_T1, SL_T2, SL_T3, SL_T4, SL_T5, SL_T6, SL_T7,
-    SL_TA0 = 8, SL_TA1, SL_TB, SL_TR, // cg_generic: (z, r) by turns, (ax, p), ||r||
+    SL_TA0 = 8, SL_TA1, SL_TB, // cg_generic: (z, r) by turns, (ax, p)
     SL_XINF = 16,  // NormInf of a residual's x (MAT::Residual shortcut)
     SL_ONE = 17,   // constant 1: disables the shortcut (MAT::Apply + XPAY paths)
     SL_XINF2 = 18, // the fused Jacobi sweeps' second NormInf slot (ping-pong with SL_XINF)
@@ -669,17 +669,18 @@ void SolverImpl::destroy()
 
 // alpha = *tmpa / *tmpb, x += alpha p, r -= alpha ax and ||r|| (CG.cxx:104-133) in one pass,
 // with the operations of v_axpy and v_norm2 one after another; nothing but the norm's slot
-// changes when |*tmpb| <= 1e-40 (the host finishes that branch).
+// changes when |*tmpb| <= 1e-40 (the host finishes that branch). host (page-locked) gets tmpa,
+// tmpb and the norm for the host's tests, without a copy after the kernel.
 __global__ void __launch_bounds__(kBlock) k_cg_step(uint32_t n, const double* __restrict__ tmpa,
                                                     const double* __restrict__ tmpb,
                                                     const double* __restrict__ p,
                                                     const double* __restrict__ ax,
                                                     double* __restrict__ x, double* __restrict__ r,
-                                                    Scratch s, double* dnorm)
+                                                    Scratch s, double* host)
 {
     pdl_wait();
     pdl_release();
-    const double tb = *tmpb, alpha = *tmpa / tb;
+    const double ta = *tmpa, tb = *tmpb, alpha = ta / tb;
     const bool go = fabs(tb) > kCloseZero * kCloseZero;
     double t = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; go && i < n;
@@ -691,7 +692,11 @@ __global__ void __launch_bounds__(kBlock) k_cg_step(uint32_t n, const double* __
     }
     double acc[1] = {t};
     const int ops[1] = {kSum};
-    grid_reduce<1>(acc, ops, s, [=] __device__(const double* v) { *dnorm = sqrt(v[0]); });
+    grid_reduce<1>(acc, ops, s, [=] __device__(const double* v) {
+        host[0] = ta;
+        host[1] = tb;
+        host[2] = sqrt(v[0]);
+    });
 }
 
 int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
@@ -731,13 +736,11 @@ int SolverImpl::cg_generic(const double* b, double* x, fasp_gpu_info* info)
         ++c.launches;
         FB_CUDA(launch_pdl(k_cg_step, dim3((unsigned)c.grid(n, kBlock)), dim3(kBlock), 0, c.stream, n,
                            (const double*)(d + SL_TA0 + turn), (const double*)(d + SL_TB),
-                           (const double*)pk, (const double*)ax, x, rk, c.red, d + SL_TR));
-        FB_CUDA(cudaMemcpyAsync(c.hslot, d + SL_TA0, 4 * sizeof(double), cudaMemcpyDeviceToHost,
-                                c.stream));
+                           (const double*)pk, (const double*)ax, x, rk, c.red, c.hslot));
         FB_CUDA(cudaStreamSynchronize(c.stream));
-        tmpa = c.hslot[turn];
-        tmpb = c.hslot[2];
-        const double rnorm = c.hslot[3];
+        tmpa = c.hslot[0];
+        tmpb = c.hslot[1];
+        const double rnorm = c.hslot[2];
         if (std::fabs(tmpb) > kCloseZero * kCloseZero)
             alpha = tmpa / tmpb;
         else {
