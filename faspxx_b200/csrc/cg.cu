@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 
 #include "cg.cuh"
+#include "plane_walk.cuh"
 
 namespace fb {
 
@@ -873,6 +874,46 @@ __global__ void __launch_bounds__(kBlock, 4)
     });
 }
 
+// cg_spmv (FP64, p formed where it is gathered) on plane walks (plane_walk.cuh): bound by what z
+// and the old p cost from L2, each of which the row kernels read 3.8 times a row, the two-row
+// kernel's registers 2.3 times (19.4 against 21.1 us at 128^3, 19.4 against 25.6 at 127^3).
+template <int JZ>
+__global__ void __launch_bounds__(kBlock)
+    cg_spmv_walk(CSRView<double> A, const double* __restrict__ z, double* P0, double* P1,
+                 double* __restrict__ q, CGCtl* c, Scratch s, PlaneWalk walk)
+{
+    pdl_wait();
+    pdl_release();
+    const int status = c->status;
+    const int mode = c->pmode, par = c->par;
+    const double zc = c->zc, beta = c->beta;
+    if (status != kRun) return;
+    const double* __restrict__ pOld = par ? P1 : P0;
+    double* __restrict__ pNew = par ? P0 : P1;
+    double acc = 0.0;
+    struct Raw {
+        double z, p;
+    };
+    plane_rows<Raw, double>(
+        A, walk, reinterpret_cast<double*>(fb_tile_smem),
+        [&](uint32_t j) { return Raw{z[j], mode ? pOld[j] : 0.0}; },
+        [&](const Raw& v) {
+            const double zi = JZ == 2 ? zc * v.z : v.z;
+            return mode ? fma(beta, v.p, zi) : zi;
+        },
+        [&](size_t row, double pi, double sum) {
+            pNew[row] = pi;
+            q[row] = sum;
+            acc = fma(sum, pi, acc);
+        });
+    double a[1] = {acc};
+    const int ops[1] = {kSum};
+    grid_reduce_ctl<1>(a, ops, s, c, [=] __device__(CGCtl* cs, const double* t) {
+        cs->par = par ^ 1;
+        if (!cs->bench) cg_after_spmv(cs, t[0]);
+    });
+}
+
 template <typename T, int JAC>
 __global__ void __launch_bounds__(kBlock, 4) cg_update(uint32_t n, T* __restrict__ x,
                                                     T* __restrict__ r, T* __restrict__ z,
@@ -1653,6 +1694,20 @@ void CGEngine<T>::launch_spmv_kernel()
                               (V.gnz || al(V.mask, 8))
                         : base && !recurrence && sh != 0 && V.nrow % 2 == 0 && al(P1, 16) &&
                               (V.gnz || al(V.mask, 4));
+    if constexpr (sizeof(T) == 8) {
+        // Where items get planes enough (kWalkChunk), walking them beats the two-row kernel's
+        // registers and the row kernel. A solve: 160^3 33.6 to 27.9 ms, 128^3 12.4 to 11.7, 127^3
+        // 13.8 to 11.8, 126^3 13.4 to 10.9, 101^3 7.6 to 6.8, 95^3 6.5 to 5.6, 85^3 5.0 to 4.8.
+        auto kern = jm == 2 ? cg_spmv_walk<2> : cg_spmv_walk<0>;
+        const WalkLaunch l = A->lanes == 1 && !recurrence
+                                 ? walk_launch(*c, V, (const void*)kern)
+                                 : WalkLaunch();
+        if (l.grid) {
+            launch_overlapped_smem(kern, l.grid, l.smem, c->stream, pdl, V, zz, P0, P1, q, ctl,
+                                   c->red, l.w);
+            return;
+        }
+    }
 #define CG_SPMV_LANES(RR, JJ)                                                              \
     switch (v4 ? 0 : A->lanes) {                                                           \
         case 0:                                                                            \

@@ -12,14 +12,15 @@ namespace fb {
 // sides are formed once, by coalesced loads two planes ahead, and shared; the planes below and
 // above are the thread's own columns, in registers. A row's products are summed in the order of
 // its offsets, as row_apply does (the same bits). Any S1 <= kWalkS1 and S2, aligned or not.
-// FP64 BiCGStab, three vectors and two: 57 to 47 us an iteration at 101^3, 51 to 47 at 100^3 and
-// 168 to 129 at 150^3 (against 16-byte groups). Operands of one vector gain nothing: products
+// FP64 CG: see cg_spmv_walk. FP64 BiCGStab, three vectors and two: 57 to 47 us an iteration at
+// 101^3, 51 to 47 at 100^3 and 168 to 129 at 150^3 (against 16-byte groups). Operands of one vector gain nothing: products
 // at 127^3 14.4 us both ways, at 128^3 14.8 against the 10.3 of 16-byte groups.
 constexpr uint32_t kWalkS1 = kBlock; // 2 S1 edge values a plane, two a thread
 constexpr int kWalkCols = 2;         // columns a thread (1: 50 us at 101^3, 139 at 150^3)
-// Planes an item walks at least; it loads two more. With 4 (90^3) an iteration went from 44 to
-// 40 us, with 3 (80^3) 36.3 to 35.9, with 2 (64^3) 29.3 to 31.3.
-constexpr uint32_t kWalkChunk = 4;
+// Planes an item walks at least; it loads two more. BiCGStab with 4 (90^3) went from 44 to 40 us an
+// iteration, with 3 (80^3) 36.3 to 35.9, with 2 (64^3) 29.3 to 31.3; FP64 CG solves with 3 (95^3,
+// 90^3, 85^3) 6.5 to 5.6, 5.6 to 5.2 and 5.0 to 4.8 ms, with 2 (80^3, 72^3) 4.3 to 4.1 and 3.7 to 3.8.
+constexpr uint32_t kWalkChunk = 3;
 
 struct PlaneWalk {
     uint32_t tiles = 0; // blocks' items: segs column segments x chunks of planes; 0: not in use

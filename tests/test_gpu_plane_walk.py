@@ -1,5 +1,5 @@
-"""FP64 BiCGStab on seven-point stencil masks, whose product kernels walk the planes of the grid
-where an item gets at least four of them: the first iterations against the same solver with two
+"""FP64 CG and BiCGStab on seven-point stencil masks, whose product kernels walk the planes of the grid
+where an item gets at least three of them: the first iterations against the same solver with two
 lanes a row, which gathers from plain CSR.
 
 Both form every row and every sum from the same values; they differ in the order of summation.
@@ -22,8 +22,10 @@ def gpu():
     return sol
 
 
-def _matrix(shape, cut):
+def _matrix(shape, cut, symmetric):
     c = [-1.0, -1.2, -1.4, 10.0, -0.6, -0.8, -1.0]
+    if symmetric:
+        c[4:] = c[2::-1]
     A = P._from_stencil(shape, P._OFF3D, lambda k: c[k])
     n = A.nrow - cut  # the last plane loses its end
     rows = np.repeat(np.arange(A.nrow), np.diff(A.rowPtr.astype(np.int64)))
@@ -33,6 +35,7 @@ def _matrix(shape, cut):
     return P.CSRMatrix(n, n, rp, A.colInd[keep], A.values[keep])
 
 
+@pytest.mark.parametrize("alg", ["bicgstab", "cg"])
 @pytest.mark.parametrize("pcd", [None, "jacobi"])
 @pytest.mark.parametrize("shape,cut", [
     ((7, 43, 1800), 0),     # one column segment, most of it empty
@@ -40,19 +43,20 @@ def _matrix(shape, cut):
     ((7, 43, 1801), 13),    # a ragged last plane
     ((101, 101, 101), 0),   # odd: no 16-byte groups
     ((96, 96, 96), 0),      # aligned
+    ((128, 32, 300), 0),    # aligned, whole warps a plane
     ((256, 20, 220), 5),    # the largest S1
     ((257, 20, 220), 0),    # too wide to walk
     ((64, 90, 20), 0),      # too few planes an item
     ((33, 33, 33), 0)])
-def test_first_iterations(gpu, shape, cut, pcd):
-    A = _matrix(shape, cut)
+def test_first_iterations(gpu, shape, cut, pcd, alg):
+    A = _matrix(shape, cut, alg == "cg")
     rng = np.random.default_rng(A.nrow)
     b, x0 = rng.uniform(-1, 1, A.nrow), rng.uniform(-1, 1, A.nrow)
     got = []
     for lanes in (1, 2):
         M = gpu.MAT(A)
         M.SetLanes(lanes)
-        s = gpu.configure("bicgstab", maxIter=4, relTol=1e-30, absTol=0.0, pcd=pcd,
+        s = gpu.configure(alg, maxIter=4, relTol=1e-30, absTol=0.0, pcd=pcd,
                           pcdWeight=2.0 / 3.0, pcdIter=1)
         s.Setup(M)
         x = x0.copy()
