@@ -16,6 +16,7 @@
 namespace fb {
 
 constexpr int kSlotResidualXinf = kSlots - 1;
+constexpr int kTileLanes = 4; // lanes a row of k_lane_tiles (mean rows of 17 to 32 entries)
 
 // y = A x (RES: r = b - A x, with the x ~ 0 shortcut of MAT::Residual) on stencil masks of
 // the fixed 5- or 7-point shape (SH), W consecutive rows per thread (stencil_group).
@@ -64,11 +65,6 @@ __global__ void __launch_bounds__(kBlock) k_spmv(CSRView<T> A, const T* __restri
         for_rows<T, PAT>(A, [&](uint32_t j) { return x[j]; }, [&](size_t r, T s) { y[r] = s; });
         return;
     }
-    if (A.tiles) { // L threads a row, the entries through shared memory: the same sums
-        csr_tile_rows<T, PAT, L>(A, *reinterpret_cast<TileSmem<T>*>(fb_tile_smem),
-                                 [&](uint32_t j) { return x[j]; }, [&](size_t r, T s) { y[r] = s; });
-        return;
-    }
     const int lane = threadIdx.x & (L - 1);
     const size_t warpRows = 32 / L;
     const size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -108,12 +104,6 @@ __global__ void __launch_bounds__(kBlock) k_residual(CSRView<T> A, const T* __re
         }
         return;
     }
-    if (A.tiles && !shortcut) {
-        csr_tile_rows<T, false, L>(A, *reinterpret_cast<TileSmem<T>*>(fb_tile_smem),
-                                   [&](uint32_t j) { return x[j]; },
-                                   [&](size_t row, T s) { r[row] = b[row] - s; });
-        return;
-    }
     const int lane = threadIdx.x & (L - 1);
     const size_t warpRows = 32 / L;
     const size_t gw = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -129,6 +119,26 @@ __global__ void __launch_bounds__(kBlock) k_residual(CSRView<T> A, const T* __re
         s = group_sum<L>(s);
         if (lane == 0 && row < A.nrow) r[row] = b[row] - s;
     }
+}
+
+// y = A x (RES: r = b - A x, or r = b by the shortcut) with kTileLanes threads a row and the entries
+// through shared memory in block tiles: the sums of the lane kernels. Kernels of their own: as a
+// branch inside k_spmv and k_residual they cost the lane kernels up to 7% where no tile is taken.
+template <bool RES>
+__global__ void __launch_bounds__(kBlock) k_lane_tiles(CSRView<double> A, const double* __restrict__ b,
+                                                       const double* __restrict__ x,
+                                                       double* __restrict__ y,
+                                                       const double* __restrict__ xinf)
+{
+    if (RES && *xinf < kCloseZero) {
+        for (size_t row = (size_t)blockIdx.x * blockDim.x + threadIdx.x; row < A.nrow;
+             row += (size_t)gridDim.x * blockDim.x)
+            y[row] = b[row] - 0.0;
+        return;
+    }
+    csr_tile_rows<double, false, kTileLanes>(
+        A, *reinterpret_cast<TileSmem<double>*>(fb_tile_smem), [&](uint32_t j) { return x[j]; },
+        [&](size_t row, double s) { y[row] = RES ? b[row] - s : s; });
 }
 
 static int spmv_grid(const Ctx& c, uint32_t nrow, int L)
@@ -147,6 +157,33 @@ int lanes_for(double mean)
     int L = 2;
     while (L < 32 && L * 8 < mean) L *= 2;
     return L;
+}
+
+// k_lane_tiles takes FP64 matrices of rows of 20 entries and more on four lanes (64 rows of more
+// than 28 do not fit a stage) whose entries take more than kLaneTileBytes, so that one product and
+// the next (A and its transpose, say) do not find each other's matrix in the 126 MB L2. Measured
+// on B200, lanes and tiles, Apply back to back / Apply, Residual and MultTransposeAdd in turn, us:
+// 571,000 rows of 23 entries 41.3 / 161 and 38.9 / 131; 238,000 of 23 (65 MB) 22.2 / 84 and 20.1 /
+// 69; 230,000 of 20 (55 MB) 28.8 / 103 and 27.6 / 96. Below: 176,000 of 23 (48 MB) 16.9 / 55 and
+// 16.5 / 57; 46,700 of 22 6.3 / 27 and 8.1 / 31; 300,000 of 18 in a band 16.5 and 18.6. More lanes:
+// 30,000 rows of 100 (16 lanes) 16 and 18.7, of 200 (32 lanes) 25 and 33.
+constexpr unsigned long long kLaneTileBytes = 50ull << 20;
+
+template <typename T>
+static bool lane_tiles(Ctx& c, CSRView<T>& A, int L, uint32_t span, const void* kern, size_t* smem,
+                       int* grid)
+{
+    if (sizeof(T) != 8 || L != kTileLanes || !A.val || A.nnz < 20ull * A.nrow ||
+        A.nnz * 12ull < kLaneTileBytes)
+        return false;
+    *smem = with_tiles(A, kBlock, span);
+    if (*smem && tiles_fit(kern, *smem)) {
+        *grid = std::min(ceil_div((long long)A.nrow * kTileLanes, kBlock),
+                         resident_grid(c, kern, kBlock, *smem));
+        return true;
+    }
+    A.tiles = 0;
+    return false;
 }
 
 template <typename T>
@@ -171,7 +208,17 @@ static int launch_spmv(Ctx& c, CSRView<T> A, int L, uint32_t span, const T* x, T
             return kOk;
         }
     }
-    const size_t tiles = with_tiles(A, kBlock, span);
+    if constexpr (std::is_same<T, double>::value) {
+        size_t smem = 0;
+        int g = 0;
+        if (lane_tiles(c, A, L, span, (const void*)k_lane_tiles<false>, &smem, &g)) {
+            ++c.launches;
+            k_lane_tiles<false><<<g, kBlock, smem, c.stream>>>(A, nullptr, x, y, nullptr);
+            FB_CUDA(cudaGetLastError());
+            return kOk;
+        }
+    }
+    const size_t tiles = L == 1 ? with_tiles(A, kBlock, span) : 0;
     auto go = [&](auto kern) {
         CSRView<T> V = A;
         size_t smem = tiles;
@@ -268,7 +315,17 @@ static int residual_t(Ctx& c, const Mat& A, CSRView<T> V, const T* b, const T* x
             return kOk;
         }
     }
-    const size_t tiles = with_tiles(V, kBlock, A.span(A.lanes));
+    if constexpr (std::is_same<T, double>::value) {
+        size_t smem = 0;
+        int g = 0;
+        if (lane_tiles(c, V, A.lanes, A.span(A.lanes), (const void*)k_lane_tiles<true>, &smem, &g)) {
+            ++c.launches;
+            k_lane_tiles<true><<<g, kBlock, smem, c.stream>>>(V, b, x, r, xinf);
+            FB_CUDA(cudaGetLastError());
+            return kOk;
+        }
+    }
+    const size_t tiles = A.lanes == 1 ? with_tiles(V, kBlock) : 0;
     auto go = [&](auto kern) {
         CSRView<T> W = V;
         size_t smem = tiles;
@@ -402,25 +459,31 @@ int m_sampled_outer(Ctx& c, const Mat& A, const double* lam, const double* x, do
 // reference's bit for bit wherever its loop bounds are right (structurally symmetric A).
 // Pattern-only matrices count every stored entry as 1, as MAT::Apply does; a grid operator
 // walks its stencil points in ascending offset, which is its CSR order.
-// Rows of some 8 to 50 entries stream through block tiles of 256 / L rows (csr_tile_rows with
-// separately rounded sums): thread per row straight from global memory reads words 12 len
-// bytes apart. On B200 a 571,000-row matrix of 23 entries a row took 63 us that way and takes
-// 47 us; seven-entry rows took 73 us thread per row (160^3), 76 us through tiles and 105 us
-// with evict-first loads four entries at a time, and keep the plain loop.
-template <bool GRID, bool PAT, int L>
-__global__ void __launch_bounds__(kBlock) k_mult_transpose_add(CSRView<double> T,
-                                                               const double* __restrict__ v1,
-                                                               const double* __restrict__ v2,
-                                                               double* __restrict__ v)
+// Rows of some 20 to 50 entries stream through block tiles of 256 / L rows (csr_tile_rows with
+// separately rounded sums) in a kernel of their own: thread per row straight from global memory
+// reads words 12 len bytes apart. On B200, thread per row and tiles, us back to back: 571,000 rows
+// of 23 entries 64.0 and 48.8, 300,000 of 32 in a band 82.5 and 61.4, 50,000 of 48 39 and 20.7,
+// 46,700 of 22 10.4 and 8.5; with scattered columns 600,000 of 30 133 and 121, 150,000 of 30 34.8
+// and 36.7. Shorter rows keep the plain loop: 300,000 of 18 18.6 and 21.2, 200,000 of 10 8.3 and
+// 10.4, seven entries (160^3) 73 and 76; so do rows whose tiles do not fit a stage on 8 lanes. As
+// a branch in the plain kernel the tiles cost it up to 19% there (5,000 rows of 1,000: 161 and 191).
+template <bool PAT, int L>
+__global__ void __launch_bounds__(kBlock) k_mult_transpose_add_tiles(CSRView<double> T,
+                                                                     const double* __restrict__ v1,
+                                                                     const double* __restrict__ v2,
+                                                                     double* __restrict__ v)
 {
-    if (!GRID && T.tiles) {
-        auto from = [&](size_t i) { return v2[i]; };
-        csr_tile_rows<double, PAT, L>(T, *reinterpret_cast<TileSmem<double>*>(fb_tile_smem),
-                                      [&](uint32_t j) { return v1[j]; },
-                                      [&](size_t i, double s) { v[i] = s; },
-                                      RowSep<decltype(from)>{from});
-        return;
-    }
+    auto from = [&](size_t i) { return v2[i]; };
+    csr_tile_rows<double, PAT, L>(T, *reinterpret_cast<TileSmem<double>*>(fb_tile_smem),
+                                  [&](uint32_t j) { return v1[j]; },
+                                  [&](size_t i, double s) { v[i] = s; },
+                                  RowSep<decltype(from)>{from});
+}
+
+template <bool GRID, bool PAT>
+__global__ void k_mult_transpose_add(CSRView<double> T, const double* __restrict__ v1,
+                                     const double* __restrict__ v2, double* __restrict__ v)
+{
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < T.nrow;
          i += (size_t)gridDim.x * blockDim.x) {
         double acc = v2[i];
@@ -444,31 +507,34 @@ int m_mult_transpose_add(Ctx& c, const Mat& T, const double* v1, const double* v
     if (T.nrow == 0) return kOk;
     CSRView<double> V = T.view<double>(T.val, nullptr);
     V.cd16 = nullptr;
-    // the fewest threads a row whose tiles fit a stage; rows short enough for one (a
-    // 7-point stencil) go straight from global memory
+    auto plain = [&](auto kern) {
+        const int g = std::max(1, std::min(ceil_div(T.nrow, kBlock), c.nsm * 8));
+        kern<<<g, kBlock, 0, c.stream>>>(V, v1, v2, v);
+    };
+    // the fewest threads a row whose tiles fit a stage
     int L = 1;
     while (L < 8 && T.span(L) > TileShape<double>::cap) L *= 2;
-    const size_t tiles = T.grid || L == 1 ? 0 : with_tiles(V, kBlock, T.span(L));
-    if (!tiles) L = 1;
-    auto go = [&](auto kern) {
-        CSRView<double> W = V;
-        size_t smem = tiles;
-        if (smem && !tiles_fit((const void*)kern, smem)) W.tiles = 0, smem = 0;
-        const int g = std::max(1, std::min(ceil_div((long long)T.nrow * L, kBlock),
-                                           resident_grid(c, (const void*)kern, kBlock, smem)));
-        kern<<<g, kBlock, smem, c.stream>>>(W, v1, v2, v);
+    const size_t smem = T.grid || L == 1 || T.nnz < 20ull * T.nrow
+                            ? 0
+                            : with_tiles(V, kBlock, T.span(L));
+    auto tiled = [&](auto kern) {
+        const int g = std::min(ceil_div((long long)T.nrow * L, kBlock),
+                               resident_grid(c, (const void*)kern, kBlock, smem));
+        if (!tiles_fit((const void*)kern, smem)) return false;
+        kern<<<g, kBlock, smem, c.stream>>>(V, v1, v2, v);
+        return true;
     };
     auto by = [&](auto PAT) {
         constexpr bool P = decltype(PAT)::value;
-        switch (L) {
-            case 1: go(k_mult_transpose_add<false, P, 1>); break;
-            case 2: go(k_mult_transpose_add<false, P, 2>); break;
-            case 4: go(k_mult_transpose_add<false, P, 4>); break;
-            default: go(k_mult_transpose_add<false, P, 8>); break;
-        }
+        if (smem && (L == 2   ? tiled(k_mult_transpose_add_tiles<P, 2>)
+                     : L == 4 ? tiled(k_mult_transpose_add_tiles<P, 4>)
+                              : tiled(k_mult_transpose_add_tiles<P, 8>)))
+            return;
+        V.tiles = 0;
+        plain(k_mult_transpose_add<false, P>);
     };
     if (T.grid)
-        go(k_mult_transpose_add<true, false, 1>);
+        plain(k_mult_transpose_add<true, false>);
     else if (!T.val)
         by(std::true_type{});
     else
