@@ -949,7 +949,7 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
 int fasp_gpu_batch_destroy(fasp_gpu_batch h)
 {
     if (!h) return kOk;
-    cudaDeviceSynchronize();
+    device_idle(h->c.dev);
     m_free(h->M);
     for (void* p : {(void*)h->sysRow, (void*)h->order, (void*)h->dinv, (void*)h->dinv32,
                     (void*)h->r64, (void*)h->z64, (void*)h->p0, (void*)h->p1, (void*)h->q64,

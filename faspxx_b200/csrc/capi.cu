@@ -317,7 +317,7 @@ int fasp_gpu_mat_add(double a, fasp_gpu_mat A, double b, fasp_gpu_mat B, fasp_gp
 int fasp_gpu_mat_destroy(fasp_gpu_mat A)
 {
     if (!A) return kOk;
-    cudaDeviceSynchronize(); // whichever streams still use the arrays
+    device_idle(A->c.dev); // whichever streams still use the arrays
     if (A->T) fasp_gpu_mat_destroy(A->T);
     m_free(A->M);
     A->c.destroy();

@@ -96,7 +96,8 @@ constexpr int kSlots = 256;
 // ---- memory (mem.cu) --------------------------------------------------------------------
 // Device memory from the current device's pool, ready for work on s (for other streams after
 // s has been waited for): kErrAlloc. dev_free takes it back at once, so whoever frees has
-// waited for the work that uses it.
+// waited for the work that uses it: a handle that is destroyed for its whole device
+// (device_idle), whichever device the calling thread has current.
 int dev_alloc_bytes(void** p, size_t bytes, cudaStream_t s);
 template <typename T>
 inline int dev_alloc(T** p, size_t bytes, cudaStream_t s)
@@ -104,6 +105,7 @@ inline int dev_alloc(T** p, size_t bytes, cudaStream_t s)
     return dev_alloc_bytes(reinterpret_cast<void**>(p), bytes, s);
 }
 void dev_free(void* p);
+void device_idle(int dev); // waits for all work on dev; the current device stays
 void dev_trim(); // the current device's free pool memory goes back to the device
 // Page-locked host blocks of kPinnedBlock bytes, zeroed; null when there are none.
 constexpr size_t kPinnedBlock = 4096;

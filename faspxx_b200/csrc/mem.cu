@@ -85,6 +85,15 @@ int dev_alloc_bytes(void** p, size_t bytes, cudaStream_t s)
 
 void dev_free(void* p) { cudaFree(p); }
 
+void device_idle(int dev)
+{
+    int cur = dev;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
+    cudaDeviceSynchronize();
+    if (cur != dev) cudaSetDevice(cur);
+}
+
 void* pinned_get()
 {
     {

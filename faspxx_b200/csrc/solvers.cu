@@ -596,7 +596,7 @@ void SolverImpl::clean()
 
 void SolverImpl::destroy()
 {
-    if (A) cudaDeviceSynchronize(); // whatever still runs on what is released below
+    if (A) device_idle(c.dev); // whatever still runs on what is released below
     for (double* p : w) dev_free(p);
     w.clear();
     for (float* p : w32) dev_free(p);

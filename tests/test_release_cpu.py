@@ -1,0 +1,76 @@
+"""Handles give their memory back only when the device they live on has nothing left to do, whatever
+device the destroying thread has current. Pool memory can go to another handle at once, so a
+product enqueued by an asynchronous call must have been waited for by then. On a runtime of two
+devices without GPUs (fakecuda.py)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from faspxx_b200 import problems as P
+from tests import fakecuda
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    return fakecuda.load(tmp_path_factory.mktemp("fake"))
+
+
+
+def _matrix(lib):
+    A, h = P.poisson2d(40), C.c_void_p()
+    assert lib.fasp_gpu_mat_create(A.nrow, A.mcol, A.nnz, A.rowPtr.ctypes.data, A.colInd.ctypes.data,
+                                   A.values.ctypes.data, C.byref(h)) == 0
+    return A, h
+
+
+def _device(lib, a):
+    p = C.c_void_p()
+    assert lib.fasp_gpu_malloc(C.byref(p), a.nbytes + 16) == 0
+    assert lib.fasp_gpu_memcpy_h2d(p, a.ctypes.data, a.nbytes) == 0
+    return p
+
+
+def _product_in_flight(lib, A, h):
+    x, y = _device(lib, np.ones(A.mcol)), _device(lib, np.ones(A.nrow))
+    assert lib.fasp_gpu_mat_apply_async(h, x, y, lib.fake_stream()) == 0
+
+
+@pytest.mark.parametrize("current", [1, 0])  # the device of the handles, and another one
+@pytest.mark.parametrize("kind", ["matrix", "transposed", "solver", "setup again", "batch"])
+def test_destroy_waits_for_the_handles_device(lib, kind, current):
+    from faspxx_b200 import capi
+    assert lib.fasp_gpu_init(1) == 0
+    lib.fasp_gpu_synchronize()
+    A, h = _matrix(lib)
+    early = lib.fake_early_frees()
+    if kind == "transposed":
+        z = _device(lib, np.ones(A.mcol))
+        assert lib.fasp_gpu_mat_mult_transpose_add_async(h, z, z, _device(lib, np.ones(A.mcol)),
+                                                         lib.fake_stream()) == 0
+    if kind in ("solver", "setup again"):
+        cfg = capi.Config()
+        lib.fasp_gpu_default_config(C.byref(cfg), capi.CG)
+        s = C.c_void_p()
+        assert lib.fasp_gpu_solver_create(C.byref(cfg), C.byref(s)) == 0
+        assert lib.fasp_gpu_solver_setup(s, h) == 0
+    if kind == "batch":
+        bt = C.c_void_p()
+        rows = _device(lib, np.array([0, 700, 1600], np.uint32))
+        B = P.CSRMatrix(1600, 1600, np.arange(1601, dtype=np.uint32), np.arange(1600, dtype=np.uint32),
+                        np.ones(1600))
+        d = [_device(lib, a) for a in (B.rowPtr, B.colInd, B.values)]
+        assert lib.fasp_gpu_batch_create(2, rows, B.nnz, *d, 1, C.byref(bt)) == 0
+    assert lib.fake_early_frees() == early
+    _product_in_flight(lib, A, h)
+    lib.fake_use_device(current)
+    if kind == "solver":
+        assert lib.fasp_gpu_solver_destroy(s) == 0
+    elif kind == "setup again":
+        assert lib.fasp_gpu_solver_setup(s, h) == 0
+    elif kind == "batch":
+        assert lib.fasp_gpu_batch_destroy(bt) == 0
+    else:
+        assert lib.fasp_gpu_mat_destroy(h) == 0
+    assert lib.fake_early_frees() == early
+    assert lib.fake_device() == current
