@@ -61,6 +61,7 @@ SIGNATURES = {
     "fasp_gpu_memcpy_d2h": (_i, [_vp, _vp, _sz]),
     "fasp_gpu_memset": (_i, [_vp, _i, _sz]),
     "fasp_gpu_synchronize": (_i, []),
+    "fasp_gpu_trim": (_i, []),
     "fasp_gpu_host_alloc": (_i, [_P(_vp), _sz]),
     "fasp_gpu_host_free": (_i, [_vp]),
     "fasp_gpu_mat_create": (_i, [_u32, _u32, _u32, _vp, _vp, _vp, _P(_vp)]),

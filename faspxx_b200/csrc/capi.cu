@@ -174,7 +174,9 @@ int fasp_gpu_malloc(void** p, size_t bytes)
 {
     if (cudaMalloc(p, bytes) != cudaSuccess) {
         cudaGetLastError();
-        dev_trim(); // what the pool keeps may be what is missing
+        int dev = 0;
+        cudaGetDevice(&dev);
+        dev_trim(dev); // what the pool keeps may be what is missing
         if (cudaMalloc(p, bytes) != cudaSuccess) {
             cudaGetLastError();
             *p = nullptr;
@@ -221,6 +223,11 @@ int fasp_gpu_synchronize(void)
 {
     FB_CUDA(cudaDeviceSynchronize());
     return kOk;
+}
+
+int fasp_gpu_trim(void)
+{
+    return dev_trim(g_device);
 }
 
 int fasp_gpu_host_alloc(void** p, size_t bytes)

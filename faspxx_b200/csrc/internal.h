@@ -106,7 +106,7 @@ inline int dev_alloc(T** p, size_t bytes, cudaStream_t s)
 }
 void dev_free(void* p);
 void device_idle(int dev); // waits for all work on dev; the current device stays
-void dev_trim(); // the current device's free pool memory goes back to the device
+int  dev_trim(int dev); // waits for dev; its free pool memory goes back to the device
 // Page-locked host blocks of kPinnedBlock bytes, zeroed; null when there are none.
 constexpr size_t kPinnedBlock = 4096;
 void* pinned_get();

@@ -17,7 +17,8 @@ namespace {
 
 constexpr int kMaxDev = 64;
 // Free memory that a device's pool keeps: about 2% of the card. The rest goes back to the
-// device at the next synchronisation, and all of it when an allocation fails.
+// device at the next synchronisation, and all of it when an allocation of the library fails or the
+// program asks for it (fasp_gpu_trim): other allocators of the process do not see it.
 constexpr unsigned long long kPoolKeeps = 4ull << 30;
 
 struct Pool {
@@ -54,16 +55,48 @@ constexpr size_t kIdleCtx = 32, kIdlePinned = 64;
 std::vector<Ctx> g_ctx;
 std::vector<void*> g_pinned;
 
+// What a context that nothing uses any more holds.
+void release(Ctx& c)
+{
+    for (cudaEvent_t& ev : c.joinEv)
+        if (ev) cudaEventDestroy(ev);
+    dev_free(c.red.partials);
+    dev_free(c.red.ticket);
+    dev_free(c.dslot);
+    pinned_put(c.hslot);
+    if (c.ownStream && c.stream) cudaStreamDestroy(c.stream);
+    c = Ctx();
+}
+
 } // namespace
 
-void dev_trim()
+void device_idle(int dev)
 {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= kMaxDev) return;
+    int cur = dev;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
     cudaDeviceSynchronize();
-    if (g_pool[dev].pool) cudaMemPoolTrimTo(g_pool[dev].pool, 0);
+    if (cur != dev) cudaSetDevice(cur);
+}
+
+int dev_trim(int dev)
+{
+    if (dev < 0 || dev >= kMaxDev) return kErrNoDevice;
+    device_idle(dev);
+    Ctx gone[kIdleCtx]; // their scratch would hold on to whole pieces of the pool
+    size_t n = 0;
+    {
+        std::lock_guard<std::mutex> hold(g_lock);
+        for (size_t k = g_ctx.size(); k-- > 0;)
+            if (g_ctx[k].dev == dev) {
+                gone[n++] = g_ctx[k];
+                g_ctx.erase(g_ctx.begin() + (ptrdiff_t)k);
+            }
+    }
+    while (n > 0) release(gone[--n]);
+    if (!g_pool[dev].pool || cudaMemPoolTrimTo(g_pool[dev].pool, 0) == cudaSuccess) return kOk;
     cudaGetLastError();
+    return kErrCuda;
 }
 
 int dev_alloc_bytes(void** p, size_t bytes, cudaStream_t s)
@@ -78,21 +111,12 @@ int dev_alloc_bytes(void** p, size_t bytes, cudaStream_t s)
         if (e == cudaSuccess) return kOk;
         cudaGetLastError();
         *p = nullptr;
-        if (attempt == 0) dev_trim();
+        if (attempt == 0) dev_trim(dev);
     }
     return kErrAlloc;
 }
 
 void dev_free(void* p) { cudaFree(p); }
-
-void device_idle(int dev)
-{
-    int cur = dev;
-    cudaGetDevice(&cur);
-    if (cur != dev) cudaSetDevice(dev);
-    cudaDeviceSynchronize();
-    if (cur != dev) cudaSetDevice(cur);
-}
 
 void* pinned_get()
 {
@@ -177,14 +201,7 @@ void Ctx::destroy()
             return;
         }
     }
-    for (cudaEvent_t& ev : joinEv)
-        if (ev) cudaEventDestroy(ev);
-    dev_free(red.partials);
-    dev_free(red.ticket);
-    dev_free(dslot);
-    pinned_put(hslot);
-    if (ownStream && stream) cudaStreamDestroy(stream);
-    *this = Ctx();
+    release(*this);
 }
 
 } // namespace fb

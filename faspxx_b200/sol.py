@@ -283,6 +283,13 @@ def tile_timeouts() -> int:
     return c.value
 
 
+def trim() -> None:
+    """Gives the library's idle device memory (up to 4 GiB kept for the next handles) back to the
+    device, for other allocators of the process such as torch's."""
+    capi.init()
+    check(lib.fasp_gpu_trim(), "trim")
+
+
 def _count(a) -> int:
     return int(a.n) if hasattr(a, "ptr") else len(a)
 

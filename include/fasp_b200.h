@@ -149,6 +149,13 @@ int fasp_gpu_memcpy_h2d(void* dst, const void* src, size_t bytes);
 int fasp_gpu_memcpy_d2h(void* dst, const void* src, size_t bytes);
 int fasp_gpu_memset(void* dptr, int value, size_t bytes); /* every byte set to value */
 int fasp_gpu_synchronize(void);
+/* Gives the library's idle memory back to the device. Matrices, solvers and batches take their
+ * memory from a pool of the library, which keeps up to 4 GiB of what destroyed handles released
+ * for the next ones (and the contexts of up to 32 of them); other allocators of the process
+ * (torch's, say) cannot use it. The library calls this itself when an allocation of its own
+ * fails; a program does when it is done with its handles, or before a large allocation
+ * elsewhere. Waits for the device. */
+int fasp_gpu_trim(void);
 int fasp_gpu_host_alloc(void** hptr, size_t bytes); /* page-locked host memory */
 int fasp_gpu_host_free(void* hptr);
 
