@@ -691,6 +691,8 @@ namespace {
 // Right-hand sides a resident kernel is built for: 1, 2 or 4 (3 run as 4, the last one zero).
 inline uint32_t res_rhs(uint32_t nrhs) { return nrhs <= 2 ? nrhs : 4; }
 
+constexpr int kNoRoom = 1; // launch_resident: the device holds no cluster of that size
+
 template <typename T, int NR, int TH, bool REL>
 int launch_resident(fasp_gpu_batch_s& B, const ResArgs<T>& a, int cluster, bool follow)
 {
@@ -714,7 +716,8 @@ int launch_resident(fasp_gpu_batch_s& B, const ResArgs<T>& a, int cluster, bool 
     cfg.numAttrs = 1;
     int resident = 0;
     FB_CUDA(cudaOccupancyMaxActiveClusters(&resident, (const void*)kern, &cfg));
-    cfg.gridDim = dim3((unsigned)(cluster * std::max(1, std::min(resident, (int)a.items))));
+    if (resident < 1) return kNoRoom;
+    cfg.gridDim = dim3((unsigned)(cluster * std::min(resident, (int)a.items)));
     cfg.numAttrs = follow ? 2 : 1;
     FB_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     B.c.launches += 1;
@@ -732,9 +735,11 @@ int launch_class(fasp_gpu_batch_s& B, const ResArgs<T>& a, const ResClass& k, bo
 }
 
 // Every class of the resident systems, largest first; the classes follow one another
-// programmatically, so a class's blocks move in as the previous one's leave.
-template <typename T, bool REL>
-int run_resident(fasp_gpu_batch_s& B, ResArgs<T> a)
+// programmatically, so a class's blocks move in as the previous one's leave. A class whose
+// clusters have no room (a process limited to some of the SMs) is solved by
+// plain(first, items, queue), in global memory.
+template <typename T, bool REL, typename Plain>
+int run_resident(fasp_gpu_batch_s& B, ResArgs<T> a, Plain plain)
 {
     const uint32_t* cls = B.cls;
     cudaMemsetAsync(B.queue, 0, sizeof(unsigned) * (kResClasses + 1), B.c.stream);
@@ -751,9 +756,82 @@ int run_resident(fasp_gpu_batch_s& B, ResArgs<T> a)
             case 2: e = launch_class<T, 2, REL>(B, a, kRes[k], follow); break;
             default: e = launch_class<T, 4, REL>(B, a, kRes[k], follow); break;
         }
+        if (e == kNoRoom) e = plain(a.first, a.items, a.queue);
         if (e) return e;
         follow = true;
     }
+    return kOk;
+}
+
+// The vectors of batch_pcg and batch_pcg_rel beyond those of every batch.
+int plain_vectors(fasp_gpu_batch_s& B)
+{
+    if (B.z64) return kOk;
+    const size_t vN = (size_t)B.nrhs * B.M.nrow;
+    int e = kOk;
+    auto get = [&](auto** p, size_t bytes) {
+        if (!e && !*p) e = dev_alloc_bytes((void**)p, bytes + 16, B.c.stream);
+    };
+    get(&B.p0, vN * 8);
+    get(&B.p1, vN * 8);
+    get(&B.q64, vN * 8);
+    get(&B.r32, vN * 4);
+    get(&B.z32, vN * 4);
+    get(&B.p032, vN * 4);
+    get(&B.p132, vN * 4);
+    get(&B.q32, vN * 4);
+    if (!e) e = B.M.ensure32(B.c.stream);
+    get(&B.z64, vN * 8); // last: the sign that all are there
+    return e;
+}
+
+// The systems order[first .. first + items) by batch_pcg.
+template <typename T>
+int launch_plain(fasp_gpu_batch_s& B, BatchArgs<T> a, uint32_t first, uint32_t items, unsigned* queue)
+{
+    int e = plain_vectors(B);
+    if (e) return e;
+    if constexpr (sizeof(T) == 8) {
+        a.z = B.z64, a.p0 = B.p0, a.p1 = B.p1, a.q = B.q64, a.val = B.M.val;
+    } else {
+        a.r = B.r32, a.z = B.z32, a.p0 = B.p032, a.p1 = B.p132, a.q = B.q32, a.val = B.M.val32;
+    }
+    a.order = B.order + first;
+    a.count = items;
+    a.queue = queue;
+    const int grid = B.c.nsm * B.blocksPerSM;
+    cudaMemsetAsync(queue, 0, sizeof(unsigned), B.c.stream);
+    switch (B.nrhs) {
+        case 1: batch_pcg<T, 1><<<grid, B.block, 0, B.c.stream>>>(a); break;
+        case 2: batch_pcg<T, 2><<<grid, B.block, 0, B.c.stream>>>(a); break;
+        case 3: batch_pcg<T, 3><<<grid, B.block, 0, B.c.stream>>>(a); break;
+        default: batch_pcg<T, 4><<<grid, B.block, 0, B.c.stream>>>(a); break;
+    }
+    B.c.launches += 1;
+    FB_CUDA(cudaGetLastError());
+    return kOk;
+}
+
+// ... by batch_pcg_rel.
+int launch_plain_rel(fasp_gpu_batch_s& B, BatchArgs<float> a, const BatchRel& f, uint32_t first,
+                     uint32_t items, unsigned* queue)
+{
+    int e = plain_vectors(B);
+    if (e) return e;
+    a.r = B.r32, a.z = B.z32, a.p0 = B.p032, a.p1 = B.p132, a.q = B.q32, a.val = B.M.val32;
+    a.order = B.order + first;
+    a.count = items;
+    a.queue = queue;
+    const int grid = B.c.nsm * B.blocksPerSM;
+    cudaMemsetAsync(queue, 0, sizeof(unsigned), B.c.stream);
+    switch (B.nrhs) {
+        case 1: batch_pcg_rel<1><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+        case 2: batch_pcg_rel<2><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+        case 3: batch_pcg_rel<3><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+        default: batch_pcg_rel<4><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
+    }
+    B.c.launches += 1;
+    FB_CUDA(cudaGetLastError());
     return kOk;
 }
 
@@ -769,26 +847,20 @@ ResArgs<T> res_args(fasp_gpu_batch_s& B, const T* val, const T* dinv, const T* b
 template <typename T>
 int launch_batch(fasp_gpu_batch_s& B, BatchArgs<T> a)
 {
+    auto plain = [&](uint32_t first, uint32_t items, unsigned* queue) {
+        return launch_plain<T>(B, a, first, items, queue);
+    };
     if (B.far < B.count) {
         int e;
         if constexpr (sizeof(T) == 8)
-            e = run_resident<T, false>(B, res_args<T>(B, B.sval, B.dinv, a.b, a.x, a.relTol, a.maxIter));
+            e = run_resident<T, false>(
+                B, res_args<T>(B, B.sval, B.dinv, a.b, a.x, a.relTol, a.maxIter), plain);
         else
-            e = run_resident<T, false>(B, res_args<T>(B, B.sval32, B.dinv32, a.b, a.x, a.relTol, a.maxIter));
+            e = run_resident<T, false>(
+                B, res_args<T>(B, B.sval32, B.dinv32, a.b, a.x, a.relTol, a.maxIter), plain);
         if (e) return e;
     }
-    a.count = B.far;
-    if (a.count == 0) return kOk;
-    const int grid = B.c.nsm * B.blocksPerSM;
-    cudaMemsetAsync(B.queue, 0, sizeof(unsigned), B.c.stream);
-    switch (B.nrhs) {
-        case 1: batch_pcg<T, 1><<<grid, B.block, 0, B.c.stream>>>(a); break;
-        case 2: batch_pcg<T, 2><<<grid, B.block, 0, B.c.stream>>>(a); break;
-        case 3: batch_pcg<T, 3><<<grid, B.block, 0, B.c.stream>>>(a); break;
-        default: batch_pcg<T, 4><<<grid, B.block, 0, B.c.stream>>>(a); break;
-    }
-    B.c.launches += 1;
-    return cudaGetLastError() == cudaSuccess ? kOk : kErrCuda;
+    return B.far ? plain(0, B.far, B.queue + kResClasses) : kOk;
 }
 
 // Sorts the systems (ord, longest first) into the resident kernels' classes and builds the
@@ -921,18 +993,7 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
     dm((void**)&h->r64, vN * 8);
     dm((void**)&h->b32, vN * 4);
     dm((void**)&h->x32, vN * 4);
-    if (h->far) {
-        dm((void**)&h->z64, vN * 8);
-        dm((void**)&h->p0, vN * 8);
-        dm((void**)&h->p1, vN * 8);
-        dm((void**)&h->q64, vN * 8);
-        dm((void**)&h->r32, vN * 4);
-        dm((void**)&h->z32, vN * 4);
-        dm((void**)&h->p032, vN * 4);
-        dm((void**)&h->p132, vN * 4);
-        dm((void**)&h->q32, vN * 4);
-        if (!e) e = h->M.ensure32(h->c.stream);
-    }
+    if (!e && h->far) e = plain_vectors(*h);
     if (!e) {
         batch_dinv<<<std::max(1, std::min(ceil_div(N, 256), 148 * 8)), 256, 0, h->c.stream>>>(
             N, h->M.diag, h->dinv, h->dinv32);
@@ -999,26 +1060,18 @@ int fasp_gpu_batch_solve(fasp_gpu_batch h, const double* b, double* x, double re
                            B.dinv32, nullptr, B.x32, B.r32, B.z32, B.p032, B.p132, B.q32,
                            B.iters, B.resRel, relTol, maxIter, B.queue};
         const BatchRel f{B.M.val, b, x, innerRelTol > 0 && innerRelTol < 1 ? innerRelTol : 1e-2};
+        auto plain = [&](uint32_t first, uint32_t items, unsigned* queue) {
+            return launch_plain_rel(B, a, f, first, items, queue);
+        };
         if (B.far < cnt) {
             ResArgs<float> r = res_args<float>(B, B.sval32, B.dinv32, nullptr, nullptr, relTol, maxIter);
             r.val64 = B.sval;
             r.b64 = b;
             r.x64 = x;
             r.delta = f.delta;
-            e = run_resident<float, true>(B, r);
+            e = run_resident<float, true>(B, r, plain);
         }
-        a.count = B.far;
-        if (!e && a.count) {
-            const int grid = B.c.nsm * B.blocksPerSM;
-            cudaMemsetAsync(B.queue, 0, sizeof(unsigned), B.c.stream);
-            switch (nr) {
-                case 1: batch_pcg_rel<1><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
-                case 2: batch_pcg_rel<2><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
-                case 3: batch_pcg_rel<3><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
-                default: batch_pcg_rel<4><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
-            }
-            B.c.launches += 1;
-        }
+        if (!e && B.far) e = plain(0, B.far, B.queue + kResClasses);
         if (cudaGetLastError() != cudaSuccess) e = kErrCuda;
     } else {
         // FP64 refinement around FP32 inner solves, x0 = 0

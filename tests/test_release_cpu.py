@@ -74,3 +74,33 @@ def test_destroy_waits_for_the_handles_device(lib, kind, current):
         assert lib.fasp_gpu_mat_destroy(h) == 0
     assert lib.fake_early_frees() == early
     assert lib.fake_device() == current
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED", "MIXED_RELIABLE"])
+def test_batch_without_room_for_clusters(lib, precision):
+    """A device that holds no cluster of the resident kernels (a process limited to some SMs) solves
+    the batch in global memory, as devices did before there were clusters; with room it does not."""
+    from faspxx_b200 import capi
+    assert lib.fasp_gpu_init(1) == 0
+    n = 1600
+    rows = _device(lib, np.array([0, 700, n], np.uint32))
+    d = [_device(lib, a) for a in (np.arange(n + 1, dtype=np.uint32), np.arange(n, dtype=np.uint32),
+                                   np.ones(n))]
+    b, x = _device(lib, np.ones(n)), _device(lib, np.ones(n))
+    bt = C.c_void_p()
+    assert lib.fasp_gpu_batch_create(2, rows, n, *d, 1, C.byref(bt)) == 0
+    try:
+        for clusters in (16, 0, 16):
+            lib.fake_set_clusters(clusters)
+            lib.fake_clear_launches()
+            refused = lib.fake_refused()
+            # the fake device computes nothing; a refined solve stops at its first residual, 0
+            code = lib.fasp_gpu_batch_solve(bt, b, x, 1e-8, 10, getattr(capi, precision), 1e-2,
+                                            None, None)
+            assert code == 0 and lib.fake_refused() == refused
+            if precision != "MIXED":
+                plain, resident = lib.fake_launches(b"batch_pcg"), lib.fake_launches(b"batch_resident")
+                assert (plain, resident) == ((0, 1) if clusters else (1, 0))
+    finally:
+        lib.fake_set_clusters(16)
+    assert lib.fasp_gpu_batch_destroy(bt) == 0
