@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(512, 2) batch_pcg(BatchArgs<T> a)
 {
     __shared__ unsigned item;
     __shared__ double sh[3 * kMaxRhs];
+    pdl_release(); // the resident kernels may move in beside it
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) item = atomicAdd(a.queue, 1u);
@@ -240,6 +241,7 @@ __global__ void __launch_bounds__(512) batch_pcg_rel(BatchArgs<float> a, BatchRe
     __shared__ unsigned item;
     __shared__ double sh[3 * kMaxRhs];
     __shared__ int nact, refresh;
+    pdl_release();
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) item = atomicAdd(a.queue, 1u);
@@ -734,17 +736,25 @@ int launch_class(fasp_gpu_batch_s& B, const ResArgs<T>& a, const ResClass& k, bo
     }
 }
 
-// Every class of the resident systems, largest first; the classes follow one another
-// programmatically, so a class's blocks move in as the previous one's leave. A class whose
-// clusters have no room (a process limited to some of the SMs) is solved by
-// plain(first, items, queue), in global memory.
+// Every system: those too large for a cluster first, by plain(first, items, queue), then the
+// classes, largest first. They follow one another programmatically, so a class's blocks move in
+// beside the large systems and as the previous class's leave: a large system keeps one block for
+// the whole of its solve. On B200, 20 systems each of 400^2, 256^2, 33^2, 20^2 and 16^2 rows with four
+// right-hand sides, FP64: 247 ms with the large ones last, 194 first
+// (217 with every system in one queue, before there were clusters). A class whose
+// clusters have no room (a process limited to some of the SMs) is solved by plain, too.
 template <typename T, bool REL, typename Plain>
 int run_resident(fasp_gpu_batch_s& B, ResArgs<T> a, Plain plain)
 {
     const uint32_t* cls = B.cls;
-    cudaMemsetAsync(B.queue, 0, sizeof(unsigned) * (kResClasses + 1), B.c.stream);
     unsigned* const queue = B.queue;
+    FB_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned) * (kResClasses + 1), B.c.stream));
     bool follow = false;
+    if (B.far) {
+        const int e = plain(0, B.far, queue + kResClasses);
+        if (e) return e;
+        follow = true;
+    }
     for (int k = 0; k < kResClasses; ++k) {
         if (cls[k] == cls[k + 1]) continue;
         a.first = cls[k];
@@ -785,6 +795,15 @@ int plain_vectors(fasp_gpu_batch_s& B)
     return e;
 }
 
+// Blocks on the queue: one an SM for few systems (64 of 300^2 rows: 132 ms on the full grid, where
+// some SMs take several, 106 this way), and never fewer than SMs, so that the SMs nearest to the
+// queue take them (one of 500^2: 47.5 ms, 49.4 with a grid of one block).
+int plain_grid(const fasp_gpu_batch_s& B, uint32_t items)
+{
+    const uint32_t most = (uint32_t)(B.c.nsm * B.blocksPerSM);
+    return (int)std::min(most, std::max(items, (uint32_t)B.c.nsm));
+}
+
 // The systems order[first .. first + items) by batch_pcg.
 template <typename T>
 int launch_plain(fasp_gpu_batch_s& B, BatchArgs<T> a, uint32_t first, uint32_t items, unsigned* queue)
@@ -799,8 +818,7 @@ int launch_plain(fasp_gpu_batch_s& B, BatchArgs<T> a, uint32_t first, uint32_t i
     a.order = B.order + first;
     a.count = items;
     a.queue = queue;
-    const int grid = B.c.nsm * B.blocksPerSM;
-    cudaMemsetAsync(queue, 0, sizeof(unsigned), B.c.stream);
+    const int grid = plain_grid(B, items);
     switch (B.nrhs) {
         case 1: batch_pcg<T, 1><<<grid, B.block, 0, B.c.stream>>>(a); break;
         case 2: batch_pcg<T, 2><<<grid, B.block, 0, B.c.stream>>>(a); break;
@@ -822,8 +840,7 @@ int launch_plain_rel(fasp_gpu_batch_s& B, BatchArgs<float> a, const BatchRel& f,
     a.order = B.order + first;
     a.count = items;
     a.queue = queue;
-    const int grid = B.c.nsm * B.blocksPerSM;
-    cudaMemsetAsync(queue, 0, sizeof(unsigned), B.c.stream);
+    const int grid = plain_grid(B, items);
     switch (B.nrhs) {
         case 1: batch_pcg_rel<1><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
         case 2: batch_pcg_rel<2><<<grid, B.block, 0, B.c.stream>>>(a, f); break;
@@ -850,17 +867,12 @@ int launch_batch(fasp_gpu_batch_s& B, BatchArgs<T> a)
     auto plain = [&](uint32_t first, uint32_t items, unsigned* queue) {
         return launch_plain<T>(B, a, first, items, queue);
     };
-    if (B.far < B.count) {
-        int e;
-        if constexpr (sizeof(T) == 8)
-            e = run_resident<T, false>(
-                B, res_args<T>(B, B.sval, B.dinv, a.b, a.x, a.relTol, a.maxIter), plain);
-        else
-            e = run_resident<T, false>(
-                B, res_args<T>(B, B.sval32, B.dinv32, a.b, a.x, a.relTol, a.maxIter), plain);
-        if (e) return e;
-    }
-    return B.far ? plain(0, B.far, B.queue + kResClasses) : kOk;
+    if constexpr (sizeof(T) == 8)
+        return run_resident<T, false>(
+            B, res_args<T>(B, B.sval, B.dinv, a.b, a.x, a.relTol, a.maxIter), plain);
+    else
+        return run_resident<T, false>(
+            B, res_args<T>(B, B.sval32, B.dinv32, a.b, a.x, a.relTol, a.maxIter), plain);
 }
 
 // Sorts the systems (ord, longest first) into the resident kernels' classes and builds the
@@ -1063,15 +1075,12 @@ int fasp_gpu_batch_solve(fasp_gpu_batch h, const double* b, double* x, double re
         auto plain = [&](uint32_t first, uint32_t items, unsigned* queue) {
             return launch_plain_rel(B, a, f, first, items, queue);
         };
-        if (B.far < cnt) {
-            ResArgs<float> r = res_args<float>(B, B.sval32, B.dinv32, nullptr, nullptr, relTol, maxIter);
-            r.val64 = B.sval;
-            r.b64 = b;
-            r.x64 = x;
-            r.delta = f.delta;
-            e = run_resident<float, true>(B, r, plain);
-        }
-        if (!e && B.far) e = plain(0, B.far, B.queue + kResClasses);
+        ResArgs<float> r = res_args<float>(B, B.sval32, B.dinv32, nullptr, nullptr, relTol, maxIter);
+        r.val64 = B.sval;
+        r.b64 = b;
+        r.x64 = x;
+        r.delta = f.delta;
+        e = run_resident<float, true>(B, r, plain);
         if (cudaGetLastError() != cudaSuccess) e = kErrCuda;
     } else {
         // FP64 refinement around FP32 inner solves, x0 = 0
