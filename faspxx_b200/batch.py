@@ -1,9 +1,9 @@
 """Batched Jacobi-PCG over many independent systems (fasp_gpu_batch_* in the C ABI).
 
 ``Batch`` uploads the systems as one block-diagonal CSRx matrix, picks the thread-block
-shape of the persistent launch by timing the candidates on the actual batch (the
-autotuner), and solves all systems and right-hand sides in one launch (FP64, or FP32 inner
-iterations inside FP64 refinement).
+shape of the launch that solves its large systems by timing the candidates on the actual batch
+(the autotuner; small systems run on chip and need none), and solves all systems and right-hand
+sides together (FP64, or FP32 inner iterations inside FP64 refinement).
 """
 from __future__ import annotations
 
@@ -94,10 +94,13 @@ class Batch:
         return x, it.reshape(self.count, self.nrhs), rr.reshape(self.count, self.nrhs), ms.value
 
     def autotune(self, b, precision=capi.FP64, relTol=1e-8, reps=1):
-        """Time each block shape on this batch and keep the fastest."""
+        """Time each block shape on this batch and keep the fastest. Systems solved on chip do not
+        depend on it: a batch of them only is timed as it is."""
         db = _Dev(np.ascontiguousarray(b, dtype=np.float64))
+        large = C.c_uint32()
+        check(lib.fasp_gpu_batch_info(self.h, C.byref(large)), "batch_info")
         best, best_ms = self.shape, float("inf")
-        for shape in SHAPES:
+        for shape in SHAPES if large.value else [self.shape]:
             self.set_shape(*shape)
             t = min(self.solve(db, relTol=relTol, precision=precision)[3] for _ in range(reps))
             if t < best_ms:

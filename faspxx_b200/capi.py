@@ -125,6 +125,7 @@ SIGNATURES = {
     "fasp_gpu_solver_solve_adjoint": (_i, [_vp, _vp, _vp, _P(Info)]),
     "fasp_gpu_solver_solve_adjoint_async": (_i, [_vp, _vp, _vp, _P(Info), _vp]),
     "fasp_gpu_batch_create": (_i, [_u32, _vp, _u32, _vp, _vp, _vp, _u32, _P(_vp)]),
+    "fasp_gpu_batch_info": (_i, [_vp, _P(_u32)]),
     "fasp_gpu_batch_set_shape": (_i, [_vp, _i, _i]),
     "fasp_gpu_batch_solve": (_i, [_vp, _vp, _vp, _d, _u32, _i, _d, _vp, _vp]),
     "fasp_gpu_batch_solve_async": (_i, [_vp, _vp, _vp, _d, _u32, _i, _d, _vp, _vp, _vp]),

@@ -1037,6 +1037,13 @@ int fasp_gpu_batch_destroy(fasp_gpu_batch h)
     return kOk;
 }
 
+int fasp_gpu_batch_info(fasp_gpu_batch h, uint32_t* large)
+{
+    if (!h || !large) return kErrInputPar;
+    *large = h->far;
+    return kOk;
+}
+
 int fasp_gpu_batch_set_shape(fasp_gpu_batch h, int block, int blocksPerSM)
 {
     if (!h || (block != 128 && block != 256 && block != 512) || blocksPerSM < 1 ||

@@ -420,6 +420,9 @@ typedef struct fasp_gpu_batch_s* fasp_gpu_batch;
 int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
                           const uint32_t* rowPtr, const uint32_t* colInd,
                           const double* values, uint32_t nrhs, fasp_gpu_batch* out);
+/* The number of systems that are too large for the on-chip kernels: the ones whose speed
+ * fasp_gpu_batch_set_shape can change. */
+int fasp_gpu_batch_info(fasp_gpu_batch bt, uint32_t* large);
 /* Thread-block shape of the persistent launch that solves the systems too large for the
  * on-chip kernels (more than 65,536 rows x right-hand sides): block (128, 256 or 512 threads)
  * and blocks per SM; the autotuner in the Python/C++ layers times the choices. The on-chip
