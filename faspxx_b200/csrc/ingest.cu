@@ -59,30 +59,56 @@ __global__ void k_count_coo(uint32_t nnz, uint32_t nrow, uint32_t mcol,
 }
 
 // Row pointers start at 0, or at 1 for 1-based files (ReadCSR shifts those,
-// ReadData.cxx:350-353); monotone; rowPtr[nrow] - rowPtr[0] == nnz; shifted columns < mcol.
-__global__ void k_count_csr(uint32_t nrow, uint32_t mcol, uint32_t nnz,
+// ReadData.cxx:350-353); monotone; rowPtr[nrow] - rowPtr[0] == nnz; shifted columns < mcol. Rows of
+// up to kCountLong entries a thread each, longer ones the whole block (a row of 8,000,000 on one
+// thread took 170 ms).
+constexpr uint32_t kCountLong = 128;
+
+__global__ void __launch_bounds__(kBlock) k_count_csr(uint32_t nrow, uint32_t mcol, uint32_t nnz,
                             const uint32_t* __restrict__ rowPtr, const uint32_t* __restrict__ colInd,
                             uint32_t* __restrict__ cnt, uint8_t* __restrict__ has,
                             Counted* __restrict__ out)
 {
+    __shared__ uint32_t lrow[kBlock], nlong;
     const uint32_t base = rowPtr[0];
-    const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool bad = base > 1u || rowPtr[nrow] - base != nnz || rowPtr[nrow] < base;
-    for (size_t i = tid; i < nrow && base <= 1u; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t b = rowPtr[i] - base, e = rowPtr[i + 1] - base;
-        cnt[i] = 0;
-        if (b > e || e > nnz) { // not CSR: its entries are not looked at
-            bad = true;
-            continue;
+    for (size_t i0 = (size_t)blockIdx.x * kBlock; i0 < nrow && base <= 1u;
+         i0 += (size_t)gridDim.x * kBlock) {
+        const size_t i = i0 + threadIdx.x;
+        if (threadIdx.x == 0) nlong = 0;
+        __syncthreads();
+        uint32_t b = 0, e = 0;
+        if (i < nrow) {
+            b = rowPtr[i] - base;
+            e = rowPtr[i + 1] - base;
+            if (b > e || e > nnz) { // not CSR: its entries are not looked at
+                bad = true;
+                e = b;
+            }
+            cnt[i] = e - b;
         }
-        bool diag = false;
-        for (uint32_t k = b; k < e; ++k) {
-            const uint32_t c = colInd[k] - base; // a 0 in a 1-based file wraps and fails too
-            bad = bad || c >= mcol;
-            diag = diag || c == i;
+        if (e - b > kCountLong) {
+            lrow[atomicAdd(&nlong, 1u)] = (uint32_t)i;
+        } else if (i < nrow) {
+            bool diag = false;
+            for (uint32_t k = b; k < e; ++k) {
+                const uint32_t c = colInd[k] - base; // a 0 in a 1-based file wraps and fails too
+                bad = bad || c >= mcol;
+                diag = diag || c == i;
+            }
+            has[i] = diag ? 1 : 0;
         }
-        cnt[i] = e - b;
-        has[i] = diag ? 1 : 0;
+        __syncthreads();
+        for (uint32_t l = 0; l < nlong; ++l) {
+            const uint32_t r = lrow[l], rb = rowPtr[r] - base, re = rowPtr[(size_t)r + 1] - base;
+#pragma unroll 4
+            for (size_t k = (size_t)rb + threadIdx.x; k < re; k += kBlock) {
+                const uint32_t c = colInd[k] - base;
+                bad = bad || c >= mcol;
+                if (c == r) has[r] = 1; // 0 before
+            }
+        }
+        __syncthreads();
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) out->bad = 1;
 }
