@@ -650,7 +650,6 @@ void BiEngine<T>::destroy()
     dev_free(ctl);
     ctl = nullptr;
     pinned_put(hctl);
-    
     hctl = nullptr;
     hstatus = nullptr;
 }

@@ -32,14 +32,6 @@ int Ctx::sync()
     return kOk;
 }
 
-int Ctx::fetch(int slot, double* out)
-{
-    FB_CUDA(cudaMemcpyAsync(hslot + slot, dslot + slot, 8, cudaMemcpyDeviceToHost, stream));
-    FB_CUDA(cudaStreamSynchronize(stream));
-    *out = hslot[slot];
-    return kOk;
-}
-
 } // namespace fb
 
 static int g_device = 0;

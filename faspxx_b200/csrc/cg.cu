@@ -2070,7 +2070,6 @@ void CGEngine<T>::destroy()
     persistent = cluster = dsmem = false;
     cgrid = 0;
     pinned_put(hctl);
-    
     x = r = z = q = P0 = P1 = nullptr;
     ctl = nullptr;
     hctl = nullptr;

@@ -451,8 +451,8 @@ struct RowSep {
 };
 
 // The first tiles of this block, on their way before csr_tile_rows<..., BEGUN = true> (thread 0
-// copies; the matrix must be complete, whatever else the kernel still waits for). A kernel that
-// returns without the rows calls csr_tiles_drain first.
+// copies; the matrix must be complete, whatever else the kernel still waits for). In a kernel that
+// returns without the rows, thread 0 waits for the copies first (drain).
 template <typename T, bool PAT, int L = 1>
 struct CsrTiles {
     static constexpr uint32_t R = kTileRows / L; // rows of a tile

@@ -134,7 +134,6 @@ struct Ctx {
     // fixed-size grids (reductions depend on them): at most perSM blocks per SM
     int  grid(long long work, int perBlock, int perSM = 8) const;
     int  sync();
-    int  fetch(int slot, double* out);               // read one device scalar (synchronous)
 };
 
 // The device chosen by fasp_gpu_init (capi.cu).
@@ -408,8 +407,8 @@ int m_adopt(Mat& M, Mat& T, cudaStream_t s);
 int after_legacy_stream(cudaStream_t s);
 // dev_alloc with the spare bytes every matrix array has.
 int dmalloc(void** p, size_t bytes, cudaStream_t s);
-// Tile waits that ran out in the kernels of spmv.cu and solvers.cu (bulk copies that never
-// landed).
+// Tile waits that ran out (bulk copies that never landed), per source file; those of solvers.cu
+// include cg.cu's, mg.cu's and dcgs2.cu's.
 unsigned tile_timeouts_spmv();
 unsigned tile_timeouts_solvers();
 unsigned tile_timeouts_cg();

@@ -254,13 +254,6 @@ __global__ void k_copy_rows(uint32_t nh, const uint2* __restrict__ rows,
     }
 }
 
-int read_flag(cudaStream_t s, const int* dflag, int* hflag)
-{
-    FB_CUDA(cudaMemcpyAsync(hflag, dflag, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FB_CUDA(cudaStreamSynchronize(s));
-    return kOk;
-}
-
 template <typename T>
 int stage(Tmp& t, cudaStream_t s, const T* src, size_t count, bool onDevice, const T** out)
 {
