@@ -694,7 +694,10 @@ __global__ void __launch_bounds__(kBlock, (V4 ? 3 : (L > 1 ? 4 : (sizeof(T) == 4
                 double2 below = k0 > 0 ? pat(g - cols) : zero, cur = pat(g);
                 double2 above = k0 + 1 < nz ? pat(g + cols) : zero;
                 for (uint32_t k = k0; k < k1; ++k, g += cols) {
-                    // the plane after the next, one step ahead of its use
+                    // The plane after the next, one step ahead of its use. Rows too wide for
+                    // cg_spmv_walk and walks of two planes come here: 200 iterations at 512 x
+                    // 128^2 38.7 to 35.0 ms, 288 x 96^2 10.8 to 10.1, 512 x 64^2 9.1 to 8.7, 64^3
+                    // 3.18 to 3.13; walks of one plane (64^2 x 40) 2.79 either way.
                     const bool more = k + 2 < nz && k + 1 < k1;
                     const double2 zN = more ? z2[g + 2 * cols] : zero;
                     const double2 oN = more && mode ? po2[g + 2 * cols] : zero;

@@ -17,9 +17,12 @@ namespace fb {
 // at 127^3 14.4 us both ways, at 128^3 14.8 against the 10.3 of 16-byte groups.
 constexpr uint32_t kWalkS1 = kBlock; // 2 S1 edge values a plane, two a thread
 constexpr int kWalkCols = 2;         // columns a thread (1: 50 us at 101^3, 139 at 150^3)
-// Planes an item walks at least; it loads two more. BiCGStab with 4 (90^3) went from 44 to 40 us an
-// iteration, with 3 (80^3) 36.3 to 35.9, with 2 (64^3) 29.3 to 31.3; FP64 CG solves with 3 (95^3,
-// 90^3, 85^3) 6.5 to 5.6, 5.6 to 5.2 and 5.0 to 4.8 ms, with 2 (80^3, 72^3) 4.3 to 4.1 and 3.7 to 3.8.
+// Planes an item walks at least; it loads two more. From three on both engines gain: BiCGStab 44 to
+// 40 us an iteration at 90^3, FP64 CG solves 6.5 to 5.6, 5.6 to 5.2 and 5.0 to 4.8 ms at 95^3, 90^3
+// and 85^3. Below, some sizes gain and their neighbours lose, the other kernels and the walk, us an
+// iteration: FP64 CG 80^3 18.7 and 18.2, 72^3 17.2 and 17.9, 64^3 16.3 and 15.7, 56^3 14.7 and 14.9,
+// 47^3 13.0 and 13.5, 24^3 11.6 and 12.1; BiCGStab 72^3 27.3 and 25.1, 64^3 23.1 and 24.6, 56^3 22.2
+// and 21.3, 50^3 20.1 and 21.2.
 constexpr uint32_t kWalkChunk = 3;
 
 struct PlaneWalk {

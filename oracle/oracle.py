@@ -222,7 +222,7 @@ def norminf(kind, a):
 def transpose(kind, mat):
     """MAT::TransInPlace: returns (rowPtr, colInd, values, diagPtr) of the transpose. It moves
     entries and computes nothing, so where the reference is not built the restatement stands in
-    for it (tests/test_oracle.py compares the two where it is)."""
+    for it (tests/test_oracle.py holds it to transposes that the reference made)."""
     lib = load(kind if kind == "port" or os.path.exists(REF_SO) else "port")
     nnz = len(mat.colInd)
     trp = np.empty(mat.mcol + 1, np.uint32)
