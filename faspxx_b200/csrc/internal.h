@@ -105,6 +105,7 @@ inline int dev_alloc(T** p, size_t bytes, cudaStream_t s)
     return dev_alloc_bytes(reinterpret_cast<void**>(p), bytes, s);
 }
 void dev_free(void* p);
+void dev_bound(int dev); // gives back what dev's pool has idle beyond what it keeps
 void device_idle(int dev); // waits for all work on dev; the current device stays
 int  dev_trim(int dev); // waits for dev; its free pool memory goes back to the device
 // Page-locked host blocks of kPinnedBlock bytes, zeroed; null when there are none.

@@ -32,6 +32,9 @@ struct Tmp {
     {
         cudaStreamSynchronize(s);
         for (void* p : ptrs) dev_free(p);
+        int dev = 0;
+        cudaGetDevice(&dev);
+        dev_bound(dev);
     }
     template <typename T>
     int get(T** p, size_t count)

@@ -171,6 +171,11 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps* pr)
     *p = (cudaMemPool_t)&g_pools[pr->location.id];
     return cudaSuccess;
 }
+cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr, void* v)
+{
+    *(unsigned long long*)v = 0;
+    return cudaSuccess;
+}
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { ++g_trims; return cudaSuccess; }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t pool, cudaStream_t s)

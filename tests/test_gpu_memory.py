@@ -46,6 +46,31 @@ def test_trim_gives_idle_memory_back(sol):
     assert np.allclose(y.numpy(), A.matvec(np.ones(A.mcol)), rtol=1e-13, atol=0)
 
 
+def test_idle_memory_is_bounded(sol):
+    """Six matrices of about 1 GB each, destroyed: 4 GiB of them may wait for the next handles."""
+    torch = pytest.importorskip("torch")
+    A = _large(20_000_000)
+    gc.collect()
+    sol.trim()
+    before = torch.cuda.mem_get_info(0)[0]
+    held = [sol.MAT(A) for _ in range(6)]
+    taken = before - torch.cuda.mem_get_info(0)[0]
+    assert taken > 5 << 30
+    del held
+    gc.collect()
+    kept = before - torch.cuda.mem_get_info(0)[0]
+    assert kept <= (4 << 30) + (256 << 20)
+    # the next one takes from there, and is right
+    M = sol.MAT(A)
+    x = np.random.default_rng(1).uniform(-1, 1, A.mcol)
+    assert np.allclose(_apply(sol, M, A, x), A.matvec(x), rtol=1e-13, atol=1e-13)
+    assert before - torch.cuda.mem_get_info(0)[0] <= kept + (512 << 20)
+    del M
+    gc.collect()
+    sol.trim()
+    assert torch.cuda.mem_get_info(0)[0] >= before - (64 << 20)
+
+
 def _apply(sol, M, A, x):
     y = sol.DVec(A.nrow)
     M.Apply(sol.DVec.from_numpy(x), y)
