@@ -11,7 +11,8 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def load(where):
-    """The library on the fake runtime, built in the folder `where`."""
+    """The library on the fake runtime, built in the folder `where`. Its own definitions win over
+    those of a CUDA runtime that another package has loaded (-Bsymbolic)."""
     from faspxx_b200 import build, capi
     try:
         cuda = os.path.dirname(os.path.dirname(build.nvcc()))
@@ -19,7 +20,7 @@ def load(where):
         pytest.skip("no CUDA toolkit")
     build.build()
     lib = os.path.join(str(where), "libfasp_fake.so")
-    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", f"-I{cuda}/include",
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", f"-I{cuda}/include",
                     os.path.join(ROOT, "tests", "fake_cuda_runtime.cc"),
                     *sorted(glob.glob(os.path.join(build.BUILD, "*.o"))), "-o", lib], check=True)
     L = C.CDLL(lib, mode=os.RTLD_LOCAL)
