@@ -875,10 +875,24 @@ int launch_batch(fasp_gpu_batch_s& B, BatchArgs<T> a)
             B, res_args<T>(B, B.sval32, B.dinv32, a.b, a.x, a.relTol, a.maxIter), plain);
 }
 
+// Every system in global memory: the sliced copy, which nothing has read, is given back.
+void drop_slices(fasp_gpu_batch_s& B)
+{
+    dev_free(B.col);
+    dev_free(B.sval);
+    dev_free(B.sval32);
+    B.col = nullptr;
+    B.sval = nullptr;
+    B.sval32 = nullptr;
+    B.far = B.count;
+    std::fill(B.cls, B.cls + kResClasses + 1, B.count);
+}
+
 // Sorts the systems (ord, longest first) into the resident kernels' classes and builds the
 // sliced copy of the matrix. Columns outside their system: kErrMatData. Where padding the
-// slices would more than double the entries (one long row among short ones), or a row is longer
-// than a 16-bit length, every system runs in batch_pcg / batch_pcg_rel instead.
+// slices would more than double the entries (one long row among short ones), a row is longer
+// than a 16-bit length or the device has no memory for the copy, every system runs in batch_pcg /
+// batch_pcg_rel instead.
 int slice_systems(fasp_gpu_batch_s& B, const std::vector<uint32_t>& hs, std::vector<uint32_t>& ord)
 {
     cudaStream_t s = B.c.stream;
@@ -934,8 +948,10 @@ int slice_systems(fasp_gpu_batch_s& B, const std::vector<uint32_t>& hs, std::vec
             sum += m;
         }
         const size_t ne = (size_t)sum * 32;
-        if ((e = get(&B.col, ne * 2)) || (e = get(&B.sval, ne * 8)) || (e = get(&B.sval32, ne * 4)))
-            return e;
+        if (get(&B.col, ne * 2) || get(&B.sval, ne * 8) || get(&B.sval32, ne * 4)) {
+            drop_slices(B);
+            return kOk;
+        }
         FB_CUDA(cudaMemcpyAsync(B.sliceOff, off.data(), (size_t)slices * 4, cudaMemcpyHostToDevice, s));
         batch_fill_slices<<<g, 256, 0, s>>>(count, slices, B.sysRow, B.sliceBase, B.sliceOff,
                                             B.M.rowPtr, B.M.colInd, B.M.val, B.col, B.sval, B.sval32);
@@ -988,6 +1004,9 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
     dm((void**)&h->resRel, (size_t)count * nrhs * 8);
     dm((void**)&h->iters, (size_t)count * nrhs * 4);
     dm((void**)&h->queue, sizeof(unsigned) * (kResClasses + 1));
+    dm((void**)&h->r64, vN * 8); // the refinement's vectors
+    dm((void**)&h->b32, vN * 4);
+    dm((void**)&h->x32, vN * 4);
     if (!e) {
         // longest systems first
         std::vector<uint32_t> ord(count);
@@ -1001,11 +1020,13 @@ int fasp_gpu_batch_create(uint32_t count, const uint32_t* sysRow, uint32_t nnz,
                    cudaStreamSynchronize(h->c.stream) != cudaSuccess))
             e = kErrCuda;
     }
-    // vectors in global memory: the refinement's, and those of systems too large for a cluster
-    dm((void**)&h->r64, vN * 8);
-    dm((void**)&h->b32, vN * 4);
-    dm((void**)&h->x32, vN * 4);
-    if (!e && h->far) e = plain_vectors(*h);
+    if (!e && h->far) {
+        e = plain_vectors(*h);
+        if (e == kErrAlloc && h->col) { // without the copy there may be room
+            drop_slices(*h);
+            e = plain_vectors(*h);
+        }
+    }
     if (!e) {
         batch_dinv<<<std::max(1, std::min(ceil_div(N, 256), 148 * 8)), 256, 0, h->c.stream>>>(
             N, h->M.diag, h->dinv, h->dinv32);

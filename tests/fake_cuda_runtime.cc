@@ -45,6 +45,7 @@ std::map<void*, Block> g_blocks;
 std::map<const void*, std::string> g_names;
 std::vector<std::string> g_launched;
 int g_early = 0, g_clusters = 16, g_trims = 0, g_refused = 0;
+int g_failIn = -1, g_failures = 0; // device allocations until two in a row fail (a retry with them)
 int g_pools[kDevices] = {0, 1};
 
 #define HOLD std::lock_guard<std::recursive_mutex> hold(g_lock)
@@ -83,9 +84,15 @@ cudaError_t launch(const void* fn, cudaStream_t st)
     enqueue(st);
     return cudaSuccess;
 }
-cudaError_t allocate(void** p, size_t n, int dev, bool pooled)
+cudaError_t allocate(void** p, size_t n, int dev, bool pooled, bool device = true)
 {
     HOLD;
+    if (device && g_failIn >= 0 && --g_failIn < 0) {
+        ++g_failures;
+        if (g_failures % 2) g_failIn = 0;
+        *p = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
     *p = std::calloc(n + 256, 1);
     if (!*p) return cudaErrorMemoryAllocation;
     g_blocks[*p] = Block{n, dev, pooled};
@@ -100,6 +107,8 @@ extern "C" {
 int  fake_early_frees() { return g_early; }
 int  fake_blocks() { return (int)g_blocks.size(); }
 void fake_set_clusters(int n) { g_clusters = n; }
+void fake_fail_in(int n) { g_failIn = n; }
+int  fake_failures() { return g_failures; }
 int  fake_refused() { return g_refused; }
 int  fake_trims() { return g_trims; }
 int  fake_device() { return t_dev; }
@@ -159,7 +168,7 @@ const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 
 // ---- memory ----
 cudaError_t cudaMalloc(void** p, size_t n) { return allocate(p, n, t_dev, false); }
-cudaError_t cudaMallocHost(void** p, size_t n) { return allocate(p, n, t_dev, false); }
+cudaError_t cudaMallocHost(void** p, size_t n) { return allocate(p, n, t_dev, false, false); }
 cudaError_t cudaFreeHost(void* p)
 {
     HOLD;

@@ -76,6 +76,55 @@ def test_destroy_waits_for_the_handles_device(lib, kind, current):
     assert lib.fake_device() == current
 
 
+def _with_each_allocation_failing(lib, make, destroy):
+    """make() once for every device allocation it does, that one failing (and its retry): the codes.
+    Nothing that a failed call allocated stays."""
+    h = C.c_void_p()
+    assert make(h) == 0 and destroy(h) == 0  # contexts and page-locked blocks are in their lists
+    blocks, codes = lib.fake_blocks(), []
+    for k in range(100):
+        failed = lib.fake_failures()
+        lib.fake_fail_in(k)
+        code = make(h)
+        lib.fake_fail_in(-1)
+        if lib.fake_failures() == failed:  # fewer than k allocations
+            assert code == 0 and destroy(h) == 0
+            break
+        assert code in (0, -20), (k, code)
+        if code == 0:
+            assert destroy(h) == 0
+        codes.append(code)
+        assert lib.fake_blocks() <= blocks, k  # an idle context may have been given back
+        assert make(h) == 0 and destroy(h) == 0
+    assert len(codes) < 100
+    return codes
+
+
+def test_batch_without_memory_for_slices(lib):
+    """The resident kernels' copy of the matrix (columns, FP64 and FP32 values) is a convenience: a
+    batch for which the device has no room left but for the matrix itself is solved without it."""
+    assert lib.fasp_gpu_init(1) == 0
+    n = 1600
+    rows = _device(lib, np.array([0, 700, n], np.uint32))
+    d = [_device(lib, a) for a in (np.arange(n + 1, dtype=np.uint32), np.arange(n, dtype=np.uint32),
+                                   np.ones(n))]
+    codes = _with_each_allocation_failing(
+        lib, lambda h: lib.fasp_gpu_batch_create(2, rows, n, *d, 1, C.byref(h)),
+        lib.fasp_gpu_batch_destroy)
+    assert codes.count(0) == 3
+    # a system too large for a cluster beside small ones: its vectors, too, come before the copy
+    n = 66000
+    rows = _device(lib, np.array([0, 65800, n], np.uint32))
+    d = [_device(lib, a) for a in (np.arange(n + 1, dtype=np.uint32), np.arange(n, dtype=np.uint32),
+                                   np.ones(n))]
+    codes = _with_each_allocation_failing(
+        lib, lambda h: lib.fasp_gpu_batch_create(2, rows, n, *d, 1, C.byref(h)),
+        lib.fasp_gpu_batch_destroy)
+    # the copy's three; nine vectors and the FP32 values of matrix and classes, for which there is
+    # room without the copy
+    assert codes.count(0) == 3 + 11
+
+
 @pytest.mark.parametrize("precision", ["FP64", "MIXED", "MIXED_RELIABLE"])
 def test_batch_without_room_for_clusters(lib, precision):
     """A device that holds no cluster of the resident kernels (a process limited to some SMs) solves
