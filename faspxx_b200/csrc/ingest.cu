@@ -286,9 +286,8 @@ int coo_arrays(Ctx& c, uint32_t nrow, uint32_t mcol, uint32_t nnz, const uint32_
     k_count_coo<<<grid_for(nnz, 256), 256, 0, s>>>(nnz, nrow, mcol, ri, ci, cnt, slot, miss, out);
     FB_CUDA(cudaGetLastError());
     if ((e = lay_out(c, t, nrow, mcol, nnz, cnt, miss, out, tiles, T, &maxLen))) return e;
-    if (maxLen <= kRankMost) {
-        Rec* rec = nullptr;
-        if ((e = t.get(&rec, T.nnz))) return e;
+    Rec* rec = nullptr;
+    if (maxLen <= kRankMost && !t.get(&rec, T.nnz)) { // without memory for records: keys, half as long
         k_scatter_rec<<<grid_for(nnz, 256), 256, 0, s>>>(nnz, ri, ci, va, T.rowPtr, slot, rec);
         FB_CUDA(cudaGetLastError());
         return rank_rows<true>(c, nrow, T.rowPtr, nullptr, T.rowPtr, miss, RecSource{rec}, T.colInd,

@@ -122,9 +122,8 @@ int transpose_arrays(Ctx& c, const Mat& A, Mat& R)
     FB_CUDA(cudaMemcpyAsync(&most, longest, 4, cudaMemcpyDeviceToHost, s));
     FB_CUDA(cudaStreamSynchronize(s));
     const int g = std::max(1, std::min(ceil_div(n, kBlock), c.nsm * 8));
-    if (most <= kRankMost) {
-        Rec* rec = nullptr;
-        if ((e = t.get(&rec, nnz))) return e;
+    Rec* rec = nullptr;
+    if (most <= kRankMost && !t.get(&rec, nnz)) { // without memory for records: keys, half as long
         k_scatter_cols<true><<<g, kBlock, 0, s>>>(n, A.rowPtr, A.colInd, A.val, R.rowPtr, slot, rec,
                                                   nullptr);
         FB_CUDA(cudaGetLastError());

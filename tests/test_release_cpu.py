@@ -125,6 +125,36 @@ def test_batch_without_memory_for_slices(lib):
     assert codes.count(0) == 3 + 11
 
 
+@pytest.mark.parametrize("what", ["transpose", "coo", "csr_raw", "create", "stencil"])
+def test_matrices_without_memory(lib, what):
+    """Every allocation on the way to a matrix may fail: the call says so and leaves nothing behind.
+    Transposes and triplets, whose short rows travel as 16-byte records, do without the records
+    where there is no memory for them (8-byte keys)."""
+    assert lib.fasp_gpu_init(1) == 0
+    A, h = _matrix(lib)
+    rows = np.repeat(np.arange(A.nrow, dtype=np.uint32), np.diff(A.rowPtr.astype(np.int64)))
+    zero, one = np.zeros(1, np.int32), np.ones(1)
+    make = {
+        "transpose": lambda t: lib.fasp_gpu_mat_transpose(h, C.byref(t)),
+        "coo": lambda t: lib.fasp_gpu_mat_create_coo(A.nrow, A.mcol, A.nnz, rows.ctypes.data,
+                                                     A.colInd.ctypes.data, A.values.ctypes.data, 0,
+                                                     C.byref(t)),
+        "csr_raw": lambda t: lib.fasp_gpu_mat_create_csr_raw(A.nrow, A.mcol, A.nnz,
+                                                             A.rowPtr.ctypes.data,
+                                                             A.colInd.ctypes.data,
+                                                             A.values.ctypes.data, 0, C.byref(t)),
+        "create": lambda t: lib.fasp_gpu_mat_create(A.nrow, A.mcol, A.nnz, A.rowPtr.ctypes.data,
+                                                    A.colInd.ctypes.data, A.values.ctypes.data,
+                                                    C.byref(t)),
+        "stencil": lambda t: lib.fasp_gpu_mat_create_stencil(
+            20, 20, 1, 1, zero.ctypes.data, zero.ctypes.data, zero.ctypes.data, one.ctypes.data,
+            C.byref(t)),
+    }[what]
+    codes = _with_each_allocation_failing(lib, make, lib.fasp_gpu_mat_destroy)
+    assert codes.count(0) == (1 if what in ("transpose", "coo") else 0)
+    assert lib.fasp_gpu_mat_destroy(h) == 0
+
+
 @pytest.mark.parametrize("precision", ["FP64", "MIXED", "MIXED_RELIABLE"])
 def test_batch_without_room_for_clusters(lib, precision):
     """A device that holds no cluster of the resident kernels (a process limited to some SMs) solves
