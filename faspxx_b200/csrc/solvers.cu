@@ -378,11 +378,15 @@ int Pcd::solve_from_zero(Ctx& c, const double* b, double* x)
 template <typename T>
 static int alloc_vecs(std::vector<T*>& w, int k, uint32_t n, cudaStream_t s)
 {
-    const size_t bytes = ((size_t)n + 4) * sizeof(T);
+    const size_t bytes = ((size_t)n + 4) * sizeof(T), had = w.size();
     for (int i = 0; i < k; ++i) {
         T* p = nullptr;
         const int e = dev_alloc(&p, bytes, s);
-        if (e) return e;
+        if (e) { // all or none: some callers' lists are their own
+            cudaStreamSynchronize(s);
+            for (; w.size() > had; w.pop_back()) dev_free(w.back());
+            return e;
+        }
         w.push_back(p);
         FB_CUDA(cudaMemsetAsync(p, 0, bytes, s));
     }

@@ -183,3 +183,34 @@ def test_batch_without_room_for_clusters(lib, precision):
     finally:
         lib.fake_set_clusters(16)
     assert lib.fasp_gpu_batch_destroy(bt) == 0
+
+
+def _solver(lib, h, cfg):
+    s = C.c_void_p()
+    code = lib.fasp_gpu_solver_create(C.byref(cfg), C.byref(s))
+    if code == 0:
+        code = lib.fasp_gpu_solver_setup(s, h)
+        assert lib.fasp_gpu_solver_destroy(s) == 0
+    return code
+
+
+@pytest.mark.parametrize("alg,more", [
+    ("CG", {}), ("CG", {"pcd": 1}), ("CG", {"pcd": 2}), ("CG", {"precision": "MIXED"}),
+    ("CG", {"persistent": 1}), ("CG", {"persistent": 2}), ("CG", {"pcd": 1, "precision": "MIXED_RELIABLE"}),
+    ("BICGSTAB", {}), ("BICGSTAB", {"precision": "MIXED"}), ("BICGSTAB", {"precision": "MIXED_RELIABLE"}),
+    ("GMRES", {}), ("GMRES", {"precision": "MIXED"}), ("FGMRES", {}), ("JACOBI", {}), ("MG", {})])
+def test_setup_without_memory(lib, alg, more):
+    """Every allocation of a solver's Setup may fail: the code says so, and nothing is left behind
+    once the solver is destroyed."""
+    from faspxx_b200 import capi
+    assert lib.fasp_gpu_init(1) == 0
+    A, h = _matrix(lib)
+    cfg = capi.Config()
+    lib.fasp_gpu_default_config(C.byref(cfg), getattr(capi, alg))
+    cfg.prm.maxIter = 20
+    cfg.pcdPrm.minIter = cfg.pcdPrm.maxIter = 1
+    for k, v in more.items():
+        setattr(cfg, k, getattr(capi, v) if isinstance(v, str) else v)
+    codes = _with_each_allocation_failing(lib, lambda t: _solver(lib, h, cfg), lambda t: 0)
+    assert codes and codes.count(0) == 0
+    assert lib.fasp_gpu_mat_destroy(h) == 0
