@@ -611,10 +611,12 @@ int BiEngine<T>::init(Ctx* ctx, const Mat* M, int jac, const T* dinvv, bool grap
     T** vecs[] = {&x, &rj, &r0s, &pj2[0], &pj2[1], &ptmp2[0], &ptmp2[1], &sj, &stmp};
     for (T** v : vecs)
         if (dev_alloc(v, bytes, c->stream)) {
+            cudaStreamSynchronize(c->stream); // dev_free does not
             destroy();
             return kErrAlloc;
         }
     if (dev_alloc(&ctl, sizeof(BiCtl), c->stream) || !(hctl = (BiCtl*)pinned_get())) {
+        cudaStreamSynchronize(c->stream);
         destroy();
         return kErrAlloc;
     }

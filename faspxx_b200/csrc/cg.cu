@@ -1867,6 +1867,7 @@ int CGEngine<T>::init(Ctx* ctx, const Mat* M, int jac, const T* dinvv, bool grap
         dev_alloc(&P0, bytes, s) || dev_alloc(&P1, bytes, s) ||
         (jacobi && dev_alloc(&z, bytes, s)) || dev_alloc(&ctl, sizeof(CGCtl), s) ||
         !(hctl = (CGCtl*)pinned_get())) {
+        cudaStreamSynchronize(s); // dev_free does not
         destroy();
         return kErrAlloc;
     }

@@ -211,6 +211,9 @@ def test_setup_without_memory(lib, alg, more):
     cfg.pcdPrm.minIter = cfg.pcdPrm.maxIter = 1
     for k, v in more.items():
         setattr(cfg, k, getattr(capi, v) if isinstance(v, str) else v)
+    lib.fasp_gpu_synchronize()
+    early = lib.fake_early_frees()
     codes = _with_each_allocation_failing(lib, lambda t: _solver(lib, h, cfg), lambda t: 0)
     assert codes and codes.count(0) == 0
+    assert lib.fake_early_frees() == early  # what was enqueued before the failure is waited for
     assert lib.fasp_gpu_mat_destroy(h) == 0
