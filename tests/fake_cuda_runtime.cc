@@ -189,8 +189,9 @@ cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { ret
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { ++g_trims; return cudaSuccess; }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t pool, cudaStream_t s)
 {
-    enqueue(s);
-    return allocate(p, n, *(int*)pool, true);
+    const cudaError_t e = allocate(p, n, *(int*)pool, true);
+    if (e == cudaSuccess) enqueue(s);
+    return e;
 }
 cudaError_t cudaFree(void* p)
 {

@@ -78,8 +78,10 @@ def test_destroy_waits_for_the_handles_device(lib, kind, current):
 
 def _with_each_allocation_failing(lib, make, destroy):
     """make() once for every device allocation it does, that one failing (and its retry): the codes.
-    Nothing that a failed call allocated stays."""
+    Nothing that a failed call allocated stays, and nothing is released under unfinished work."""
     h = C.c_void_p()
+    lib.fasp_gpu_synchronize()
+    early = lib.fake_early_frees()
     assert make(h) == 0 and destroy(h) == 0  # contexts and page-locked blocks are in their lists
     blocks, codes = lib.fake_blocks(), []
     for k in range(100):
@@ -97,6 +99,7 @@ def _with_each_allocation_failing(lib, make, destroy):
         assert lib.fake_blocks() <= blocks, k  # an idle context may have been given back
         assert make(h) == 0 and destroy(h) == 0
     assert len(codes) < 100
+    assert lib.fake_early_frees() == early  # what was enqueued before a failure is waited for
     return codes
 
 
@@ -211,9 +214,6 @@ def test_setup_without_memory(lib, alg, more):
     cfg.pcdPrm.minIter = cfg.pcdPrm.maxIter = 1
     for k, v in more.items():
         setattr(cfg, k, getattr(capi, v) if isinstance(v, str) else v)
-    lib.fasp_gpu_synchronize()
-    early = lib.fake_early_frees()
     codes = _with_each_allocation_failing(lib, lambda t: _solver(lib, h, cfg), lambda t: 0)
     assert codes and codes.count(0) == 0
-    assert lib.fake_early_frees() == early  # what was enqueued before the failure is waited for
     assert lib.fasp_gpu_mat_destroy(h) == 0
